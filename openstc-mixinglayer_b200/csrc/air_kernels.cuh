@@ -9,7 +9,7 @@
 //                      per-thread ring of 2*ngg+1 nodes in shared memory (no halo re-reads)
 //   k_visc_update      [viscous_flux_fv/gv/hv + update_cv_and_bv_rk + update_physical_properties]
 //                      3-D tile, face fluxes staged in shared memory, RK combine and EOS fused
-//   k_bc_face          [apply_farfield/outflow/symmetry/periodic, in the reference priority order]
+//   k_bc_group, k_bc_face  [apply_* of the boundary faces, in the reference priority order]
 // The three RK stages ping-pong over three state buffers (A -> B -> C -> A) so no stage overwrites
 // data another block still reads; buffer A doubles as q^n (RK.cuh:99-102 needs no copy).
 // Part of the ostc_b200.cu translation unit (included in order; not a standalone header).
@@ -807,13 +807,6 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 8 ? 2 : 4) k_visc_update(
 
 // ------------------------------------------------------------------------------ boundaries
 
-__device__ __forceinline__ void copy_bv(const DevBlock &b, DevState s, long long dst, long long src) {
-#pragma unroll
-  for (int l = 0; l < 6; ++l) s.bv[l * b.plane + dst] = s.bv[l * b.plane + src];
-  if (s.sv)
-    for (int l = 0; l < c_mix.ns; ++l) s.sv[l * b.plane + dst] = s.sv[l * b.plane + src];
-}
-
 __device__ __forceinline__ void finish_node(const DevBlock &b, DevState s, long long p) {
   if (s.sv) {
     // mixtures: properties of the ghost come from the properties sweep over the padded block
@@ -824,94 +817,10 @@ __device__ __forceinline__ void finish_node(const DevBlock &b, DevState s, long 
   s.mul[p] = sutherland(s.bv[5 * b.plane + p]);
 }
 
-// apply_farfield for mixtures (BoundCond.cuh:755-1022) at face node pb: the node's gamma, its mixture
-// molecular weight from its mass fractions; supersonic inflow takes the far-field state and mass
-// fractions, supersonic outflow copies the node; subsonic faces take the Riemann invariants, the
-// velocity and composition of the far field (inflow, u_n < 0) or of the node, and a gamma iterated
-// with cp of the face temperature until it changes by less than 1e-4.  As in the reference, the
-// entropy of the inflow branch is chosen for u_n <= 0 but its velocity and composition for u_n < 0.
-__device__ void farfield_mixture(const DevBlock &b, DevState s, const DevFace &f, long long pb, long long dstep,
-                                 const double *gam_prev) {
-  const long long P = b.plane;
-  const int ns = c_mix.ns;
-  double nx = b.met[(f.face * 3 + 0) * P + pb], ny = b.met[(f.face * 3 + 1) * P + pb],
-         nz = b.met[(f.face * 3 + 2) * P + pb];
-  const double gni = f.direction / sqrt(nx * nx + ny * ny + nz * nz);
-  nx *= gni;
-  ny *= gni;
-  nz *= gni;
-  const double ub = s.bv[P + pb], vb = s.bv[2 * P + pb], wb = s.bv[3 * P + pb];
-  const double uf = nx * ub + ny * vb + nz * wb;
-  double svb[kMS];
-  for (int l = 0; l < ns; ++l) svb[l] = s.sv[l * P + pb];
-  const double gb = gam_prev[pb];
-  double mw_inv = 0;
-  for (int l = 0; l < ns; ++l) mw_inv += svb[l] / c_mix.mw[l];
-  double mw = 1.0 / mw_inv;
-  const double pbv = s.bv[4 * P + pb], rb = s.bv[pb];
-  const double ab = sqrt(gb * pbv / rb);
-  const double mb = uf / ab;
-  double vals[6];
-  if (mb <= -1) {
-    vals[0] = f.density; vals[1] = f.u; vals[2] = f.v; vals[3] = f.w; vals[4] = f.pressure; vals[5] = f.temperature;
-    for (int l = 0; l < ns; ++l) svb[l] = f.y[l];
-  } else if (mb >= 1) {
-    for (int g = 1; g <= b.g; ++g) {
-      const long long pg = b.chk(pb + g * dstep);
-      for (int l = 0; l < 6; ++l) s.bv[l * P + pg] = s.bv[l * P + pb];
-      for (int l = 0; l < ns; ++l) s.sv[l * P + pg] = s.sv[l * P + pb];
-      mix_cv_from_bv_node<0>(b, s, pg);
-    }
-    return;
-  } else {
-    const double rpos = uf + 2 * ab / (gb - 1);
-    const double uinf = f.u * nx + f.v * ny + f.w * nz;
-    const double rneg = uinf - 2 * f.acoustic_speed / (f.gamma - 1);
-    const double Un = 0.5 * (rpos + rneg);
-    if (mb < 0) {
-      vals[1] = f.u + (Un - uinf) * nx;
-      vals[2] = f.v + (Un - uinf) * ny;
-      vals[3] = f.w + (Un - uinf) * nz;
-      for (int l = 0; l < ns; ++l) svb[l] = f.y[l];
-      mw = f.mw;
-    } else {
-      vals[1] = ub + (Un - uf) * nx;
-      vals[2] = vb + (Un - uf) * ny;
-      vals[3] = wb + (Un - uf) * nz;
-    }
-    double gamma = kGamma, err = 1, rho = 0, pr = 0, t = 0;
-    // the reference's loop has no bound; 100 iterations (far more than the few it takes) end it here
-    for (int it = 0; err > 1e-4 && it < 100; ++it) {
-      const double glast = gamma;
-      const double cb = 0.25 * (gamma - 1) * (rpos - rneg);
-      const double sb = mb <= 0 ? f.entropy : pbv / pow(rb, gamma);
-      rho = pow(cb * cb / (gamma * sb), 1 / (gamma - 1));
-      pr = rho * cb * cb / gamma;
-      t = pr * mw / (rho * kRuD);
-      double cp[kMS];
-      mix_h_cp<0>(t, (double *)nullptr, cp);
-      double cpt = 0;
-      for (int l = 0; l < ns; ++l) cpt += cp[l] * svb[l];
-      gamma = cpt / (cpt - kRuD / mw);
-      err = fabs(1 - gamma / glast);
-    }
-    vals[0] = rho;
-    vals[4] = pr;
-    vals[5] = t;
-  }
-  for (int g = 0; g <= b.g; ++g) {
-    const long long pg = b.chk(pb + g * dstep);
-#pragma unroll
-    for (int l = 0; l < 6; ++l) s.bv[l * P + pg] = vals[l];
-    for (int l = 0; l < ns; ++l) s.sv[l * P + pg] = svb[l];
-    mix_cv_from_bv_node<0>(b, s, pg);
-  }
-}
-
-// One boundary face: apply_symmetry / apply_outflow / apply_periodic / apply_farfield<Air>
-// (BoundCond.cuh:137-233, 755-1022, 1443-1486).  Threads cover the two tangential index ranges,
-// which include ngg ghost layers on each side (Mesh.cpp:14-32).
-__global__ void __launch_bounds__(128) k_bc_face(DevBlock b, DevState s, DevFace f, const double *gam_prev) {
+// One boundary face: apply_inflow, apply_back_pressure / apply_subsonic_inflow, apply_wall (BoundCond.cuh:235-613,
+// 1024-1441); copy, symmetry and far-field faces are k_bc_group.  Threads cover the two tangential index
+// ranges, which include ngg ghost layers on each side (Mesh.cpp:14-32).
+__global__ void __launch_bounds__(128) k_bc_face(DevBlock b, DevState s, DevFace f) {
   const int t0 = f.face == 0 ? 1 : 0;
   const int t1 = f.face == 2 ? 1 : 2;
   const int n0 = f.re[t0] - f.rs[t0] + 1, n1 = f.re[t1] - f.rs[t1] + 1;
@@ -927,48 +836,7 @@ __global__ void __launch_bounds__(128) k_bc_face(DevBlock b, DevState s, DevFace
     idx[t0] = f.rs[t0] + (int)(n % n0);
     idx[t1] = f.rs[t1] + (int)(n / n0);
     const long long pb = b.id(idx[0], idx[1], idx[2]);
-    if (f.type == kSymmetry) {
-      const long long pin = b.chk(pb - dstep);
-      double kx = b.met[(f.face * 3 + 0) * P + pb], ky = b.met[(f.face * 3 + 1) * P + pb],
-             kz = b.met[(f.face * 3 + 2) * P + pb];
-      const double km = sqrt(kx * kx + ky * ky + kz * kz);
-      kx /= km;
-      ky /= km;
-      kz /= km;
-      const double u1 = s.bv[P + pin], v1 = s.bv[2 * P + pin], w1 = s.bv[3 * P + pin];
-      double uk = kx * u1 + ky * v1 + kz * w1;
-      s.bv[P + pb] = u1 - kx * uk;
-      s.bv[2 * P + pb] = v1 - ky * uk;
-      s.bv[3 * P + pb] = w1 - kz * uk;
-      s.bv[pb] = s.bv[pin];
-      s.bv[4 * P + pb] = s.bv[4 * P + pin];
-      s.bv[5 * P + pb] = s.bv[5 * P + pin];
-      if (s.sv) {
-        for (int l = 0; l < c_mix.ns; ++l) s.sv[l * P + pb] = s.sv[l * P + pin];
-      } else {
-        s.mul[pb] = sutherland(s.bv[5 * P + pb]);
-      }
-      for (int g = 1; g <= b.g; ++g) {
-        const long long pg = b.chk(pb + g * dstep), pi = b.chk(pb - g * dstep);
-        s.bv[pg] = s.bv[pi];
-        const double u = s.bv[P + pi], v = s.bv[2 * P + pi], w = s.bv[3 * P + pi];
-        uk = kx * u + ky * v + kz * w;
-        s.bv[P + pg] = u - 2 * uk * kx;
-        s.bv[2 * P + pg] = v - 2 * uk * ky;
-        s.bv[3 * P + pg] = w - 2 * uk * kz;
-        s.bv[4 * P + pg] = s.bv[4 * P + pi];
-        s.bv[5 * P + pg] = s.bv[5 * P + pi];
-        if (s.sv)
-          for (int l = 0; l < c_mix.ns; ++l) s.sv[l * P + pg] = s.sv[l * P + pi];
-        finish_node(b, s, pg);
-      }
-    } else if (f.type == kOutflow) {
-      for (int g = 1; g <= b.g; ++g) {
-        const long long pg = b.chk(pb + g * dstep);
-        copy_bv(b, s, pg, pb);
-        finish_node(b, s, pg);
-      }
-    } else if (f.type == kInflow) {
+    if (f.type == kInflow) {
       // apply_inflow (BoundCond.cuh:235-613): the face node and every ghost layer take one state -
       // the constant one, or the mixing-layer profile at the face node's y - with the white noise of
       // fluctuation_type 1 added to its velocity
@@ -1141,71 +1009,6 @@ __global__ void __launch_bounds__(128) k_bc_face(DevBlock b, DevState s, DevFace
         s.bv[3 * P + pg] = -s.bv[3 * P + pi];
         s.bv[4 * P + pg] = p_i;
         s.bv[5 * P + pg] = t_g;
-        finish_node(b, s, pg);
-      }
-    } else if (f.type == kPeriodic) {
-      const int ext[3] = {b.mx, b.my, b.mz};
-      int other[3] = {idx[0], idx[1], idx[2]};
-      other[f.face] = f.direction < 0 ? ext[f.face] - 1 : 0;
-      const long long po = b.id(other[0], other[1], other[2]);
-      for (int g = 1; g <= b.g; ++g) {
-        const long long pg = b.chk(pb + g * dstep), ps = b.chk(po + g * dstep);
-        copy_bv(b, s, pg, ps);
-        finish_node(b, s, pg);
-      }
-    } else if (f.type == kFarfield && s.sv) {
-      farfield_mixture(b, s, f, pb, dstep, gam_prev);
-    } else if (f.type == kFarfield) {
-      double nx = b.met[(f.face * 3 + 0) * P + pb], ny = b.met[(f.face * 3 + 1) * P + pb],
-             nz = b.met[(f.face * 3 + 2) * P + pb];
-      const double gni = f.direction / sqrt(nx * nx + ny * ny + nz * nz);
-      nx *= gni;
-      ny *= gni;
-      nz *= gni;
-      const double ub = s.bv[P + pb], vb = s.bv[2 * P + pb], wb = s.bv[3 * P + pb];
-      const double uf = nx * ub + ny * vb + nz * wb;
-      const double pbv = s.bv[4 * P + pb], rb = s.bv[pb];
-      const double ab = sqrt(kGamma * pbv / rb);
-      const double mb = uf / ab;
-      double vals[6];
-      if (mb <= -1) {
-        vals[0] = f.density; vals[1] = f.u; vals[2] = f.v; vals[3] = f.w; vals[4] = f.pressure; vals[5] = f.temperature;
-      } else if (mb >= 1) {
-        for (int g = 1; g <= b.g; ++g) {
-          const long long pg = b.chk(pb + g * dstep);
-          copy_bv(b, s, pg, pb);
-          finish_node(b, s, pg);
-        }
-        continue;
-      } else {
-        const double rpos = uf + 2 * ab / (kGamma - 1);
-        const double uinf = f.u * nx + f.v * ny + f.w * nz;
-        const double rneg = uinf - 2 * f.acoustic_speed / (f.gamma - 1);
-        const double Un = 0.5 * (rpos + rneg);
-        const double cb = 0.25 * (kGamma - 1) * (rpos - rneg);
-        double sb;
-        if (mb <= 0) {
-          sb = f.entropy;
-          vals[1] = f.u + (Un - uinf) * nx;
-          vals[2] = f.v + (Un - uinf) * ny;
-          vals[3] = f.w + (Un - uinf) * nz;
-        } else {
-          sb = pbv / pow(rb, kGamma);
-          vals[1] = ub + (Un - uf) * nx;
-          vals[2] = vb + (Un - uf) * ny;
-          vals[3] = wb + (Un - uf) * nz;
-        }
-        vals[0] = pow(cb * cb / (kGamma * sb), 1 / (kGamma - 1));
-        vals[4] = vals[0] * cb * cb / kGamma;
-        vals[5] = vals[4] * kMwD / (vals[0] * kRuD);
-      }
-#pragma unroll
-      for (int l = 0; l < 6; ++l) s.bv[l * P + pb] = vals[l];
-      finish_node(b, s, pb);
-      for (int g = 1; g <= b.g; ++g) {
-        const long long pg = b.chk(pb + g * dstep);
-#pragma unroll
-        for (int l = 0; l < 6; ++l) s.bv[l * P + pg] = vals[l];
         finish_node(b, s, pg);
       }
     }

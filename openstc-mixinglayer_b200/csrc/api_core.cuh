@@ -458,6 +458,12 @@ int ostc_create(const char *setup_txt, const char *input_dir, int device, ostc_c
                                                                      (unsigned long long)std::time(nullptr));
     }
   }
+  for (size_t b = 0; b < ctx->blk.size(); ++b)
+    if (group_bcs(ctx.get(), (int)b) != OSTC_OK) {
+      g_create_error = "device allocation failed";
+      ostc_destroy(ctx.release());
+      return OSTC_ENOMEM;
+    }
   const double dt0 = ctx->der.fixed_time_step ? ctx->der.dt : 1e6;
   cudaMemcpy(ctx->d_dt, &dt0, sizeof(double), cudaMemcpyHostToDevice);
   cudaMemset(ctx->d_time, 0, sizeof(double));
@@ -527,6 +533,7 @@ void ostc_destroy(ostc_ctx *ctx) {
     cudaFree(B.jac);
     cudaFree(B.met32);
     cudaFree(B.dq);
+    cudaFree(B.d_faces);
     cudaFree(B.last);
     cudaFree(B.adj);
     cudaFree(B.dqb);

@@ -15,6 +15,14 @@ struct BlockRes {
   double *dq = nullptr;
   double *last = nullptr;
   std::vector<DevFace> faces;  // file order
+  // boundary-face launches in application order: `count` faces from d_faces + first (the faces in
+  // that order on the device), or, where the kind is not grouped, the one face `single` of faces
+  struct BcLaunch {
+    int first, count, single;
+    long long nodes;  // of the largest face
+  };
+  std::vector<BcLaunch> bc_launches;
+  DevFace *d_faces = nullptr;
   std::vector<double *> face_y;  // per face: y of its nodes (mixing-layer inflows), else null
   double *plt_xyz = nullptr;     // flow-field output: the zone's coordinates for output width plt_g
   int plt_g = -1;

@@ -490,26 +490,72 @@ void df_start(ostc_ctx *ctx, unsigned long long seed) {
   k_df_first<<<grid_for(ctx, np, 128), 128, 0, st>>>(d);
 }
 
-// gam_prev: where a mixture far-field face reads the gamma of its face node - the properties of the
-// stage input (the reference's in-place state holds the last properties sweep there); null = out's.
-void launch_bcs(ostc_ctx *ctx, int block, DevState out, const double *gam_prev = nullptr) {
+// Groups block's boundary faces, in the reference's order, into launches (once, at create).  Faces join
+// the launch of the one before them when they lie along the same axis and none reads what another
+// writes: a face writes its own layer of nodes and the ghosts beyond it, and reads its own layer, up to
+// ngg interior layers on its own side (symmetry) or on the other (periodic).  The two sides of an axis
+// are therefore always independent (every extent is at least ngg + 2, read_mesh); on one side only
+// outflow patches share a launch (their ghost layers overlap in the padded corners, where both write
+// the same values).  A periodic or far-field box then takes one launch per axis instead of one per face.
+int group_bcs(ostc_ctx *ctx, int block) {
+  BlockRes &B = ctx->blk[block];
+  std::vector<DevFace> seq;
+  std::vector<BlockRes::BcLaunch> &out = B.bc_launches;
   for (const auto &bf : ctx->order) {
     if (bf.first != block) continue;
-    BlockRes &B = ctx->blk[block];
     const DevFace &f = B.faces[bf.second];
     const int t0 = f.face == 0 ? 1 : 0, t1 = f.face == 2 ? 1 : 2;
     const long long nn = (long long)(f.re[t0] - f.rs[t0] + 1) * (f.re[t1] - f.rs[t1] + 1);
-    long tok = begin_t(ctx, "bc_face");
-    if (f.type == kInflow && f.fluct == 11) {
-      // the digital filter (BoundCond.cuh:1561-1573): new random field, its convolutions, the time
-      // correlation with the current dt (zero at the initial application unless dt is fixed), then the
-      // inflow plane
-      enqueue_df_fluctuations(ctx, ctx->bc_initial && !ctx->der.fixed_time_step ? ctx->d_zero : ctx->d_dt, f);
-      const long long np = (long long)ctx->df.py * ctx->df.pz;
-      k_df_apply<<<grid_for(ctx, np, 128), 128, 0, ctx->stream>>>(B.db, out, f, ctx->df, ctx->df_mw_up,
-                                                                   ctx->df_mw_lo);
+    seq.push_back(f);
+    const int at = (int)seq.size() - 1;
+    if (!bc_grouped(f.type)) {
+      out.push_back({at, 1, bf.second, nn});
+      continue;
+    }
+    bool join = !out.empty() && out.back().single < 0;
+    for (int q = join ? out.back().first : at; q < at && join; ++q)
+      join = seq[q].face == f.face && (seq[q].rs[f.face] != f.rs[f.face] || (seq[q].type == kOutflow && f.type == kOutflow));
+    if (join) {
+      ++out.back().count;
+      out.back().nodes = std::max(out.back().nodes, nn);
     } else {
-      k_bc_face<<<grid_for(ctx, nn, 128), 128, 0, ctx->stream>>>(B.db, out, f, gam_prev ? gam_prev : out.gam);
+      out.push_back({at, 1, -1, nn});
+    }
+  }
+  if (seq.empty()) return OSTC_OK;
+  if (cudaMalloc(&B.d_faces, seq.size() * sizeof(DevFace)) != cudaSuccess ||
+      cudaMemcpy(B.d_faces, seq.data(), seq.size() * sizeof(DevFace), cudaMemcpyHostToDevice) != cudaSuccess)
+    return OSTC_ENOMEM;
+  return OSTC_OK;
+}
+
+// gam_prev: where a mixture far-field face reads the gamma of its face node - the properties of the
+// stage input (the reference's in-place state holds the last properties sweep there); null = out's.
+void launch_bcs(ostc_ctx *ctx, int block, DevState out, const double *gam_prev = nullptr) {
+  BlockRes &B = ctx->blk[block];
+  for (const auto &L : B.bc_launches) {
+    long tok = begin_t(ctx, "bc_face");
+    if (L.single >= 0) {
+      const DevFace &f = B.faces[L.single];
+      if (f.type == kInflow && f.fluct == 11) {
+        // the digital filter (BoundCond.cuh:1561-1573): new random field, its convolutions, the time
+        // correlation with the current dt (zero at the initial application unless dt is fixed), then the
+        // inflow plane
+        enqueue_df_fluctuations(ctx, ctx->bc_initial && !ctx->der.fixed_time_step ? ctx->d_zero : ctx->d_dt, f);
+        const long long np = (long long)ctx->df.py * ctx->df.pz;
+        k_df_apply<<<grid_for(ctx, np, 128), 128, 0, ctx->stream>>>(B.db, out, f, ctx->df, ctx->df_mw_up,
+                                                                     ctx->df_mw_lo);
+      } else {
+        k_bc_face<<<grid_for(ctx, L.nodes, 128), 128, 0, ctx->stream>>>(B.db, out, f);
+      }
+    } else {
+      const dim3 grid(grid_for(ctx, L.nodes, 128), L.count, B.db.g);
+      const double *gp = gam_prev ? gam_prev : out.gam;
+      const DevFace *fs = B.d_faces + L.first;
+      if (!ctx->mixture) k_bc_group<false, 0><<<grid, 128, 0, ctx->stream>>>(B.db, out, fs, gp);
+      else if (ctx->der.n_spec == kFixedNS)
+        k_bc_group<true, kFixedNS><<<grid, 128, 0, ctx->stream>>>(B.db, out, fs, gp);
+      else k_bc_group<true, 0><<<grid, 128, 0, ctx->stream>>>(B.db, out, fs, gp);
     }
     end_t(ctx, tok);
   }

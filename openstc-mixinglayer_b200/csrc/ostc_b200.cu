@@ -5,7 +5,8 @@
 // without relocatable device code every translation unit would get its own copy, so every kernel
 // and every launch is compiled here.  The parts, in include order:
 //   dev_types.cuh    device views of blocks, states, faces and interfaces
-//   air_kernels.cuh  air fluxes, viscous + update, time step, boundary faces, interfaces, set-up
+//   air_kernels.cuh  air fluxes, viscous + update, time step, interfaces, walls and inflows, set-up
+//   bc_faces.cuh     symmetry, outflow, periodic and far-field faces
 //   ostc_adj_air.cuh the air right-hand side's adjoint
 //   ostc_mix.cuh, ostc_adj.cuh, ostc_stat.cuh, ostc_steady.cuh, pv_mix.cuh, ostc_df.cuh
 //                    mixture kernels, adjoint, statistics, steady / DPLUR, mixture primitive
@@ -48,6 +49,7 @@
 static_assert(ostc::kMS <= 16, "DevFace::y holds the inflow mass fractions of at most 16 species");
 
 #include "air_kernels.cuh"
+#include "bc_faces.cuh"
 #include "ostc_adj_air.cuh"
 #include "context.cuh"
 #include "enqueue.cuh"
