@@ -59,6 +59,12 @@ int ostc_create(const char *setup_txt, const char *input_dir, int device, ostc_c
         m.low[i][q] = c.low[i * 7 + q];
         m.high[i][q] = c.high[i * 7 + q];
       }
+      for (int hi = 0; hi < 2; ++hi)
+        for (int q = 0; q < 4; ++q) {
+          const double aq = (hi ? m.high : m.low)[i][q + 1];
+          m.hint[hi][i][q] = aq / (q + 2);
+          m.gint[hi][i][q] = aq / ((q + 1) * (q + 2));
+        }
       m.lj_potent_inv[i] = c.lj_potent_inv[i];
       m.ln_lj[i] = std::log(c.lj_potent_inv[i]);
       m.vis_coeff[i] = c.vis_coeff[i];

@@ -33,6 +33,9 @@ struct MixTables {
   double weno_eps_scale, v_ref;
   double mw[kMS], imw[kMS], ru_mw[kMS], t_low[kMS], t_mid[kMS];
   double low[kMS][7], high[kMS][7];
+  // the polynomials' integrals below / above t_mid: h / Ru T's a1/2, a2/3, a3/4, a4/5 and the Gibbs
+  // energy's a1/2, a2/6, a3/12, a4/20, so that no evaluation divides
+  double hint[2][kMS][4], gint[2][kMS][4];
   double lj_potent_inv[kMS], vis_coeff[kMS];
   double wj_div_wi_1_4[kMS][kMS], sqrt_wiwj_8[kMS][kMS], binary_diff[kMS][kMS], kb_over_eps[kMS][kMS];
   // ln of lj_potent_inv and of kb_over_eps: the reduced temperatures' powers T*^a = exp(a (ln T + ln c))
@@ -47,47 +50,53 @@ struct MixTables {
 // the tables of the bound context (one translation unit includes this header)
 __constant__ MixTables c_mix;
 
-// compute_enthalpy_and_cp (Thermo.cu:136-192): h_k and cp_k in J/kg, linear h extrapolation below
-// t_low.  Either output may be null (compute_enthalpy / compute_cp).
+// One species of compute_enthalpy_and_cp (Thermo.cu:136-192): h_i and cp_i in J/kg, cp frozen and h
+// extrapolated linearly below t_low.  Horner form on the integrated coefficients of the tables: 10
+// multiply-adds where the powers, products and quotients of the written form took about 45 operations,
+// a division by 3 among them.
+template <typename T = double>
+__device__ __forceinline__ void mix_h_cp_one(int i, T t, T &h, T &cp) {
+  const T tl = (T)c_mix.t_low[i];
+  const T tt = t < tl ? tl : t;
+  const int hi = tt < (T)c_mix.t_mid[i] ? 0 : 1;
+  const double *a = hi ? c_mix.high[i] : c_mix.low[i];
+  const double *q = c_mix.hint[hi][i];
+  cp = ((((T)a[4] * tt + (T)a[3]) * tt + (T)a[2]) * tt + (T)a[1]) * tt + (T)a[0];
+  h = ((((T)q[3] * tt + (T)q[2]) * tt + (T)q[1]) * tt + (T)q[0]) * tt + (T)a[0];
+  h = h * tt + (T)a[5];
+  h = cp * (t - tt) + h;
+  h = h * (T)c_mix.ru_mw[i];
+  cp = cp * (T)c_mix.ru_mw[i];
+}
+
+// compute_enthalpy_and_cp (Thermo.cu:136-192) of every species.  Either output may be null
+// (compute_enthalpy / compute_cp).
 template <int NS, typename T = double>
 __device__ __forceinline__ void mix_h_cp(T t, T *h, T *cp) {
-  const T t2 = t * t, t3 = t2 * t, t4 = t3 * t, t5 = t4 * t;
 #pragma unroll
   for (int i = 0; i < OSTC_NS; ++i) {
     T hh, cc;
-    if (t < (T)c_mix.t_low[i]) {
-      const T tt = (T)c_mix.t_low[i], tt2 = tt * tt, tt3 = tt2 * tt, tt4 = tt3 * tt, tt5 = tt4 * tt;
-      const double *a = c_mix.low[i];
-      hh = (T)a[0] * tt + T(0.5) * (T)a[1] * tt2 + (T)a[2] * tt3 / T(3) + T(0.25) * (T)a[3] * tt4 +
-           T(0.2) * (T)a[4] * tt5 + (T)a[5];
-      cc = (T)a[0] + (T)a[1] * tt + (T)a[2] * tt2 + (T)a[3] * tt3 + (T)a[4] * tt4;
-      hh += cc * (t - tt);
-    } else {
-      const double *a = t < (T)c_mix.t_mid[i] ? c_mix.low[i] : c_mix.high[i];
-      hh = (T)a[0] * t + T(0.5) * (T)a[1] * t2 + (T)a[2] * t3 / T(3) + T(0.25) * (T)a[3] * t4 +
-           T(0.2) * (T)a[4] * t5 + (T)a[5];
-      cc = (T)a[0] + (T)a[1] * t + (T)a[2] * t2 + (T)a[3] * t3 + (T)a[4] * t4;
-    }
-    if (h) h[i] = hh * (T)c_mix.ru_mw[i];
-    if (cp) cp[i] = cc * (T)c_mix.ru_mw[i];
+    mix_h_cp_one<T>(i, t, hh, cc);
+    if (h) h[i] = hh;
+    if (cp) cp[i] = cc;
   }
 }
 
-// compute_gibbs_div_rt (Thermo.cu:194-210)
+// compute_gibbs_div_rt (Thermo.cu:194-210), evaluated at t_low below it
 template <int NS, typename T = double>
 __device__ __forceinline__ void mix_gibbs_rt(T t, T *g) {
-  const T t2 = t * t, t3 = t2 * t, t4 = t3 * t, ti = 1 / t, lt = log(t);
+  const T ti = 1 / t, lt = log(t);
 #pragma unroll
   for (int i = 0; i < OSTC_NS; ++i) {
     if (t < c_mix.t_low[i]) {
-      const double tt = c_mix.t_low[i], tt2 = tt * tt, tt3 = tt2 * tt, tt4 = tt3 * tt, tti = 1 / tt, ltt = log(tt);
-      const double *a = c_mix.low[i];
-      g[i] = a[0] * (1.0 - ltt) - 0.5 * a[1] * tt - a[2] * tt2 / 6.0 - a[3] * tt3 / 12.0 - a[4] * tt4 * 0.05 +
-             a[5] * tti - a[6];
+      const double tt = c_mix.t_low[i];
+      const double *a = c_mix.low[i], *q = c_mix.gint[0][i];
+      g[i] = a[0] * (1.0 - log(tt)) - tt * (q[0] + tt * (q[1] + tt * (q[2] + tt * q[3]))) + a[5] / tt - a[6];
     } else {
-      const double *a = t < c_mix.t_mid[i] ? c_mix.low[i] : c_mix.high[i];
-      g[i] = a[0] * (1.0 - lt) - 0.5 * a[1] * t - a[2] * t2 / 6.0 - a[3] * t3 / 12.0 - a[4] * t4 * 0.05 + a[5] * ti -
-             a[6];
+      const int hi = t < c_mix.t_mid[i] ? 0 : 1;
+      const double *a = hi ? c_mix.high[i] : c_mix.low[i];
+      const double *q = c_mix.gint[hi][i];
+      g[i] = a[0] * (1.0 - lt) - t * (q[0] + t * (q[1] + t * (q[2] + t * q[3]))) + a[5] * ti - a[6];
     }
   }
 }
