@@ -420,7 +420,7 @@ __device__ __forceinline__ void mix_lu_solve(double *lhs, double *b) {
 
 template <typename T>
 __device__ __forceinline__ T fvs_beta7(T s1, T s2, T s3) {
-  return s1 * s1 + T(13.0 / 12.0) * s2 * s2 + T(1043.0 / 960) * s3 * s3 + T(1.0 / 12) * s1 * s3;
+  return s1 * (s1 + T(1.0 / 12) * s3) + T(13.0 / 12.0) * s2 * s2 + T(1043.0 / 960) * s3 * s3;
 }
 
 // (eps + beta)^2 of the Z weights; in FP32 floored at 1e-30 so that a smooth stencil (beta = 0,
@@ -432,81 +432,78 @@ __device__ __forceinline__ T fvs_den(T eps, T beta) {
   return d;
 }
 
-// Unnormalised Z weights a_k = c_k (1 + tau / D_k), D_k = (eps + beta_k)^2.  FP64 forms the four
-// quotients from two divisions, 1 / D0 = D1 / (D0 D1) and alike (D_k >= eps^2 keeps the pair products
-// in range for any practical eps; if one underflows the four divisions are taken); FP32 divides each
-// (its scaled D_k may be as small as 1e-30).
-template <typename T>
-__device__ __forceinline__ void fvs_weights(T c0, T c1, T c2, T c3, T tau, T d0, T d1, T d2, T d3, T &a0, T &a1, T &a2,
-                                            T &a3) {
-  const T p01 = d0 * d1, p23 = d2 * d3;
-  if (sizeof(T) == 8 && p01 > T(0) && p23 > T(0)) {  // pair products representable (always, for eps > 1e-77)
-    const T r01 = tau / p01, r23 = tau / p23;
-    a0 = c0 + c0 * (d1 * r01);
-    a1 = c1 + c1 * (d0 * r01);
-    a2 = c2 + c2 * (d3 * r23);
-    a3 = c3 + c3 * (d2 * r23);
+// tau / D_k of the four Z weights, D_k = (eps + beta_k)^2.  FP64: one division where the product of the
+// four D_k is representable, else one per pair (D_k >= eps^2 keeps the pair products in range for any
+// practical eps), else four.  FP32 (its scaled D_k may be as small as 1e-30): four fast divisions.
+__device__ __forceinline__ void fvs_ratios(double tau, const double *d, double *r) {
+  const double p01 = d[0] * d[1], p23 = d[2] * d[3], p = p01 * p23;
+  double r01, r23;
+  if (p > 1e-290) {
+    const double q = 1.0 / p;
+    r01 = tau * (p23 * q);
+    r23 = tau * (p01 * q);
+  } else if (p01 > 0.0 && p23 > 0.0) {
+    r01 = tau / p01;
+    r23 = tau / p23;
   } else {
-    a0 = c0 + c0 * tau / d0;
-    a1 = c1 + c1 * tau / d1;
-    a2 = c2 + c2 * tau / d2;
-    a3 = c3 + c3 * tau / d3;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r[k] = tau / d[k];
+    return;
+  }
+  r[0] = d[1] * r01;
+  r[1] = d[0] * r01;
+  r[2] = d[3] * r23;
+  r[3] = d[2] * r23;
+}
+__device__ __forceinline__ void fvs_ratios(float tau, const float *d, float *r) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) r[k] = __fdividef(tau, d[k]);
+}
+
+// One side of the flux-split WENO7-Z (WENO.cu:1619-1693), its points v0..v6 upwind first: the face value
+// is v3 + num / den.  The reference's derivatives s1, s2, s3 of each substencil and its interpolants are
+// written with the first, second and third differences the substencils share: s1 = d + e/2 + t/3 and
+// alike (the coefficients are those of WENO.cu:1626-1655 term by term), and the interpolant of every
+// substencil is v3 + s1/2 + s2/12.  That takes 50 operations for the four indicators and interpolants
+// instead of 110 from the points, and its differences lose no digits to the points' size.
+template <typename T>
+__device__ __forceinline__ void fvs_side(T v0, T v1, T v2, T v3, T v4, T v5, T v6, T eps, T &num, T &den) {
+  const T d2 = v3 - v2, d3 = v4 - v3;
+  const T e0 = (v2 - v1) - (v1 - v0), e1 = d2 - (v2 - v1), e2 = d3 - d2, e3 = (v5 - v4) - d3;
+  const T e4 = (v6 - v5) - (v5 - v4);
+  const T t0 = e1 - e0, t1 = e2 - e1, t2 = e3 - e2, t3 = e4 - e3;
+  const T mid = d2 + T(0.5) * e2;
+  const T s1[4] = {d2 + (T(0.5) * e1 + T(1.0 / 3) * t0), mid - T(1.0 / 6) * t1, mid - T(1.0 / 6) * t2,
+                   d3 - (T(0.5) * e3 - T(1.0 / 3) * t3)};
+  const T s2[4] = {e1 + t0, e2, e2, e3 - t3};
+  const T s3[4] = {t0, t1, t2, t3};
+  const T c[4] = {T(1.0 / 35), T(12.0 / 35), T(18.0 / 35), T(4.0 / 35)};
+  T b[4], d[4], r[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    b[k] = fvs_beta7(s1[k], s2[k], s3[k]);
+    d[k] = fvs_den(eps, b[k]);
+  }
+  fvs_ratios((b[0] - b[3]) * (b[0] - b[3]), d, r);
+  num = T(0);
+  den = T(0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const T a = c[k] + c[k] * r[k];
+    num += a * (T(0.5) * s1[k] + T(1.0 / 12) * s2[k]);
+    den += a;
   }
 }
 
-// WENO7 of the flux-split path (WENO.cu:1619-1693): returns f+ + f-.
+// Both sides of the flux-split WENO7-Z: f+ + f-, the - side mirrored.  FP64 forms the two quotients with
+// one division (a weight sum is at most (v^2 / eps)^2 ~ 1e110, far from the range's end when squared).
 template <typename T>
 __device__ __forceinline__ T fvs_weno7_core(const T *vp, const T *vm, T eps) {
-  const T one6th = T(1.0 / 6), one12th = T(1.0 / 12);
-  const T c0 = T(1.0 / 35), c1 = T(12.0 / 35), c2 = T(18.0 / 35), c3 = T(4.0 / 35);
-  T s1 = one6th * (-2 * vp[0] + 9 * vp[1] - 18 * vp[2] + 11 * vp[3]);
-  T s2 = -vp[0] + 4 * vp[1] - 5 * vp[2] + 2 * vp[3];
-  T s3 = -vp[0] + 3 * vp[1] - 3 * vp[2] + vp[3];
-  T b0 = fvs_beta7(s1, s2, s3);
-  s1 = one6th * (vp[1] - 6 * vp[2] + 3 * vp[3] + 2 * vp[4]);
-  s2 = vp[2] - 2 * vp[3] + vp[4];
-  s3 = -vp[1] + 3 * vp[2] - 3 * vp[3] + vp[4];
-  T b1 = fvs_beta7(s1, s2, s3);
-  s1 = one6th * (-2 * vp[2] - 3 * vp[3] + 6 * vp[4] - vp[5]);
-  s3 = -vp[2] + 3 * vp[3] - 3 * vp[4] + vp[5];
-  T b2 = fvs_beta7(s1, s2, s3);
-  s1 = one6th * (-11 * vp[3] + 18 * vp[4] - 9 * vp[5] + 2 * vp[6]);
-  s2 = 2 * vp[3] - 5 * vp[4] + 4 * vp[5] - vp[6];
-  s3 = -vp[3] + 3 * vp[4] - 3 * vp[5] + vp[6];
-  T b3 = fvs_beta7(s1, s2, s3);
-  T tau = (b0 - b3) * (b0 - b3);
-  T a0, a1, a2, a3;
-  fvs_weights(c0, c1, c2, c3, tau, fvs_den(eps, b0), fvs_den(eps, b1), fvs_den(eps, b2), fvs_den(eps, b3), a0, a1, a2,
-              a3);
-  T v0 = one12th * (-3 * vp[0] + 13 * vp[1] - 23 * vp[2] + 25 * vp[3]);
-  T v1 = one12th * (vp[1] - 5 * vp[2] + 13 * vp[3] + 3 * vp[4]);
-  T v2 = one12th * (-vp[2] + 7 * vp[3] + 7 * vp[4] - vp[5]);
-  T v3 = one12th * (3 * vp[3] + 13 * vp[4] - 5 * vp[5] + vp[6]);
-  const T fp = (a0 * v0 + a1 * v1 + a2 * v2 + a3 * v3) / (a0 + a1 + a2 + a3);
-  s1 = one6th * (-2 * vm[6] + 9 * vm[5] - 18 * vm[4] + 11 * vm[3]);
-  s2 = -vm[6] + 4 * vm[5] - 5 * vm[4] + 2 * vm[3];
-  s3 = -vm[6] + 3 * vm[5] - 3 * vm[4] + vm[3];
-  b0 = fvs_beta7(s1, s2, s3);
-  s1 = one6th * (vm[5] - 6 * vm[4] + 3 * vm[3] + 2 * vm[2]);
-  s2 = vm[4] - 2 * vm[3] + vm[2];
-  s3 = -vm[5] + 3 * vm[4] - 3 * vm[3] + vm[2];
-  b1 = fvs_beta7(s1, s2, s3);
-  s1 = one6th * (-2 * vm[4] - 3 * vm[3] + 6 * vm[2] - vm[1]);
-  s3 = -vm[4] + 3 * vm[3] - 3 * vm[2] + vm[1];
-  b2 = fvs_beta7(s1, s2, s3);
-  s1 = one6th * (-11 * vm[3] + 18 * vm[2] - 9 * vm[1] + 2 * vm[0]);
-  s2 = 2 * vm[3] - 5 * vm[2] + 4 * vm[1] - vm[0];
-  s3 = -vm[3] + 3 * vm[2] - 3 * vm[1] + vm[0];
-  b3 = fvs_beta7(s1, s2, s3);
-  tau = (b0 - b3) * (b0 - b3);
-  fvs_weights(c0, c1, c2, c3, tau, fvs_den(eps, b0), fvs_den(eps, b1), fvs_den(eps, b2), fvs_den(eps, b3), a0, a1, a2,
-              a3);
-  v0 = one12th * (-3 * vm[6] + 13 * vm[5] - 23 * vm[4] + 25 * vm[3]);
-  v1 = one12th * (vm[5] - 5 * vm[4] + 13 * vm[3] + 3 * vm[2]);
-  v2 = one12th * (-vm[4] + 7 * vm[3] + 7 * vm[2] - vm[1]);
-  v3 = one12th * (3 * vm[3] + 13 * vm[2] - 5 * vm[1] + vm[0]);
-  const T fm = (a0 * v0 + a1 * v1 + a2 * v2 + a3 * v3) / (a0 + a1 + a2 + a3);
-  return fp + fm;
+  T np, dp, nm, dm;
+  fvs_side(vp[0], vp[1], vp[2], vp[3], vp[4], vp[5], vp[6], eps, np, dp);
+  fvs_side(vm[6], vm[5], vm[4], vm[3], vm[2], vm[1], vm[0], eps, nm, dm);
+  if constexpr (sizeof(T) == 8) return vp[3] + vm[3] + (np * dm + nm * dp) / (dp * dm);
+  else return vp[3] + vm[3] + (__fdividef(np, dp) + __fdividef(nm, dm));
 }
 
 __device__ __forceinline__ double fvs_weno7(const double *vp, const double *vm, double eps) {

@@ -126,9 +126,10 @@ template <int DIR> struct FvsTile {
   static constexpr int NST = TD + 7;  // staged nodes: stencils of 8 nodes around TD faces
 };
 
+// split fluxes of the staged nodes [2][nv][NST][TXL], then the face fluxes [nv][TD][TXL]
 template <int DIR, typename T>
 __host__ __device__ constexpr size_t fvs_smem_bytes(int nv) {
-  return (size_t)FvsTile<DIR>::NST * FvsTile<DIR>::TXL * nv * 2 * sizeof(T);
+  return (size_t)(2 * FvsTile<DIR>::NST + FvsTile<DIR>::TD) * FvsTile<DIR>::TXL * nv * sizeof(T);
 }
 
 // compute_convective_term_weno_x/_y/_z (WENO.cu:8-461) for inviscid_scheme 72 (characteristic,
@@ -137,21 +138,26 @@ __host__ __device__ constexpr size_t fvs_smem_bytes(int nv) {
 // computed once into shared memory; each thread then forms one face flux from the 8-node stencil,
 // and after a barrier the node threads difference neighbouring faces into dq.  T is the arithmetic
 // type of the fluxes (FP32 in the mixed precision mode: state read in FP64, dq accumulated in FP64).
-// Resident blocks per SM (measured on the 384 x 192 x 96 layer): FP64 4; FP32 8 (64 registers, some
-// spills; 6, 7 and 8 blocks ran the mixed step in 79.5, 77.0 and 76.9 ms against 84.6 ms at 4).
+// Bound by FP64 arithmetic at the occupancy its shared memory and registers leave (40 % of the FP64 pipe;
+// DRAM 8 %).  The staged values are laid out variable by variable, so that a warp's threads read
+// consecutive words; with the variables of a node side by side (a stride of 14 doubles) every read was a
+// two-way bank conflict.  Species arrays live in the thread's face-flux slots and the staged values are read
+// again per row: spills 2.8 KB -> 0.3 KB a thread.  192 x 96 x 48, FP64: 0.86 / 0.79 / 0.85 -> 0.60 / 0.58 /
+// 0.64 ms (x / y / z); 257 x 129 x 65, FP32: 1.32 / 1.19 / 1.27 -> 0.85 / 0.78 / 0.85 ms.  Resident blocks
+// per SM: FP64 4 (three sweeps 1.82 ms; 3: 1.92), FP32 6 (2.48 ms; 8: 2.54).
 template <int DIR, int NS, typename T>
-__global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T) == 8 ? 4 : 8) k_fvs(DevBlock b, DevState s,
+__global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T) == 8 ? 4 : 6) k_fvs(DevBlock b, DevState s,
                                                                                double *__restrict__ dq, int nv,
                                                                                int scheme) {
   constexpr int TXL = FvsTile<DIR>::TXL, TD = FvsTile<DIR>::TD, NST = FvsTile<DIR>::NST;
   extern __shared__ __align__(16) unsigned char mix_smem[];
-  T *fsm = reinterpret_cast<T *>(mix_smem);
-  T *Fp = fsm;                        // [NST][TXL][nv]
-  T *Fm = fsm + NST * TXL * nv;       // [NST][TXL][nv]
-  const int lane = DIR == 0 ? 0 : (int)threadIdx.x;
-  const int t = DIR == 0 ? (int)threadIdx.x : (int)threadIdx.y;
   const int ns = OSTC_NS;
   if (NS > 0) nv = 5 + NS;
+  T *Fp = reinterpret_cast<T *>(mix_smem);
+  T *Fm = Fp + nv * NST * TXL;
+  T *fcs = Fm + nv * NST * TXL;
+  const int lane = DIR == 0 ? 0 : (int)threadIdx.x;
+  const int t = DIR == 0 ? (int)threadIdx.x : (int)threadIdx.y;
   const long long P = b.plane;
   const int nd = DIR == 0 ? b.mx : DIR == 1 ? b.my : b.mz;
   const int start = (DIR == 0 ? blockIdx.x : blockIdx.y) * (TD - 1);
@@ -175,6 +181,7 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
       if (n > nd + 3) continue;
       const long long p = pid(n);
       T Q[Spec<NS>::A + 5];
+#pragma unroll
       for (int l = 0; l < nv; ++l) Q[l] = (T)s.cv[l * P + p];
       const T pk = (T)s.bv[4 * P + p];
       const T c = (T)(s.acs ? s.acs[p] : sqrt(kGamma * (kRuD / kMwD) * s.bv[5 * P + p]));
@@ -184,30 +191,22 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
       const T Uk = (Q[1] * k0m + Q[2] * k1m + Q[3] * k2m) / Q[0];
       const T cg = c * tsqrt(k0m * k0m + k1m * k1m + k2m * k2m);
       const T l0 = tabs(Uk) + cg;
-      T *fp = Fp + ((long long)st * TXL + lane) * nv, *fm = Fm + ((long long)st * TXL + lane) * nv;
-      fp[0] = half * jac * (Uk * Q[0] + l0 * Q[0]);
-      fp[1] = half * jac * (Uk * Q[1] + pk * k0m + l0 * Q[1]);
-      fp[2] = half * jac * (Uk * Q[2] + pk * k1m + l0 * Q[2]);
-      fp[3] = half * jac * (Uk * Q[3] + pk * k2m + l0 * Q[3]);
-      fp[4] = half * jac * (Uk * (Q[4] + pk) + l0 * Q[4]);
-      fm[0] = half * jac * (Uk * Q[0] - l0 * Q[0]);
-      fm[1] = half * jac * (Uk * Q[1] + pk * k0m - l0 * Q[1]);
-      fm[2] = half * jac * (Uk * Q[2] + pk * k1m - l0 * Q[2]);
-      fm[3] = half * jac * (Uk * Q[3] + pk * k2m - l0 * Q[3]);
-      fm[4] = half * jac * (Uk * (Q[4] + pk) - l0 * Q[4]);
-      for (int l = 5; l < nv; ++l) {
-        fp[l] = half * jac * (Uk * Q[l] + l0 * Q[l]);
-        fm[l] = half * jac * (Uk * Q[l] - l0 * Q[l]);
+      const T hj = half * jac, up = hj * (Uk + l0), um = hj * (Uk - l0), pj = hj * pk;
+      T *fp = Fp + st * TXL + lane, *fm = Fm + st * TXL + lane;
+#pragma unroll
+      for (int l = 0; l < nv; ++l) {
+        const T pl = l == 1 ? pj * k0m : l == 2 ? pj * k1m : l == 3 ? pj * k2m : l == 4 ? pj * Uk : T(0);
+        fp[l * NST * TXL] = up * Q[l] + pl;
+        fm[l * NST * TXL] = um * Q[l] + pl;
       }
     }
   }
   __syncthreads();
   const int n = start - 1 + t;  // left node of this thread's face
   const bool face_ok = lane_ok && n < nd;
-  T fc[Spec<NS>::A + 5];
-  for (int l = 0; l < kMV; ++l) fc[l] = T(0);
-  auto FP = [&](int m, int l) -> T { return Fp[((long long)(t + m) * TXL + lane) * nv + l]; };
-  auto FM = [&](int m, int l) -> T { return Fm[((long long)(t + m) * TXL + lane) * nv + l]; };
+  auto FP = [&](int m, int l) -> T { return Fp[(l * NST + t + m) * TXL + lane]; };
+  auto FM = [&](int m, int l) -> T { return Fm[(l * NST + t + m + 1) * TXL + lane]; };  // node m of the - side
+  auto FC = [&](int tt, int l) -> T & { return fcs[(l * TD + tt) * TXL + lane]; };
   if (face_ok && scheme == 71) {
     const long long pl = pid(n), pr = pid(n + 1);
     const double j1 = b.jac[pl], j2 = b.jac[pr];
@@ -216,162 +215,181 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
     const double eps_ref = 1e-20 * c_mix.weno_eps_scale * 0.25 * (a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
     const double e1 = eps_ref * c_mix.v_ref * c_mix.v_ref;
     const double e2 = e1 * c_mix.v_ref * c_mix.v_ref;
+#pragma unroll 1
     for (int l = 0; l < nv; ++l) {
       const double e = (l >= 1 && l <= 3) ? e1 : (l == 4 ? e2 : eps_ref);
       T vp[7], vm[7];
+#pragma unroll
       for (int m = 0; m < 7; ++m) {
         vp[m] = FP(m, l);
-        vm[m] = FM(m + 1, l);
+        vm[m] = FM(m, l);
       }
-      fc[l] = fvs_weno7(vp, vm, e);
+      FC(t, l) = fvs_weno7(vp, vm, e);
     }
   } else if (face_ok) {
-    // Roe-averaged mixture eigensystem at the face (WENO.cu:747-821)
+    // Roe-averaged mixture eigensystem at the face (WENO.cu:747-821).  The species' alpha_l of L wait in
+    // this thread's own face-flux slots until the species loop replaces them.
     const long long pl = pid(n), pr = pid(n + 1);
-    T cvl[Spec<NS>::A + 5], cvr[Spec<NS>::A + 5];
-    for (int l = 0; l < nv; ++l) {
-      cvl[l] = (T)s.cv[l * P + pl];
-      cvr[l] = (T)s.cv[l * P + pr];
-    }
+    const T rl = (T)s.cv[pl], rr = (T)s.cv[pr];
     const T p_l = (T)s.bv[4 * P + pl], p_r = (T)s.bv[4 * P + pr];
-    const T rli = T(1) / cvl[0], rri = T(1) / cvr[0];
-    const T sl = tsqrt(cvl[0]), sr = tsqrt(cvr[0]);
-    const T rlc = sl / (sl + sr), rrc = sr / (sl + sr);
-    const T um = rlc * cvl[1] * rli + rrc * cvr[1] * rri;
-    const T vm_ = rlc * cvl[2] * rli + rrc * cvr[2] * rri;
-    const T wm = rlc * cvl[3] * rli + rrc * cvr[3] * rri;
+    const T rli = T(1) / rl, rri = T(1) / rr;
+    const T sl = tsqrt(rl), sr = tsqrt(rr);
+    const T isum = T(1) / (sl + sr);
+    const T wl = sl * isum * rli, wr = sr * isum * rri;  // Roe weights over rho
+    auto roe = [&](int l) -> T { return wl * (T)s.cv[l * P + pl] + wr * (T)s.cv[l * P + pr]; };
+    const T um = roe(1), vm_ = roe(2), wm = roe(3);
     const T ekm = half * (um * um + vm_ * vm_ + wm * wm);
-    const T hm = rlc * ((cvl[4] + p_l) * rli) + rrc * ((cvr[4] + p_r) * rri);
-    T svm[Spec<NS>::A], hi[Spec<NS>::A], cpi[Spec<NS>::A], al[Spec<NS>::A];
-    T mw_inv = 0;
-    for (int l = 0; l < ns; ++l) {
-      svm[l] = rlc * cvl[l + 5] * rli + rrc * cvr[l + 5] * rri;
-      mw_inv += svm[l] / (T)c_mix.mw[l];
+    const T hm = roe(4) + (wl * p_l + wr * p_r);
+    T cm, gm1, c2i;
+    T sp[7], sm[7];
+    {
+      T mw_inv = 0;
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) {
+        const T sv = roe(5 + l);
+        mw_inv += sv * (T)c_mix.imw[l];
+        FC(t, 5 + l) = sv;
+      }
+      const T tm = (wl * p_l + wr * p_r) / (T(kRuD) * mw_inv);
+      T cp = 0, cvt = 0;
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) {
+        T h, c;
+        mix_h_cp_one<T>(l, tm, h, c);
+        const T sv = FC(t, 5 + l);
+        cp += sv * c;
+        cvt += sv * (c - (T)c_mix.ru_mw[l]);
+        FC(t, 5 + l) = h;
+      }
+      const T gamma = cp / cvt;
+      const T c2 = gamma * T(kRuD) * mw_inv * tm;
+      cm = tsqrt(c2);
+      gm1 = gamma - 1;
+      c2i = T(1) / c2;
+      // The species columns of the five flow rows of L are cs_l * al[q] (cs = 1/2, -kx, -ky, -kz, 1/2):
+      // their products with the split fluxes share one sum per stencil node, formed once for all rows.
+#pragma unroll
+      for (int m = 0; m < 7; ++m) sp[m] = sm[m] = T(0);
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) {
+        const T al = (gamma * (T)c_mix.ru_mw[l] * tm - gm1 * FC(t, 5 + l)) * c2i;
+        FC(t, 5 + l) = al;
+#pragma unroll
+        for (int m = 0; m < 7; ++m) {
+          sp[m] += al * FP(m, 5 + l);
+          sm[m] += al * FM(m, 5 + l);
+        }
+      }
     }
-    const T tm = (rlc * (p_l * rli) + rrc * (p_r * rri)) / (T(kRuD) * mw_inv);
-    mix_h_cp<NS, T>(tm, hi, cpi);
-    T cp = 0, cvt = 0;
-    for (int l = 0; l < ns; ++l) {
-      cp += svm[l] * cpi[l];
-      cvt += svm[l] * (cpi[l] - (T)c_mix.ru_mw[l]);
-    }
-    const T gamma = cp / cvt;
-    const T cm = tsqrt(gamma * T(kRuD) * mw_inv * tm);
-    const T gm1 = gamma - 1;
     const double jld = b.jac[pl], jrd = b.jac[pr];
     const double kxJd = b.met[(DIR * 3 + 0) * P + pl] * jld + b.met[(DIR * 3 + 0) * P + pr] * jrd;
     const double kyJd = b.met[(DIR * 3 + 1) * P + pl] * jld + b.met[(DIR * 3 + 1) * P + pr] * jrd;
     const double kzJd = b.met[(DIR * 3 + 2) * P + pl] * jld + b.met[(DIR * 3 + 2) * P + pr] * jrd;
     const double eps = 1e-40 * c_mix.weno_eps_scale * 0.25 * (kxJd * kxJd + kyJd * kyJd + kzJd * kzJd);
-    const T jlr = (T)(jld + jrd);
-    T kx = (T)kxJd / jlr, ky = (T)kyJd / jlr, kz = (T)kzJd / jlr;
-    const T gradK = tsqrt(kx * kx + ky * ky + kz * kz);
-    kx /= gradK;
-    ky /= gradK;
-    kz /= gradK;
+    // the unit normal: the Jacobian-weighted mean metric, its length cancels
+    T kx = (T)kxJd, ky = (T)kyJd, kz = (T)kzJd;
+    const T igk = T(1) / tsqrt(kx * kx + ky * ky + kz * kz);
+    kx *= igk;
+    ky *= igk;
+    kz *= igk;
     const T Ukb = kx * um + ky * vm_ + kz * wm;
-    const T alpha = gm1 * ekm;
-    const T c2i = T(1) / (cm * cm);
-    for (int l = 0; l < ns; ++l) {
-      al[l] = gamma * T(kRuD) / (T)c_mix.mw[l] * tm - (gamma - 1) * hi[l];
-      al[l] *= c2i;
-    }
-    // The species columns of the five flow rows of L are cs_l * al[q] (cs = 1/2, -kx, -ky, -kz, 1/2):
-    // their products with the split fluxes share one sum per stencil node, formed once for all rows.
-    T sp[7], sm[7];
-    for (int m = 0; m < 7; ++m) {
-      T a = 0, bq = 0;
-      for (int q = 0; q < ns; ++q) {
-        a += al[q] * FP(m, 5 + q);
-        bq += al[q] * FM(m + 1, 5 + q);
-      }
-      sp[m] = a;
-      sm[m] = bq;
-    }
-    T fch[Spec<NS>::A + 5];
+    const T alpha = gm1 * ekm, icm = cm * c2i, h2 = half * c2i;
+    const T hc = hm - cm * cm / gm1;
+    T fc[5] = {T(0), T(0), T(0), T(0), T(0)};
+    // The staged values are read again for every row (the empty asm keeps the compiler from holding them
+    // across the rows: their 70 values do not fit the registers).
+#pragma unroll
     for (int l = 0; l < 5; ++l) {
-      T cs = half, L[5];
+      asm volatile("" ::: "memory");
+      // row l of L over the flow variables, and column l of R
+      T cs = half, L[5], R[5];
       if (l == 0) {
-        L[0] = (alpha + Ukb * cm) * c2i * half;
-        L[1] = -(gm1 * um + kx * cm) * c2i * half;
-        L[2] = -(gm1 * vm_ + ky * cm) * c2i * half;
-        L[3] = -(gm1 * wm + kz * cm) * c2i * half;
-        L[4] = gm1 * c2i * half;
+        L[0] = (alpha + Ukb * cm) * h2;
+        L[1] = -(gm1 * um + kx * cm) * h2;
+        L[2] = -(gm1 * vm_ + ky * cm) * h2;
+        L[3] = -(gm1 * wm + kz * cm) * h2;
+        L[4] = gm1 * h2;
+        R[0] = T(1); R[1] = um - kx * cm; R[2] = vm_ - ky * cm; R[3] = wm - kz * cm; R[4] = hm - Ukb * cm;
       } else if (l == 1) {
         cs = -kx;
-        L[0] = kx * (1 - alpha * c2i) - (kz * vm_ - ky * wm) / cm;
+        L[0] = kx * (1 - alpha * c2i) - (kz * vm_ - ky * wm) * icm;
         L[1] = kx * gm1 * um * c2i;
         L[2] = (kx * gm1 * vm_ + kz * cm) * c2i;
         L[3] = (kx * gm1 * wm - ky * cm) * c2i;
         L[4] = -kx * gm1 * c2i;
+        R[0] = kx; R[1] = kx * um; R[2] = kx * vm_ + kz * cm; R[3] = kx * wm - ky * cm;
+        R[4] = kx * hc + (kz * vm_ - ky * wm) * cm;
       } else if (l == 2) {
         cs = -ky;
-        L[0] = ky * (1 - alpha * c2i) - (kx * wm - kz * um) / cm;
+        L[0] = ky * (1 - alpha * c2i) - (kx * wm - kz * um) * icm;
         L[1] = (ky * gm1 * um - kz * cm) * c2i;
         L[2] = ky * gm1 * vm_ * c2i;
         L[3] = (ky * gm1 * wm + kx * cm) * c2i;
         L[4] = -ky * gm1 * c2i;
+        R[0] = ky; R[1] = ky * um - kz * cm; R[2] = ky * vm_; R[3] = ky * wm + kx * cm;
+        R[4] = ky * hc + (kx * wm - kz * um) * cm;
       } else if (l == 3) {
         cs = -kz;
-        L[0] = kz * (1 - alpha * c2i) - (ky * um - kx * vm_) / cm;
+        L[0] = kz * (1 - alpha * c2i) - (ky * um - kx * vm_) * icm;
         L[1] = (kz * gm1 * um + ky * cm) * c2i;
         L[2] = (kz * gm1 * vm_ - kx * cm) * c2i;
         L[3] = kz * gm1 * wm * c2i;
         L[4] = -kz * gm1 * c2i;
+        R[0] = kz; R[1] = kz * um + ky * cm; R[2] = kz * vm_ - kx * cm; R[3] = kz * wm;
+        R[4] = kz * hc + (ky * um - kx * vm_) * cm;
       } else {
-        L[0] = (alpha - Ukb * cm) * c2i * half;
-        L[1] = -(gm1 * um - kx * cm) * c2i * half;
-        L[2] = -(gm1 * vm_ - ky * cm) * c2i * half;
-        L[3] = -(gm1 * wm - kz * cm) * c2i * half;
-        L[4] = gm1 * c2i * half;
+        L[0] = (alpha - Ukb * cm) * h2;
+        L[1] = -(gm1 * um - kx * cm) * h2;
+        L[2] = -(gm1 * vm_ - ky * cm) * h2;
+        L[3] = -(gm1 * wm - kz * cm) * h2;
+        L[4] = gm1 * h2;
+        R[0] = T(1); R[1] = um + kx * cm; R[2] = vm_ + ky * cm; R[3] = wm + kz * cm; R[4] = hm + Ukb * cm;
       }
       T vp[7], vmn[7];
+#pragma unroll
       for (int m = 0; m < 7; ++m) {
-        T a = 0, bq = 0;
+        vp[m] = cs * sp[m];
+        vmn[m] = cs * sm[m];
+#pragma unroll
         for (int q = 0; q < 5; ++q) {
-          a += L[q] * FP(m, q);
-          bq += L[q] * FM(m + 1, q);
+          vp[m] += L[q] * FP(m, q);
+          vmn[m] += L[q] * FM(m, q);
         }
-        vp[m] = a + cs * sp[m];
-        vmn[m] = bq + cs * sm[m];
       }
-      fch[l] = fvs_weno7(vp, vmn, eps);
+      const T fch = fvs_weno7(vp, vmn, eps);
+#pragma unroll
+      for (int q = 0; q < 5; ++q) fc[q] += R[q] * fch;
     }
-    for (int l = 0; l < ns; ++l) {
-      T vp[7], vmn[7];
-      for (int m = 0; m < 7; ++m) {
-        vp[m] = -svm[l] * FP(m, 0) + FP(m, 5 + l);
-        vmn[m] = -svm[l] * FM(m + 1, 0) + FM(m + 1, 5 + l);
-      }
-      fch[5 + l] = fvs_weno7(vp, vmn, eps);
+    // species fields; fc[0] is also the factor of the mass fractions in their fluxes
+    T p0[7], m0[7];
+#pragma unroll
+    for (int m = 0; m < 7; ++m) {
+      p0[m] = FP(m, 0);
+      m0[m] = FM(m, 0);
     }
-    fc[0] = fch[0] + kx * fch[1] + ky * fch[2] + kz * fch[3] + fch[4];
-    fc[1] = (um - kx * cm) * fch[0] + kx * um * fch[1] + (ky * um - kz * cm) * fch[2] + (kz * um + ky * cm) * fch[3] +
-            (um + kx * cm) * fch[4];
-    fc[2] = (vm_ - ky * cm) * fch[0] + (kx * vm_ + kz * cm) * fch[1] + ky * vm_ * fch[2] +
-            (kz * vm_ - kx * cm) * fch[3] + (vm_ + ky * cm) * fch[4];
-    fc[3] = (wm - kz * cm) * fch[0] + (kx * wm - ky * cm) * fch[1] + (ky * wm + kx * cm) * fch[2] + kz * wm * fch[3] +
-            (wm + kz * cm) * fch[4];
-    const T hc = hm - cm * cm / gm1;
-    fc[4] = (hm - Ukb * cm) * fch[0] + (kx * hc + (kz * vm_ - ky * wm) * cm) * fch[1] +
-            (ky * hc + (kx * wm - kz * um) * cm) * fch[2] + (kz * hc + (ky * um - kx * vm_) * cm) * fch[3] +
-            (hm + Ukb * cm) * fch[4];
     T add = 0;
-    const T ca = fch[0] + kx * fch[1] + ky * fch[2] + kz * fch[3] + fch[4];
+#pragma unroll 1
     for (int l = 0; l < ns; ++l) {
-      fc[5 + l] = svm[l] * ca + fch[l + 5];
-      add += al[l] * fch[l + 5];
+      const T sv = roe(5 + l);
+      T vp[7], vmn[7];
+#pragma unroll
+      for (int m = 0; m < 7; ++m) {
+        vp[m] = FP(m, 5 + l) - sv * p0[m];
+        vmn[m] = FM(m, 5 + l) - sv * m0[m];
+      }
+      const T fch = fvs_weno7(vp, vmn, eps);
+      add += FC(t, 5 + l) * fch;
+      FC(t, 5 + l) = sv * fc[0] + fch;
     }
     fc[4] -= add * cm * cm / gm1;
+#pragma unroll
+    for (int l = 0; l < 5; ++l) FC(t, l) = fc[l];
   }
-  __syncthreads();  // every thread is done with the staged fluxes: reuse them for the face fluxes
-  T *fcs = fsm;  // [TD][TXL][nv]
-  for (int l = 0; l < nv; ++l) fcs[((long long)t * TXL + lane) * nv + l] = fc[l];
   __syncthreads();
   if (face_ok && t >= 1) {
     const long long q = DIR == 0 ? b.iq(n, j0, k0) : DIR == 1 ? b.iq(i0, n, k0) : b.iq(i0, j0, n);
-    for (int l = 0; l < nv; ++l)
-      dq[l * b.n + q] -= (double)(fc[l] - fcs[((long long)(t - 1) * TXL + lane) * nv + l]);
+#pragma unroll
+    for (int l = 0; l < nv; ++l) dq[l * b.n + q] -= (double)(FC(t, l) - FC(t - 1, l));
   }
 }
 
