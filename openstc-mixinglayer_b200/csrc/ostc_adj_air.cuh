@@ -28,19 +28,19 @@ template <> __device__ __forceinline__ Dual tmax<Dual>(Dual a, Dual b) { return 
 
 // The FP64 weight combination (same products of the D_k) on dual numbers.
 template <> struct WenoComb<Dual> {
-  static __device__ __forceinline__ void c3(Dual d0, Dual d1, Dual d2, Dual D0, Dual D1, Dual D2, Dual tau, Dual v0,
-                                            Dual v1, Dual v2, Dual &num, Dual &den) {
-    const Dual w0 = d0 * (D0 + tau) * (D1 * D2), w1 = d1 * (D1 + tau) * (D0 * D2), w2 = d2 * (D2 + tau) * (D0 * D1);
-    num = w0 * v0 + w1 * v1 + w2 * v2;
-    den = w0 + w1 + w2;
+  static __device__ __forceinline__ void c3(const Dual *d, const Dual *D, Dual tau, const Dual *q, Dual lin, Dual &num,
+                                            Dual &den) {
+    const Dual e0 = d[0] * (D[1] * D[2]), a = D[0] * D[2], e1 = d[1] * a, e2 = d[2] * (D[0] * D[1]);
+    const Dual P = a * D[1];
+    num = P * lin + tau * (e0 * q[0] + e1 * q[1] + e2 * q[2]);
+    den = P + tau * (e0 + e1 + e2);
   }
-  static __device__ __forceinline__ void c4(Dual d0, Dual d1, Dual d2, Dual d3, Dual D0, Dual D1, Dual D2, Dual D3,
-                                            Dual tau, Dual v0, Dual v1, Dual v2, Dual v3, Dual &num, Dual &den) {
-    const Dual a = D0 * D1, b = D2 * D3;
-    const Dual w0 = d0 * (D0 + tau) * (D1 * b), w1 = d1 * (D1 + tau) * (D0 * b);
-    const Dual w2 = d2 * (D2 + tau) * (a * D3), w3 = d3 * (D3 + tau) * (a * D2);
-    num = w0 * v0 + w1 * v1 + w2 * v2 + w3 * v3;
-    den = w0 + w1 + w2 + w3;
+  static __device__ __forceinline__ void c4(const Dual *d, const Dual *D, Dual tau, const Dual *q, Dual lin, Dual &num,
+                                            Dual &den) {
+    const Dual a = D[0] * D[1], b = D[2] * D[3], P = a * b;
+    const Dual e0 = d[0] * (D[1] * b), e1 = d[1] * (D[0] * b), e2 = d[2] * (D[3] * a), e3 = d[3] * (D[2] * a);
+    num = P * lin + tau * (e0 * q[0] + e1 * q[1] + e2 * q[2] + e3 * q[3]);
+    den = P + tau * (e0 + e1 + e2 + e3);
   }
   static __device__ __forceinline__ void finish(Dual nm, Dual dm, Dual np, Dual dp, Dual &vm, Dual &vp) {
     vm = nm / dm;
