@@ -877,8 +877,8 @@ int vjp_air(ostc_ctx *ctx, int block, int slot, unsigned mask, double *out) {
   BlockRes &B = ctx->blk[block];
   const DevBlock &b = B.db;
   const long long P = b.plane;
-  double *acv = B.adj;
-  CK(cudaMemsetAsync(acv, 0, (size_t)5 * P * sizeof(double), ctx->stream));
+  double *acv = B.adj, *apr = acv + 5 * P;  // adjoints of cv, and of u, v, w, T
+  CK(cudaMemsetAsync(acv, 0, (size_t)9 * P * sizeof(double), ctx->stream));
   const DevState in = state_of(B, slot);
   if (mask & OSTC_TERM_INVISCID) {
     const int ng = ctx->der.ngg, rs = ctx->der.riemann;
@@ -897,13 +897,14 @@ int vjp_air(ostc_ctx *ctx, int block, int slot, unsigned mask, double *out) {
     const long long fx = (long long)(b.mx + 1) * b.my * b.mz, fy = (long long)b.mx * (b.my + 1) * b.mz;
     if (b.mz > 1) {
       const long long fz = (long long)b.mx * b.my * (b.mz + 1);
-      k_adj_air_visc<0, true><<<grid_for(ctx, fx, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, acv);
-      k_adj_air_visc<1, true><<<grid_for(ctx, fy, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, acv);
-      k_adj_air_visc<2, true><<<grid_for(ctx, fz, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, acv);
+      k_adj_air_visc<0, true><<<grid_for(ctx, fx, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, apr);
+      k_adj_air_visc<1, true><<<grid_for(ctx, fy, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, apr);
+      k_adj_air_visc<2, true><<<grid_for(ctx, fz, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, apr);
     } else {
-      k_adj_air_visc<0, false><<<grid_for(ctx, fx, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, acv);
-      k_adj_air_visc<1, false><<<grid_for(ctx, fy, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, acv);
+      k_adj_air_visc<0, false><<<grid_for(ctx, fx, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, apr);
+      k_adj_air_visc<1, false><<<grid_for(ctx, fy, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, pr, apr);
     }
+    k_adj_air_prim<<<grid_for(ctx, P, 128), 128, 0, ctx->stream>>>(b, in, apr, acv);
   }
   for (auto it = ctx->order.rbegin(); it != ctx->order.rend(); ++it) {
     if (it->first != block) continue;
