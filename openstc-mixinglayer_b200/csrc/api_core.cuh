@@ -100,6 +100,26 @@ int ostc_create(const char *setup_txt, const char *input_dir, int device, ostc_c
         m.third_body[r][i] = c.third_body[r * c.n_spec + i];
       }
     }
+    m.listed = 1;
+    for (int r = 0; r < c.n_reac; ++r) {
+      int nf = 0, nb = 0, nn = 0;
+      for (int i = 0; i < c.n_spec; ++i) {
+        for (int q = 0; q < m.stoi_f[r][i]; ++q, ++nf)
+          if (nf < kMol) m.mol_f[r][nf] = (signed char)i;
+        for (int q = 0; q < m.stoi_b[r][i]; ++q, ++nb)
+          if (nb < kMol) m.mol_b[r][nb] = (signed char)i;
+        if (m.stoi_f[r][i] == m.stoi_b[r][i]) continue;
+        if (nn < kNet) {
+          m.net[r][nn] = (signed char)i;
+          m.nu[r][nn] = m.stoi_b[r][i] - m.stoi_f[r][i];
+        }
+        ++nn;
+      }
+      if (nf > kMol || nb > kMol || nn > kNet) m.listed = 0;
+      m.n_f[r] = (signed char)nf;
+      m.n_b[r] = (signed char)nb;
+      m.n_net[r] = (signed char)nn;
+    }
     ctx->mixture = true;
     ctx->nv = 5 + c.n_spec;
     ctx->der.n_spec = c.n_spec;

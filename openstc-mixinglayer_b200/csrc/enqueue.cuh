@@ -183,18 +183,29 @@ void launch_mix_inviscid(ostc_ctx *ctx, BlockRes &B, DevState in) {
 }
 template <int NS>
 void launch_mix_source_t(ostc_ctx *ctx, BlockRes &B, DevState in, bool chem) {
-  k_mix_source<NS><<<grid_for(ctx, B.db.n, 128), 128, 0, ctx->stream>>>(B.db, in, B.dq, ctx->nv, chem ? 1 : 0);
+  const int g = grid_for(ctx, B.db.n, 128);
+  if (ctx->mixtab.listed)
+    k_mix_source<NS, true><<<g, 128, chem_columns(ctx->der.n_spec, false) * 128 * sizeof(double), ctx->stream>>>(
+        B.db, in, B.dq, ctx->nv, chem ? 1 : 0);
+  else
+    k_mix_source<NS, false><<<g, 128, 0, ctx->stream>>>(B.db, in, B.dq, ctx->nv, chem ? 1 : 0);
 }
 void launch_mix_source(ostc_ctx *ctx, BlockRes &B, DevState in, bool chem) {
   if (ctx->der.n_spec == kFixedNS) launch_mix_source_t<kFixedNS>(ctx, B, in, chem);
   else launch_mix_source_t<0>(ctx, B, in, chem);
 }
+template <int NS>
+void launch_chem_epi_t(ostc_ctx *ctx, BlockRes &B, DevState in) {
+  if (ctx->mixtab.listed)
+    k_mix_chem_epi<NS, true><<<grid_for(ctx, B.db.n, 64), 64, chem_columns(ctx->der.n_spec, true) * 64 * sizeof(double),
+                               ctx->stream>>>(B.db, in, B.dq, ctx->d_dt);
+  else
+    k_mix_chem_epi<NS, false><<<grid_for(ctx, B.db.n, 128), 128, 0, ctx->stream>>>(B.db, in, B.dq, ctx->d_dt);
+}
 void launch_chem_epi(ostc_ctx *ctx, BlockRes &B, DevState in) {
   long tok = begin_t(ctx, "chem_implicit");
-  if (ctx->der.n_spec == kFixedNS)
-    k_mix_chem_epi<kFixedNS><<<grid_for(ctx, B.db.n, 128), 128, 0, ctx->stream>>>(B.db, in, B.dq, ctx->d_dt);
-  else
-    k_mix_chem_epi<0><<<grid_for(ctx, B.db.n, 128), 128, 0, ctx->stream>>>(B.db, in, B.dq, ctx->d_dt);
+  if (ctx->der.n_spec == kFixedNS) launch_chem_epi_t<kFixedNS>(ctx, B, in);
+  else launch_chem_epi_t<0>(ctx, B, in);
   end_t(ctx, tok);
 }
 
@@ -641,6 +652,14 @@ bool set_mix_attrs(int nv) {
   OSTC_FSET(double)
   OSTC_FSET(float)
 #undef OSTC_FSET
+  const int ns = nv - 5;
+  if (ns > 0) {
+    const size_t src = chem_columns(ns, false) * 128 * sizeof(double), epi = chem_columns(ns, true) * 64 * sizeof(double);
+    set((const void *)k_mix_source<0, true>, src);
+    set((const void *)k_mix_source<kFixedNS, true>, src);
+    set((const void *)k_mix_chem_epi<0, true>, epi);
+    set((const void *)k_mix_chem_epi<kFixedNS, true>, epi);
+  }
   set((const void *)k_adj_fvs<0, 0>, adj_fvs_smem_bytes<0>(nv));
   set((const void *)k_adj_fvs<1, 0>, adj_fvs_smem_bytes<1>(nv));
   set((const void *)k_adj_fvs<2, 0>, adj_fvs_smem_bytes<2>(nv));

@@ -11,6 +11,7 @@ namespace ostc {
 constexpr int kMS = 16;  // species capacity of the device tables
 constexpr int kMR = 64;  // reaction capacity
 constexpr int kMV = 5 + kMS;
+constexpr int kMol = 4, kNet = 6;  // molecules a side and species of a reaction in the lists of MixTables
 constexpr double kPatmD = 101325.0;
 
 // Species count as a compile-time constant: NS > 0 instantiates for exactly NS species (arrays in
@@ -44,6 +45,11 @@ struct MixTables {
   double lj_pow[kMS], kbe_pow[kMS][kMS], inv_diff[kMS][kMS];
   int label[kMR], rev_type[kMR], order[kMR];
   signed char stoi_f[kMR][kMS], stoi_b[kMR][kMS];
+  // the same by molecules: species of every forward / backward molecule of a reaction (kMol at most) and
+  // its net coefficients by species (kNet at most); listed = 0 if some reaction has more
+  int listed;
+  signed char n_f[kMR], n_b[kMR], n_net[kMR], mol_f[kMR][kMol], mol_b[kMR][kMol], net[kMR][kNet];
+  double nu[kMR][kNet];
   double A[kMR], b[kMR], Ea[kMR], A2[kMR], b2[kMR], Ea2[kMR], third_body[kMR][kMS];
   double troe_alpha[kMR], troe_t3[kMR], troe_t1[kMR], troe_t2[kMR];
 };
@@ -255,14 +261,13 @@ __device__ __forceinline__ T ipow(T x, int n) {
   }
 }
 
-// Forward and backward rate constants of reaction r (forward_reaction_rate, backward_reaction_rate,
-// FiniteRateChem.cu:60-150) at T (with ln T, 1/T), third-body concentration sum cc and, where the
-// equilibrium constant is used, g = g_k / (Ru T) of every species.  Irreversible: kb = 0; the
-// equilibrium constant for every other type but 2 when any reaction needs it (it also overwrites
-// REV coefficients); else the REV Arrhenius coefficients (times the third-body sum for type 4).
-template <int NS, typename T>
-__device__ __forceinline__ void reaction_rates(int r, T t, T lt, T ti, T cc, const T *g, T &kf_out, T &kb_out) {
-  const int ns = OSTC_NS;
+__device__ __forceinline__ double texp10(double x) { return exp10(x); }
+__device__ __forceinline__ Dual texp10(const Dual &x) { return pow(10.0, x); }
+
+// Forward rate constant of reaction r (forward_reaction_rate, FiniteRateChem.cu:60-102) at T (with ln T,
+// 1/T) and the third-body concentration sum cc.
+template <typename T>
+__device__ __forceinline__ T reaction_kf(int r, T t, T lt, T ti, T cc) {
   const int ty = c_mix.label[r];
   T kf = arrhenius(lt, ti, c_mix.A[r], c_mix.b[r], c_mix.Ea[r]);
   if (ty == 3) {
@@ -281,25 +286,112 @@ __device__ __forceinline__ void reaction_rates(int r, T t, T lt, T ti, T cc, con
       const T cq = -0.4 - 0.67 * lfc, nq = 0.75 - 1.27 * lfc;
       const T lpr = log10(pr);
       const T tmp = (lpr + cq) / (nq - 0.14 * (lpr + cq));
-      F = pow(10.0, lfc / (1.0 + tmp * tmp));
+      F = texp10(lfc / (1.0 + tmp * tmp));
     }
     kf = kf * pr / (1.0 + pr) * F;
   }
-  T kb = 0;
-  if (ty == 0) {
-    kb = 0;
-  } else if (ty != 2 && c_mix.use_gibbs) {
-    T dg = 0;
-    for (int l = 0; l < ns; ++l) dg += g[l] * (c_mix.stoi_b[r][l] - c_mix.stoi_f[r][l]);
-    const T temp_t = kPatmD / kRuD * 1e-3 / t;
-    const T kc = ipow(temp_t, c_mix.order[r]) * exp(-dg);
-    kb = kf / kc;
-  } else if (c_mix.rev_type[r] == 1) {
-    kb = arrhenius(lt, ti, c_mix.A2[r], c_mix.b2[r], c_mix.Ea2[r]);
-    if (ty == 4) kb *= cc;
+  return kf;
+}
+
+// Backward rate constant (backward_reaction_rate, FiniteRateChem.cu:104-150), dg = sum (nu_b - nu_f) g / (Ru T)
+// where the equilibrium constant is used.  Irreversible: 0; the equilibrium constant for every other type
+// but 2 when any reaction needs it (it also overwrites REV coefficients); else the REV Arrhenius
+// coefficients (times the third-body sum for type 4).
+template <typename T>
+__device__ __forceinline__ T reaction_kb(int r, T lt, T ti, T cc, T kf, T dg) {
+  const int ty = c_mix.label[r];
+  if (ty == 0) return T(0.0);
+  if (ty != 2 && c_mix.use_gibbs) {
+    // kf / (temp_t^order exp(-dg)), temp_t = p_atm / (Ru T) 1e-3
+    const T q = kf * exp(dg), temp_t = (kPatmD / kRuD * 1e-3) * ti;
+    switch (c_mix.order[r]) {
+      case 0: return q;
+      case -1: return q * temp_t;
+      case 1: return q / temp_t;
+      default: return q / ipow(temp_t, c_mix.order[r]);
+    }
   }
+  if (c_mix.rev_type[r] == 1) {
+    const T kb = arrhenius(lt, ti, c_mix.A2[r], c_mix.b2[r], c_mix.Ea2[r]);
+    return ty == 4 ? kb * cc : kb;
+  }
+  return T(0.0);
+}
+
+// Both rate constants of reaction r; g: g_k / (Ru T) of every species.
+template <int NS, typename T>
+__device__ __forceinline__ void reaction_rates(int r, T t, T lt, T ti, T cc, const T *g, T &kf_out, T &kb_out) {
+  const T kf = reaction_kf<T>(r, t, lt, ti, cc);
+  T dg = 0;
+  if (c_mix.use_gibbs && c_mix.label[r] != 0 && c_mix.label[r] != 2)
+    for (int l = 0; l < OSTC_NS; ++l) dg += g[l] * (double)(c_mix.stoi_b[r][l] - c_mix.stoi_f[r][l]);
   kf_out = kf;
-  kb_out = kb;
+  kb_out = reaction_kb<T>(r, lt, ti, cc, kf, dg);
+}
+
+// The species arrays of one thread in shared memory: element e of `threads` interleaved columns, so that
+// a reaction can address its species by list (a register array cannot be indexed) and consecutive threads
+// stay on consecutive words.
+struct ChemColumn {
+  double *base;
+  int threads;
+  __device__ __forceinline__ double &operator()(int e) const { return base[(long long)e * threads]; }
+};
+// columns: concentrations, Gibbs energies, rates (ns each), and with the Jacobian ns x ns
+__host__ __device__ constexpr int chem_columns(int ns, bool jac) { return 3 * ns + (jac ? ns * ns : 0); }
+
+// finite_rate_chemistry (FiniteRateChem.cu:7-58, rates :60-195) over the reaction lists: omega_k in kg/(m^3 s)
+// into om(k), and with JAC the Jacobian of compute_chem_src_jacobian (:197-217) into jc(m ns + n), in 1/s.
+// Per reaction the sums run over its own species instead of all of them; the rates of a species add its
+// net coefficient times q1 - q2 per reaction (the reference adds creation and destruction apart).
+template <int NS, bool JAC>
+__device__ __forceinline__ void mix_chemistry_listed(double rho, double t, const double *y, ChemColumn c, ChemColumn g,
+                                                     ChemColumn om, ChemColumn jc) {
+  const int ns = OSTC_NS, nr = c_mix.nr;
+  const double lt = log(t), ti = 1.0 / t;
+  for (int l = 0; l < ns; ++l) {
+    c(l) = rho * y[l] * c_mix.imw[l] * 1e-3;
+    om(l) = 0.0;
+  }
+  if (c_mix.use_gibbs) {
+    double gr[Spec<NS>::A];
+    mix_gibbs_rt<NS, double>(t, gr);
+    for (int l = 0; l < ns; ++l) g(l) = gr[l];
+  }
+  if (JAC)
+    for (int e = 0; e < ns * ns; ++e) jc(e) = 0.0;
+#pragma unroll 1
+  for (int r = 0; r < nr; ++r) {
+    double cc = 0;
+    if (c_mix.label[r] >= 4)
+      for (int l = 0; l < ns; ++l) cc += c(l) * c_mix.third_body[r][l];
+    const int nf = c_mix.n_f[r], nb = c_mix.n_b[r], nn = c_mix.n_net[r];
+    double dg = 0;
+    if (c_mix.use_gibbs)
+      for (int e = 0; e < nn; ++e) dg += c_mix.nu[r][e] * g(c_mix.net[r][e]);
+    double q1 = reaction_kf<double>(r, t, lt, ti, cc);
+    double q2 = reaction_kb<double>(r, lt, ti, cc, q1, dg);
+    for (int e = 0; e < nf; ++e) q1 *= c(c_mix.mol_f[r][e]);
+    for (int e = 0; e < nb; ++e) q2 *= c(c_mix.mol_b[r][e]);
+    const double q = q1 - q2;
+    for (int e = 0; e < nn; ++e) {
+      const int m = c_mix.net[r][e];
+      const double nu = c_mix.nu[r][e];
+      om(m) += nu * q;
+      if (JAC) {
+        for (int a = 0; a < nf; ++a) jc(m * ns + c_mix.mol_f[r][a]) += nu * q1;
+        for (int a = 0; a < nb; ++a) jc(m * ns + c_mix.mol_b[r][a]) -= nu * q2;
+      }
+    }
+  }
+  for (int l = 0; l < ns; ++l) om(l) = om(l) * (c_mix.mw[l] * 1e+3);
+  if (JAC) {
+    for (int n = 0; n < ns; ++n) {
+      const bool live = y[n] > 1e-25;
+      const double inv = live ? 1.0 / (rho * y[n]) : 0.0;
+      for (int m = 0; m < ns; ++m) jc(m * ns + n) = c_mix.mw[m] * (live ? jc(m * ns + n) * inv : 0.0) * 1e+3;
+    }
+  }
 }
 
 // finite_rate_chemistry (FiniteRateChem.cu:7-58, rates :60-195): omega_k in kg/(m^3 s) at one node.
@@ -373,6 +465,48 @@ __device__ __forceinline__ void mix_chemistry(T rho, T t, const T *y, T *omega, 
 #pragma unroll
       for (int m = 0; m < ns; ++m) jac[m * ns + n] = c_mix.mw[m] * (live ? jac[m * ns + n] * inv : 0.0) * 1e+3;
     }
+  }
+}
+
+// solve_chem_system (FiniteRateChem.cu:302-357) on columns: LU with partial pivoting of the ns x ns matrix
+// a in place, right-hand side x solved in place.  The pivot search and the row exchange index the matrix
+// by a value of their own per thread, which registers cannot; the row at hand is held in registers.
+template <int NS>
+__device__ __forceinline__ void mix_lu_solve_columns(ChemColumn a, ChemColumn x) {
+  const int dim = OSTC_NS;
+#pragma unroll 1
+  for (int n = 0; n < dim; ++n) {
+    int ik = n;
+    double best = fabs(a(n * dim + n));
+    for (int m = n + 1; m < dim; ++m) {
+      const double v = fabs(a(m * dim + n));
+      if (v > best) {
+        best = v;
+        ik = m;
+      }
+    }
+    double row[Spec<NS>::A];
+    for (int t = 0; t < dim; ++t) {
+      row[t] = a(ik * dim + t);
+      if (ik != n) a(ik * dim + t) = a(n * dim + t);
+      a(n * dim + t) = row[t];
+    }
+    const double xn = x(ik);
+    if (ik != n) x(ik) = x(n);
+    x(n) = xn;
+    const double ip = 1.0 / a(n * dim + n);
+    for (int m = n + 1; m < dim; ++m) {
+      const double f = a(m * dim + n) * ip;
+      for (int t = 0; t < dim; ++t)
+        if (t > n) a(m * dim + t) -= f * row[t];
+      x(m) -= f * xn;
+    }
+  }
+#pragma unroll 1
+  for (int m = dim - 1; m >= 0; --m) {
+    double v = x(m);
+    for (int t = m + 1; t < dim; ++t) v -= a(m * dim + t) * x(t);
+    x(m) = v / a(m * dim + m);
   }
 }
 
