@@ -435,8 +435,7 @@ __device__ __forceinline__ void mix_visc_face(const DevBlock &b, const DevState 
   T m[9];
   for (int r = 0; r < 9; ++r) m[r] = (T)(0.5 * (b.met[r * P + p0] + b.met[r * P + p1]));
   // gradient of plane B at the face: 2-point normal difference, 4-point averages across
-  auto grad = [&](const double *B, T *out) {
-    T g[3];
+  auto diff = [&](const double *B, T *g) {
     for (int c = 0; c < 3; ++c) {
       if (c == d) {
         g[c] = (T)(B[p1] - B[p0]);
@@ -447,26 +446,44 @@ __device__ __forceinline__ void mix_visc_face(const DevBlock &b, const DevState 
         g[c] = (T)(0.25 * (B[p0 + a] - B[p0 - a] + B[p1 + a] - B[p1 - a]));
       }
     }
+  };
+  auto grad = [&](const double *B, T *out) {
+    T g[3];
+    diff(B, g);
     out[0] = g[0] * m[0] + g[1] * m[3] + g[2] * m[6];
     out[1] = g[0] * m[1] + g[1] * m[4] + g[2] * m[7];
     out[2] = g[0] * m[2] + g[1] * m[5] + g[2] * m[8];
   };
-  T gu[3], gv[3], gw[3], gt[3];
-  grad(s.bv + P, gu);
-  grad(s.bv + 2 * P, gv);
-  grad(s.bv + 3 * P, gw);
-  grad(s.bv + 5 * P, gt);
-  const T mul = (T)(0.5 * (s.mul[p0] + s.mul[p1]));
-  const T txx = mul * (4 * gu[0] - 2 * gv[1] - 2 * gw[2]) / T(3);
-  const T tyy = mul * (4 * gv[1] - 2 * gu[0] - 2 * gw[2]) / T(3);
-  const T tzz = mul * (4 * gw[2] - 2 * gu[0] - 2 * gv[1]) / T(3);
-  const T txy = mul * (gu[1] + gv[0]);
-  const T txz = mul * (gu[2] + gw[0]);
-  const T tyz = mul * (gv[2] + gw[1]);
   const double j0 = b.jac[p0], j1 = b.jac[p1];
   const T nx = (T)(0.5 * (b.met[(d * 3 + 0) * P + p0] * j0 + b.met[(d * 3 + 0) * P + p1] * j1));
   const T ny = (T)(0.5 * (b.met[(d * 3 + 1) * P + p0] * j0 + b.met[(d * 3 + 1) * P + p1] * j1));
   const T nz = (T)(0.5 * (b.met[(d * 3 + 2) * P + p0] * j0 + b.met[(d * 3 + 2) * P + p1] * j1));
+  // T and the mass fractions enter by their derivative along the face normal alone: the weight of each
+  // difference is the normal's product with that row of the mean metric.  Where the face normal is
+  // orthogonal to the other two rows (every rectilinear grid) the cross differences have weight zero and
+  // are not formed: 2 loads a field instead of 10.  192 x 96 x 48, three sweeps: 0.91 -> 0.69 ms (bound by
+  // the latency of its loads; 24 % of HBM).
+  T wn[3];
+  for (int c = 0; c < 3; ++c) wn[c] = nx * m[c * 3] + ny * m[c * 3 + 1] + nz * m[c * 3 + 2];
+  const bool cross = wn[(d + 1) % 3] != T(0) || wn[(d + 2) % 3] != T(0);
+  auto normal = [&](const double *B) -> T {
+    if (!cross) return wn[d] * (T)(B[p1] - B[p0]);
+    T g[3];
+    diff(B, g);
+    return wn[0] * g[0] + wn[1] * g[1] + wn[2] * g[2];
+  };
+  T gu[3], gv[3], gw[3];
+  grad(s.bv + P, gu);
+  grad(s.bv + 2 * P, gv);
+  grad(s.bv + 3 * P, gw);
+  const T mul = (T)(0.5 * (s.mul[p0] + s.mul[p1]));
+  const T m3 = mul * T(1.0 / 3.0);
+  const T txx = m3 * (4 * gu[0] - 2 * gv[1] - 2 * gw[2]);
+  const T tyy = m3 * (4 * gv[1] - 2 * gu[0] - 2 * gw[2]);
+  const T tzz = m3 * (4 * gw[2] - 2 * gu[0] - 2 * gv[1]);
+  const T txy = mul * (gu[1] + gv[0]);
+  const T txz = mul * (gu[2] + gw[0]);
+  const T tyz = mul * (gv[2] + gw[1]);
   fv[0] = 0;
   fv[1] = nx * txx + ny * txy + nz * txz;
   fv[2] = nx * txy + ny * tyy + nz * tyz;
@@ -475,7 +492,7 @@ __device__ __forceinline__ void mix_visc_face(const DevBlock &b, const DevState 
   const T vm = (T)(0.5 * (s.bv[2 * P + p0] + s.bv[2 * P + p1]));
   const T wm = (T)(0.5 * (s.bv[3 * P + p0] + s.bv[3 * P + p1]));
   const T cond = (T)(0.5 * (s.cond[p0] + s.cond[p1]));
-  fv[4] = um * fv[1] + vm * fv[2] + wm * fv[3] + cond * (nx * gt[0] + ny * gt[1] + nz * gt[2]);
+  fv[4] = um * fv[1] + vm * fv[2] + wm * fv[3] + cond * normal(s.bv + 5 * P);
   const int ns = OSTC_NS;
   T dif[Spec<NS>::A], yk[Spec<NS>::A], ddf[Spec<NS>::A];
   T sgw = 0, srdy = 0, corr = 0, mwt = 0;
@@ -483,13 +500,11 @@ __device__ __forceinline__ void mix_visc_face(const DevBlock &b, const DevState 
     const double *Y = s.sv + (long long)l * P;
     yk[l] = (T)(0.5 * (Y[p0] + Y[p1]));
     dif[l] = (T)(0.5 * (s.rhod[l * P + p0] + s.rhod[l * P + p1]));
-    T gy[3];
-    grad(Y, gy);
-    const T gdy = nx * gy[0] + ny * gy[1] + nz * gy[2];
+    const T gdy = normal(Y);
     ddf[l] = gdy;
     corr += dif[l] * gdy;
-    sgw += gdy / (T)c_mix.mw[l];
-    mwt += yk[l] / (T)c_mix.mw[l];
+    sgw += gdy * (T)c_mix.imw[l];
+    mwt += yk[l] * (T)c_mix.imw[l];
     srdy += dif[l] * yk[l];
   }
   mwt = T(1) / mwt;
