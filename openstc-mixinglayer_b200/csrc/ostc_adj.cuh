@@ -24,115 +24,101 @@ struct DevAdj {
   double *cv, *p, *c, *rho, *vel, *T, *Y, *mu, *lam, *rhod;
 };
 
-// One side of the flux-split WENO7-Z (fvs_weno7_core) with its gradient.  v[0..6] in the orientation
-// of the + side (the - side passes its stencil mirrored, v[j] = vm[6 - j]); returns the side's face
-// value and adds af * d(value)/d(v[j]) to g[j].  The third smoothness indicator reuses the second
-// stencil's second difference, as the forward function does.
+// One side of the flux-split WENO7-Z (fvs_side) and its gradient: v[0..6] upwind first; returns the side's
+// face value and sets g[j] = af d(value) / d v[j].  In the differences fvs_side shares; the third
+// smoothness indicator reuses the second stencil's second difference, as the forward function does.
 __device__ __forceinline__ double weno7_side_bwd(const double *v, double eps, double af, double *g) {
   const double c[4] = {1.0 / 35, 12.0 / 35, 18.0 / 35, 4.0 / 35};
-  const double one6th = 1.0 / 6, one12th = 1.0 / 12;
-  double s1[4], s2[4], s3[4], b[4], q[4], d[4], a[4];
-  s1[0] = one6th * (-2 * v[0] + 9 * v[1] - 18 * v[2] + 11 * v[3]);
-  s2[0] = -v[0] + 4 * v[1] - 5 * v[2] + 2 * v[3];
-  s3[0] = -v[0] + 3 * v[1] - 3 * v[2] + v[3];
-  s1[1] = one6th * (v[1] - 6 * v[2] + 3 * v[3] + 2 * v[4]);
-  s2[1] = v[2] - 2 * v[3] + v[4];
-  s3[1] = -v[1] + 3 * v[2] - 3 * v[3] + v[4];
-  s1[2] = one6th * (-2 * v[2] - 3 * v[3] + 6 * v[4] - v[5]);
-  s2[2] = s2[1];
-  s3[2] = -v[2] + 3 * v[3] - 3 * v[4] + v[5];
-  s1[3] = one6th * (-11 * v[3] + 18 * v[4] - 9 * v[5] + 2 * v[6]);
-  s2[3] = 2 * v[3] - 5 * v[4] + 4 * v[5] - v[6];
-  s3[3] = -v[3] + 3 * v[4] - 3 * v[5] + v[6];
+  const double d2 = v[3] - v[2], d3 = v[4] - v[3];
+  const double e0 = (v[2] - v[1]) - (v[1] - v[0]), e1 = d2 - (v[2] - v[1]), e2 = d3 - d2, e3 = (v[5] - v[4]) - d3;
+  const double e4 = (v[6] - v[5]) - (v[5] - v[4]);
+  const double t0 = e1 - e0, t1 = e2 - e1, t2 = e3 - e2, t3 = e4 - e3;
+  const double mid = d2 + 0.5 * e2;
+  const double s1[4] = {d2 + (0.5 * e1 + (1.0 / 3) * t0), mid - (1.0 / 6) * t1, mid - (1.0 / 6) * t2,
+                        d3 - (0.5 * e3 - (1.0 / 3) * t3)};
+  const double s2[4] = {e1 + t0, e2, e2, e3 - t3};
+  const double s3[4] = {t0, t1, t2, t3};
+  double b[4], id[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) b[k] = fvs_beta7(s1[k], s2[k], s3[k]);
-  q[0] = one12th * (-3 * v[0] + 13 * v[1] - 23 * v[2] + 25 * v[3]);
-  q[1] = one12th * (v[1] - 5 * v[2] + 13 * v[3] + 3 * v[4]);
-  q[2] = one12th * (-v[2] + 7 * v[3] + 7 * v[4] - v[5]);
-  q[3] = one12th * (3 * v[3] + 13 * v[4] - 5 * v[5] + v[6]);
-  const double tau = (b[0] - b[3]) * (b[0] - b[3]);
-  double S = 0, num = 0;
+  {
+    // 1 / (eps + b_k) from one division; their product is at least eps^4, and where that leaves the range
+    // (an eps below 1e-75) each takes its own
+    const double g0 = eps + b[0], g1 = eps + b[1], g2 = eps + b[2], g3 = eps + b[3];
+    const double p01 = g0 * g1, p23 = g2 * g3, P = p01 * p23;
+    if (P > 1e-300) {
+      const double q = 1.0 / P, q01 = p23 * q, q23 = p01 * q;
+      id[0] = g1 * q01;
+      id[1] = g0 * q01;
+      id[2] = g3 * q23;
+      id[3] = g2 * q23;
+    } else {
+      id[0] = 1.0 / g0;
+      id[1] = 1.0 / g1;
+      id[2] = 1.0 / g2;
+      id[3] = 1.0 / g3;
+    }
+  }
+  const double db = b[0] - b[3], tau = db * db;
+  double a[4], q[4], S = 0, num = 0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    d[k] = eps + b[k];
-    a[k] = c[k] + c[k] * tau / (d[k] * d[k]);
+    a[k] = c[k] + c[k] * tau * (id[k] * id[k]);
+    q[k] = 0.5 * s1[k] + (1.0 / 12) * s2[k];
     S += a[k];
     num += a[k] * q[k];
   }
-  const double f = num / S;
-  // reverse
-  double aq[4], ab[4], atau = 0;
+  const double iS = 1.0 / S, f = num * iS, w = af * iS;
+  double a1[4], a2[4], a3[4], ab[4], aq[4], atau = 0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    aq[k] = af * a[k] / S;
-    const double aa = af * (q[k] - f) / S;
-    const double id2 = 1.0 / (d[k] * d[k]);
-    atau += aa * c[k] * id2;
-    ab[k] = -2.0 * aa * c[k] * tau * id2 / d[k];
+    aq[k] = w * a[k];
+    const double aa = w * (q[k] - f) * c[k] * (id[k] * id[k]);
+    atau += aa;
+    ab[k] = -2.0 * aa * tau * id[k];
   }
-  ab[0] += 2.0 * atau * (b[0] - b[3]);
-  ab[3] -= 2.0 * atau * (b[0] - b[3]);
-  double a1[4], a2[4], a3[4];
+  ab[0] += 2.0 * atau * db;
+  ab[3] -= 2.0 * atau * db;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    a1[k] = ab[k] * (2 * s1[k] + s3[k] / 12);
-    a2[k] = ab[k] * (26.0 / 12.0) * s2[k];
-    a3[k] = ab[k] * (2 * (1043.0 / 960) * s3[k] + s1[k] / 12);
+    a1[k] = ab[k] * (2 * s1[k] + (1.0 / 12) * s3[k]) + 0.5 * aq[k];
+    a2[k] = ab[k] * (26.0 / 12.0) * s2[k] + (1.0 / 12) * aq[k];
+    a3[k] = ab[k] * (2 * (1043.0 / 960) * s3[k] + (1.0 / 12) * s1[k]);
   }
-  a2[1] += a2[2];  // the reused second difference
-  // stencil 0: v0..v3
-  g[0] += one6th * -2 * a1[0] - a2[0] - a3[0] + one12th * -3 * aq[0];
-  g[1] += one6th * 9 * a1[0] + 4 * a2[0] + 3 * a3[0] + one12th * 13 * aq[0];
-  g[2] += one6th * -18 * a1[0] - 5 * a2[0] - 3 * a3[0] + one12th * -23 * aq[0];
-  g[3] += one6th * 11 * a1[0] + 2 * a2[0] + a3[0] + one12th * 25 * aq[0];
-  // stencil 1: v1..v4
-  g[1] += one6th * a1[1] - a3[1] + one12th * aq[1];
-  g[2] += one6th * -6 * a1[1] + a2[1] + 3 * a3[1] + one12th * -5 * aq[1];
-  g[3] += one6th * 3 * a1[1] - 2 * a2[1] - 3 * a3[1] + one12th * 13 * aq[1];
-  g[4] += one6th * 2 * a1[1] + a2[1] + a3[1] + one12th * 3 * aq[1];
-  // stencil 2: v2..v5
-  g[2] += one6th * -2 * a1[2] - a3[2] - one12th * aq[2];
-  g[3] += one6th * -3 * a1[2] + 3 * a3[2] + one12th * 7 * aq[2];
-  g[4] += one6th * 6 * a1[2] - 3 * a3[2] + one12th * 7 * aq[2];
-  g[5] += one6th * -1 * a1[2] + a3[2] - one12th * aq[2];
-  // stencil 3: v3..v6
-  g[3] += one6th * -11 * a1[3] + 2 * a2[3] - a3[3] + one12th * 3 * aq[3];
-  g[4] += one6th * 18 * a1[3] - 5 * a2[3] + 3 * a3[3] + one12th * 13 * aq[3];
-  g[5] += one6th * -9 * a1[3] + 4 * a2[3] - 3 * a3[3] + one12th * -5 * aq[3];
-  g[6] += one6th * 2 * a1[3] - a2[3] + a3[3] + one12th * aq[3];
-  return f;
-}
-
-// fvs_weno7 (both sides) reverse: gp[j] += af d/d vp[j], gm[j] += af d/d vm[j]
-__device__ __forceinline__ void weno7_bwd(const double *vp, const double *vm, double eps, double af, double *gp,
-                                          double *gm) {
-  weno7_side_bwd(vp, eps, af, gp);
-  double r[7], gr[7];
-#pragma unroll
-  for (int j = 0; j < 7; ++j) {
-    r[j] = vm[6 - j];
-    gr[j] = 0.0;
-  }
-  weno7_side_bwd(r, eps, af, gr);
-#pragma unroll
-  for (int j = 0; j < 7; ++j) gm[6 - j] += gr[j];
+  const double am = a1[1] + a1[2];
+  const double h0 = (1.0 / 3) * a1[0] + a2[0] + a3[0], h1 = a3[1] - (1.0 / 6) * a1[1], h2 = a3[2] - (1.0 / 6) * a1[2],
+               h3 = (1.0 / 3) * a1[3] - a2[3] + a3[3];  // of the third differences
+  const double k0 = -h0, k1 = 0.5 * a1[0] + a2[0] + h0 - h1, k2 = 0.5 * am + a2[1] + a2[2] + h1 - h2,
+               k3 = a2[3] - 0.5 * a1[3] + h2 - h3, k4 = h3;  // of the second differences
+  const double l0 = -k0, l1 = k0 - k1, l2 = a1[0] + am + k1 - k2, l3 = a1[3] + k2 - k3, l4 = k3 - k4, l5 = k4;  // first
+  g[0] = -l0;
+  g[1] = l0 - l1;
+  g[2] = l1 - l2;
+  g[3] = af + l2 - l3;
+  g[4] = l3 - l4;
+  g[5] = l4 - l5;
+  g[6] = l5;
+  return v[3] + f;
 }
 
 // Reverse of the node's split fluxes F+- = J/2 (Uk Q + p grad k (+ p Uk in energy) +- l0 Q),
 // Uk = (Q1 kx + Q2 ky + Q3 kz) / Q0, l0 = |Uk| + c |grad k| (compute_flux, WENO.cu:697-720):
-// adds to aQ[nv], ap, ac.
+// sets aQ[nv], ap, ac; the adjoints aFp, aFm of F+- are strided by `step`.
+template <int NS>
 __device__ __forceinline__ void fvs_node_bwd(const double *Q, double pk, double c, double k0m, double k1m, double k2m,
-                                             double jac, const double *aFp, const double *aFm, int nv, double *aQ,
+                                             double jac, const double *aFp, const double *aFm, int step, double *aQ,
                                              double &ap, double &ac) {
+  const int nv = 5 + OSTC_NS;
   const double Uk = (Q[1] * k0m + Q[2] * k1m + Q[3] * k2m) / Q[0];
   const double kn = sqrt(k0m * k0m + k1m * k1m + k2m * k2m);
   const double l0 = fabs(Uk) + c * kn;
   const double hj = 0.5 * jac;
   double aUk = 0, al0 = 0;
   const double km[3] = {k0m, k1m, k2m};
+  ap = ac = 0;
   for (int q = 0; q < nv; ++q) {
-    const double S = aFp[q] + aFm[q], D = aFp[q] - aFm[q];
-    aQ[q] += hj * (Uk * S + l0 * D);
+    const double fp = aFp[q * step], fm = aFm[q * step], S = fp + fm, D = fp - fm;
+    aQ[q] = hj * (Uk * S + l0 * D);
     aUk += hj * Q[q] * S;
     al0 += hj * Q[q] * D;
     if (q >= 1 && q <= 3) ap += hj * km[q - 1] * S;
@@ -150,18 +136,16 @@ __device__ __forceinline__ void fvs_node_bwd(const double *Q, double pk, double 
   aQ[0] -= aUk * Uk * iq0;
 }
 
-// d cp_i / dT of the NASA-7 polynomials (0 below t_low, where cp is frozen), per species
+// d cp_i / dT of the NASA-7 polynomials (0 below t_low, where cp is frozen)
+__device__ __forceinline__ double mix_dcp_dt_one(int i, double t) {
+  if (t < c_mix.t_low[i]) return 0.0;
+  const double *a = t < c_mix.t_mid[i] ? c_mix.low[i] : c_mix.high[i];
+  return (a[1] + t * (2 * a[2] + t * (3 * a[3] + t * 4 * a[4]))) * c_mix.ru_mw[i];
+}
 template <int NS>
 __device__ __forceinline__ void mix_dcp_dt(double t, double *dcp) {
 #pragma unroll
-  for (int i = 0; i < OSTC_NS; ++i) {
-    if (t < c_mix.t_low[i]) {
-      dcp[i] = 0.0;
-    } else {
-      const double *a = t < c_mix.t_mid[i] ? c_mix.low[i] : c_mix.high[i];
-      dcp[i] = (a[1] + t * (2 * a[2] + t * (3 * a[3] + t * 4 * a[4]))) * c_mix.ru_mw[i];
-    }
-  }
+  for (int i = 0; i < OSTC_NS; ++i) dcp[i] = mix_dcp_dt_one(i, t);
 }
 
 // Left-eigenvector row l (0..4) of the Roe-averaged mixture eigensystem (WENO.cu:822-898) as the
@@ -267,30 +251,41 @@ __device__ __forceinline__ void fvs_lrow_bwd(int l, const double *AL, double alp
 
 template <int DIR>
 __host__ __device__ constexpr size_t adj_fvs_smem_bytes(int nv) {
-  // F+, F- (recomputed), their adjoints, and the Roe-average adjoints (cv and p) per staged node
-  return (size_t)FvsTile<DIR>::NST * FvsTile<DIR>::TXL * (5 * nv + 1) * sizeof(double);
+  // F+, F- (recomputed) and their adjoints per staged node; per thread alpha_l of L and its adjoint, and the
+  // adjoint of the Roe-averaged mass fraction, per species
+  return ((size_t)FvsTile<DIR>::NST * FvsTile<DIR>::TXL * 4 * nv +
+          (size_t)FvsTile<DIR>::TD * FvsTile<DIR>::TXL * 3 * (nv - 5)) * sizeof(double);
 }
 
 // Reverse of k_fvs: the tile recomputes the staged split fluxes, every face thread turns its face
-// adjoint (from dq_bar of the nodes this tile owns) into adjoints of the staged split fluxes (shared
-// atomics) and of the Roe-averaged face state, and after a barrier every staged node maps its split-
-// flux adjoints back to cv, p and c and adds them to the node planes.
+// adjoint (from dq_bar of the nodes this tile owns) into adjoints of the staged split fluxes and of the
+// Roe-averaged face state, and after a barrier every staged node maps its split-flux adjoints back to cv,
+// p and c and adds them to the node planes.
+// A face adds to the 7 staged nodes of each side's stencil, which its neighbours' faces add to as well.
+// FP64 atomics on shared memory are compare-and-swap loops, and 728 of them a face were most of this
+// kernel's time; instead the threads of the block step through the stencil together (scatter below): at
+// step m every face adds to the node m places along, a different one each, with a barrier between the
+// steps.  The flow rows reach the species' split fluxes with one factor alpha_l times a sum W[m] over the
+// rows, and the species fields reach the density's with a sum Z[m], so those go out once per side.  One
+// pass over the fields: the WENO reverse returns the face value too, which the adjoints of R need.
+// [96 x 64 x 48, 9 species: 2.4-2.6 ms a direction with the atomics; without, and with the tables of
+// k_adj_props, the whole VJP went from 11.6 to 5.0 ms]
 template <int DIR, int NS>
-__global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL) k_adj_fvs(DevBlock b, DevState s,
-                                                                                   const double *__restrict__ dqb,
-                                                                                   int nv, int scheme, DevAdj A) {
-  constexpr int TXL = FvsTile<DIR>::TXL, TD = FvsTile<DIR>::TD, NST = FvsTile<DIR>::NST;
+__global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, 2) k_adj_fvs(DevBlock b, DevState s,
+                                                                                      const double *__restrict__ dqb,
+                                                                                      int nv, int scheme, DevAdj A) {
+  constexpr int TXL = FvsTile<DIR>::TXL, TD = FvsTile<DIR>::TD, NST = FvsTile<DIR>::NST, NN = NST * TXL, NT = TD * TXL;
   extern __shared__ __align__(16) unsigned char adj_smem[];
   if (NS > 0) nv = 5 + NS;
   const int ns = OSTC_NS;
-  double *Fp = reinterpret_cast<double *>(adj_smem);
-  double *Fm = Fp + NST * TXL * nv;
-  double *aFp = Fm + NST * TXL * nv;
-  double *aFm = aFp + NST * TXL * nv;
-  double *aR = aFm + NST * TXL * nv;  // [NST][TXL][nv + 1]
+  double *Fp = reinterpret_cast<double *>(adj_smem);  // [nv][NST][TXL]
+  double *Fm = Fp + NN * nv;
+  double *aFp = Fm + NN * nv;
+  double *aFm = aFp + NN * nv;
+  double *slots = aFm + NN * nv;  // [3][ns][NT]
   const int lane = DIR == 0 ? 0 : (int)threadIdx.x;
   const int t = DIR == 0 ? (int)threadIdx.x : (int)threadIdx.y;
-  const int tid = DIR == 0 ? t : t * TXL + lane;
+  const int tid = t * TXL + lane;
   const long long P = b.plane;
   const int nd = DIR == 0 ? b.mx : DIR == 1 ? b.my : b.mz;
   const int start = (DIR == 0 ? blockIdx.x : blockIdx.y) * (TD - 1);
@@ -309,7 +304,7 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL) k_adj_fv
   auto qid = [&](int n) -> long long {
     return DIR == 0 ? b.iq(n, j0, k0) : DIR == 1 ? b.iq(i0, n, k0) : b.iq(i0, j0, n);
   };
-  for (int e = tid; e < NST * TXL * (3 * nv + 1); e += TD * TXL) aFp[e] = 0.0;
+  for (int e = tid; e < 2 * NN * nv; e += NT) aFp[e] = 0.0;
   if (lane_ok) {
     for (int st = t; st < NST; st += TD) {
       const int n = start - 4 + st;
@@ -323,291 +318,330 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL) k_adj_fv
       const double jac = b.jac[p];
       const double Uk = (Q[1] * k0m + Q[2] * k1m + Q[3] * k2m) / Q[0];
       const double l0 = fabs(Uk) + c * sqrt(k0m * k0m + k1m * k1m + k2m * k2m);
-      double *fp = Fp + ((long long)st * TXL + lane) * nv, *fm = Fm + ((long long)st * TXL + lane) * nv;
+      double *fp = Fp + st * TXL + lane, *fm = Fm + st * TXL + lane;
       for (int l = 0; l < nv; ++l) {
         const double pt = l >= 1 && l <= 3 ? pk * (l == 1 ? k0m : l == 2 ? k1m : k2m) : 0.0;
         const double conv = l == 4 ? Uk * (Q[4] + pk) : Uk * Q[l] + pt;
-        fp[l] = 0.5 * jac * (conv + l0 * Q[l]);
-        fm[l] = 0.5 * jac * (conv - l0 * Q[l]);
+        fp[l * NN] = 0.5 * jac * (conv + l0 * Q[l]);
+        fm[l * NN] = 0.5 * jac * (conv - l0 * Q[l]);
       }
     }
   }
   __syncthreads();
   const int n = start - 1 + t;  // left node of this thread's face
-  const bool face_ok = lane_ok && n < nd;
-  auto FP = [&](int m, int l) -> double { return Fp[((long long)(t + m) * TXL + lane) * nv + l]; };
-  auto FM = [&](int m, int l) -> double { return Fm[((long long)(t + m) * TXL + lane) * nv + l]; };
-  auto AFP = [&](int m, int l) -> double * { return aFp + ((long long)(t + m) * TXL + lane) * nv + l; };
-  auto AFM = [&](int m, int l) -> double * { return aFm + ((long long)(t + m) * TXL + lane) * nv + l; };
-  double afc[Spec<NS>::A + 5];
-  bool any = false;
-  for (int l = 0; l < nv; ++l) {
+  // a face carries an adjoint where this tile owns one of its nodes
+  const bool own_l = lane_ok && n < nd && t >= 1, own_r = lane_ok && t <= TD - 2 && n + 1 < nd;
+  auto afc = [&](int l) -> double {
     double a = 0.0;
-    if (face_ok && t >= 1) a -= dqb[l * b.n + qid(n)];
-    if (face_ok && t <= TD - 2 && n + 1 < nd) a += dqb[l * b.n + qid(n + 1)];
-    afc[l] = a;
-    any = any || a != 0.0;
-  }
-  if (face_ok && any && scheme == 71) {
-    const long long pl = pid(n), pr = pid(n + 1);
-    const double j1 = b.jac[pl], j2 = b.jac[pr];
-    double a[3];
-    for (int q = 0; q < 3; ++q) a[q] = b.met[(DIR * 3 + q) * P + pl] * j1 + b.met[(DIR * 3 + q) * P + pr] * j2;
-    const double eps_ref = 1e-20 * c_mix.weno_eps_scale * 0.25 * (a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
-    const double e1 = eps_ref * c_mix.v_ref * c_mix.v_ref;
-    const double e2 = e1 * c_mix.v_ref * c_mix.v_ref;
-    for (int l = 0; l < nv; ++l) {
-      const double e = (l >= 1 && l <= 3) ? e1 : (l == 4 ? e2 : eps_ref);
-      double vp[7], vm[7], gp[7], gm[7];
-      for (int m = 0; m < 7; ++m) {
-        vp[m] = FP(m, l);
-        vm[m] = FM(m + 1, l);
-        gp[m] = gm[m] = 0.0;
+    if (own_l) a -= dqb[l * b.n + qid(n)];
+    if (own_r) a += dqb[l * b.n + qid(n + 1)];
+    return a;
+  };
+  bool act = false;
+  for (int l = 0; l < nv; ++l) act = act || afc(l) != 0.0;
+  // Side sd (0: +, 1: -) of variable l at stencil place m, upwind first: + nodes t .. t + 6, - nodes t + 7
+  // down to t + 1.
+  auto at = [&](int sd, int m) -> int { return (t + (sd ? 7 - m : m)) * TXL + lane; };
+  auto F = [&](int sd, int l, int m) -> double { return (sd ? Fm : Fp)[l * NN + at(sd, m)]; };
+  // adds w[q] g[m] to the adjoints of variables l0 + q (q < N) of the 7 nodes of side sd
+  auto scatter = [&](int sd, int l0, auto N, const double *w, const double *g) {
+#pragma unroll
+    for (int m = 0; m < 7; ++m) {
+      if (act) {
+        double *p = (sd ? aFm : aFp) + l0 * NN + at(sd, m);
+#pragma unroll
+        for (int q = 0; q < decltype(N)::value; ++q) p[q * NN] += w[q] * g[m];
       }
-      weno7_bwd(vp, vm, e, afc[l], gp, gm);
-      for (int m = 0; m < 7; ++m) {
-        atomicAdd(AFP(m, l), gp[m]);
-        atomicAdd(AFM(m + 1, l), gm[m]);
+      __syncthreads();
+    }
+  };
+  using One = std::integral_constant<int, 1>;
+  using Five = std::integral_constant<int, 5>;
+  const double one[1] = {1.0};
+  if (scheme == 71) {
+    double e0 = 0;
+    if (act) {
+      const long long pl = pid(n), pr = pid(n + 1);
+      const double j1 = b.jac[pl], j2 = b.jac[pr];
+      double a[3];
+      for (int q = 0; q < 3; ++q) a[q] = b.met[(DIR * 3 + q) * P + pl] * j1 + b.met[(DIR * 3 + q) * P + pr] * j2;
+      e0 = 1e-20 * c_mix.weno_eps_scale * 0.25 * (a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
+    }
+    const double e1 = e0 * c_mix.v_ref * c_mix.v_ref, e2 = e1 * c_mix.v_ref * c_mix.v_ref;
+#pragma unroll 1
+    for (int l = 0; l < nv; ++l)
+#pragma unroll 1
+      for (int sd = 0; sd < 2; ++sd) {
+        double v[7], g[7];
+        if (act) {
+#pragma unroll
+          for (int m = 0; m < 7; ++m) v[m] = F(sd, l, m);
+          weno7_side_bwd(v, (l >= 1 && l <= 3) ? e1 : (l == 4 ? e2 : e0), afc(l), g);
+        }
+        scatter(sd, l, One(), one, g);
       }
+  } else {
+    auto AL_ = [&](int l) -> double & { return slots[l * NT + tid]; };             // alpha_l
+    auto A_AL = [&](int l) -> double & { return slots[(ns + l) * NT + tid]; };     // its adjoint
+    auto A_SV = [&](int l) -> double & { return slots[(2 * ns + l) * NT + tid]; };  // of the mass fraction
+    double rli = 1, rri = 1, wl = 0, wr = 0, sl = 1, sr = 1;  // wl, wr: Roe weights over rho
+    double um = 0, vm = 0, wm = 0, hm = 0, tm = 1, mw_inv = 1, gamma = 2, cm = 1, eps = 1, kx = 1, ky = 0, kz = 0;
+    const long long pl = act ? pid(n) : 0, pr = act ? pid(n + 1) : 0;
+    auto roe = [&](int l) -> double { return wl * s.cv[l * P + pl] + wr * s.cv[l * P + pr]; };
+    if (act) {
+      // forward: Roe-averaged mixture state at the face (as k_fvs)
+      const double rl = s.cv[pl], rr = s.cv[pr];
+      const double p_l = s.bv[4 * P + pl], p_r = s.bv[4 * P + pr];
+      rli = 1.0 / rl;
+      rri = 1.0 / rr;
+      sl = sqrt(rl);
+      sr = sqrt(rr);
+      const double isum = 1.0 / (sl + sr);
+      wl = sl * isum * rli;
+      wr = sr * isum * rri;
+      um = roe(1);
+      vm = roe(2);
+      wm = roe(3);
+      hm = roe(4) + (wl * p_l + wr * p_r);
+      mw_inv = 0;
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) {
+        const double sv = roe(5 + l);
+        mw_inv += sv * c_mix.imw[l];
+        A_SV(l) = sv;
+      }
+      tm = (wl * p_l + wr * p_r) / (kRuD * mw_inv);
+      double cp = 0, cvt = 0;
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) {
+        double h, c;
+        mix_h_cp_one<double>(l, tm, h, c);
+        const double sv = A_SV(l);
+        cp += sv * c;
+        cvt += sv * (c - c_mix.ru_mw[l]);
+        AL_(l) = h;
+        A_SV(l) = A_AL(l) = 0.0;
+      }
+      gamma = cp / cvt;
+      const double c2 = gamma * kRuD * mw_inv * tm;
+      cm = sqrt(c2);
+      const double jl = b.jac[pl], jr = b.jac[pr];
+      kx = b.met[(DIR * 3 + 0) * P + pl] * jl + b.met[(DIR * 3 + 0) * P + pr] * jr;
+      ky = b.met[(DIR * 3 + 1) * P + pl] * jl + b.met[(DIR * 3 + 1) * P + pr] * jr;
+      kz = b.met[(DIR * 3 + 2) * P + pl] * jl + b.met[(DIR * 3 + 2) * P + pr] * jr;
+      const double k2 = kx * kx + ky * ky + kz * kz, igk = 1.0 / sqrt(k2);
+      eps = 1e-40 * c_mix.weno_eps_scale * 0.25 * k2;
+      kx *= igk;
+      ky *= igk;
+      kz *= igk;
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) AL_(l) = (gamma * c_mix.ru_mw[l] * tm - (gamma - 1) * AL_(l)) / c2;
     }
-  } else if (face_ok && any) {
-    // forward: Roe-averaged mixture state at the face (as k_fvs)
-    const long long pl = pid(n), pr = pid(n + 1);
-    double cvl[Spec<NS>::A + 5], cvr[Spec<NS>::A + 5];
-    for (int l = 0; l < nv; ++l) {
-      cvl[l] = s.cv[l * P + pl];
-      cvr[l] = s.cv[l * P + pr];
-    }
-    const double p_l = s.bv[4 * P + pl], p_r = s.bv[4 * P + pr];
-    const double rli = 1.0 / cvl[0], rri = 1.0 / cvr[0];
-    const double sl = sqrt(cvl[0]), sr = sqrt(cvr[0]);
-    const double den = sl + sr, rlc = sl / den, rrc = sr / den;
-    const double um = rlc * cvl[1] * rli + rrc * cvr[1] * rri;
-    const double vm = rlc * cvl[2] * rli + rrc * cvr[2] * rri;
-    const double wm = rlc * cvl[3] * rli + rrc * cvr[3] * rri;
+    const double gm1 = gamma - 1, c2i = 1.0 / (cm * cm);
     const double ekm = 0.5 * (um * um + vm * vm + wm * wm);
-    const double hm = rlc * ((cvl[4] + p_l) * rli) + rrc * ((cvr[4] + p_r) * rri);
-    double svm[Spec<NS>::A], hi[Spec<NS>::A], cpi[Spec<NS>::A], al[Spec<NS>::A];
-    double mw_inv = 0;
-    for (int l = 0; l < ns; ++l) {
-      svm[l] = rlc * cvl[l + 5] * rli + rrc * cvr[l + 5] * rri;
-      mw_inv += svm[l] / c_mix.mw[l];
-    }
-    const double prm = rlc * (p_l * rli) + rrc * (p_r * rri);
-    const double tm = prm / (kRuD * mw_inv);
-    mix_h_cp<NS, double>(tm, hi, cpi);
-    double cp = 0, cvt = 0;
-    for (int l = 0; l < ns; ++l) {
-      cp += svm[l] * cpi[l];
-      cvt += svm[l] * (cpi[l] - c_mix.ru_mw[l]);
-    }
-    const double gamma = cp / cvt;
-    const double cm = sqrt(gamma * kRuD * mw_inv * tm);
-    const double gm1 = gamma - 1;
-    const double jl = b.jac[pl], jr = b.jac[pr];
-    const double kxJ = b.met[(DIR * 3 + 0) * P + pl] * jl + b.met[(DIR * 3 + 0) * P + pr] * jr;
-    const double kyJ = b.met[(DIR * 3 + 1) * P + pl] * jl + b.met[(DIR * 3 + 1) * P + pr] * jr;
-    const double kzJ = b.met[(DIR * 3 + 2) * P + pl] * jl + b.met[(DIR * 3 + 2) * P + pr] * jr;
-    double kx = kxJ / (jl + jr), ky = kyJ / (jl + jr), kz = kzJ / (jl + jr);
-    const double gradK = sqrt(kx * kx + ky * ky + kz * kz);
-    kx /= gradK;
-    ky /= gradK;
-    kz /= gradK;
-    const double Ukb = kx * um + ky * vm + kz * wm;
-    const double alpha = gm1 * ekm;
-    const double c2i = 1.0 / (cm * cm);
-    const double eps = 1e-40 * c_mix.weno_eps_scale * 0.25 * (kxJ * kxJ + kyJ * kyJ + kzJ * kzJ);
-    for (int l = 0; l < ns; ++l) al[l] = (gamma * kRuD / c_mix.mw[l] * tm - (gamma - 1) * hi[l]) * c2i;
-    // characteristic projections and face values
-    auto project = [&](int l, double *vp, double *vmn) {
-      if (l < 5) {
-        double L[5], cs;
-        fvs_lrow(l, alpha, Ukb, cm, c2i, gm1, um, vm, wm, kx, ky, kz, L, cs);
-        for (int m = 0; m < 7; ++m) {
-          double a = 0, bq = 0;
-          for (int q = 0; q < 5; ++q) {
-            a += L[q] * FP(m, q);
-            bq += L[q] * FM(m + 1, q);
-          }
-          for (int q = 0; q < ns; ++q) {
-            a += cs * al[q] * FP(m, 5 + q);
-            bq += cs * al[q] * FM(m + 1, 5 + q);
-          }
-          vp[m] = a;
-          vmn[m] = bq;
-        }
-      } else {
-        for (int m = 0; m < 7; ++m) {
-          vp[m] = -svm[l - 5] * FP(m, 0) + FP(m, l);
-          vmn[m] = -svm[l - 5] * FM(m + 1, 0) + FM(m + 1, l);
-        }
-      }
-    };
-    double fch[Spec<NS>::A + 5];
-    for (int l = 0; l < nv; ++l) {
-      double vp[7], vmn[7];
-      project(l, vp, vmn);
-      fch[l] = fvs_weno7(vp, vmn, eps);
-    }
-    // reverse of fc = R fch (WENO.cu:1069-1117)
-    const double ca = fch[0] + kx * fch[1] + ky * fch[2] + kz * fch[3] + fch[4];
+    const double Ukb = kx * um + ky * vm + kz * wm, alpha = gm1 * ekm;
     const double cg = cm * cm / gm1;
-    const double hc = hm - cg;
-    double add = 0, aca = afc[0];
-    for (int l = 0; l < ns; ++l) {
-      add += al[l] * fch[l + 5];
-      aca += svm[l] * afc[5 + l];
-    }
-    double afch[Spec<NS>::A + 5], a_svm[Spec<NS>::A], a_al[Spec<NS>::A];
-    for (int l = 0; l < ns; ++l) {
-      afch[5 + l] = afc[5 + l] - afc[4] * al[l] * cg;
-      a_svm[l] = ca * afc[5 + l];
-      a_al[l] = -afc[4] * fch[5 + l] * cg;
-    }
-    double a_cg = -afc[4] * add;
-    afch[0] = aca + afc[1] * (um - kx * cm) + afc[2] * (vm - ky * cm) + afc[3] * (wm - kz * cm) + afc[4] * (hm - Ukb * cm);
-    afch[1] = aca * kx + afc[1] * kx * um + afc[2] * (kx * vm + kz * cm) + afc[3] * (kx * wm - ky * cm) +
-              afc[4] * (kx * hc + (kz * vm - ky * wm) * cm);
-    afch[2] = aca * ky + afc[1] * (ky * um - kz * cm) + afc[2] * ky * vm + afc[3] * (ky * wm + kx * cm) +
-              afc[4] * (ky * hc + (kx * wm - kz * um) * cm);
-    afch[3] = aca * kz + afc[1] * (kz * um + ky * cm) + afc[2] * (kz * vm - kx * cm) + afc[3] * kz * wm +
-              afc[4] * (kz * hc + (ky * um - kx * vm) * cm);
-    afch[4] = aca + afc[1] * (um + kx * cm) + afc[2] * (vm + ky * cm) + afc[3] * (wm + kz * cm) + afc[4] * (hm + Ukb * cm);
     RoeBar r{};
-    r.um = afc[1] * ca + afc[4] * cm * (-kz * fch[2] + ky * fch[3]);
-    r.vm = afc[2] * ca + afc[4] * cm * (kz * fch[1] - kx * fch[3]);
-    r.wm = afc[3] * ca + afc[4] * cm * (-ky * fch[1] + kx * fch[2]);
-    r.cm = afc[1] * (-kx * fch[0] - kz * fch[2] + ky * fch[3] + kx * fch[4]) +
-           afc[2] * (-ky * fch[0] + kz * fch[1] - kx * fch[3] + ky * fch[4]) +
-           afc[3] * (-kz * fch[0] - ky * fch[1] + kx * fch[2] + kz * fch[4]) +
-           afc[4] * (-Ukb * fch[0] + (kz * vm - ky * wm) * fch[1] + (kx * wm - kz * um) * fch[2] +
-                     (ky * um - kx * vm) * fch[3] + Ukb * fch[4]);
-    double a_hm = afc[4] * (fch[0] + fch[4]);
-    const double a_hc = afc[4] * (kx * fch[1] + ky * fch[2] + kz * fch[3]);
-    r.Ukb = afc[4] * cm * (fch[4] - fch[0]);
-    a_hm += a_hc;
-    a_cg -= a_hc;
-    r.cm += a_cg * 2 * cm / gm1;
-    r.gm1 -= a_cg * cg / gm1;
-    // WENO and projection reverse per characteristic field; split-flux adjoints into shared memory
-    for (int l = 0; l < nv; ++l) {
-      double vp[7], vmn[7], gp[7], gm[7];
-      project(l, vp, vmn);
-      for (int m = 0; m < 7; ++m) gp[m] = gm[m] = 0.0;
-      weno7_bwd(vp, vmn, eps, afch[l], gp, gm);
-      if (l < 5) {
-        double L[5], cs, AL[5];
-        fvs_lrow(l, alpha, Ukb, cm, c2i, gm1, um, vm, wm, kx, ky, kz, L, cs);
-        for (int q = 0; q < 5; ++q) {
-          double s_ = 0;
-          for (int m = 0; m < 7; ++m) {
-            s_ += FP(m, q) * gp[m] + FM(m + 1, q) * gm[m];
-            atomicAdd(AFP(m, q), L[q] * gp[m]);
-            atomicAdd(AFM(m + 1, q), L[q] * gm[m]);
-          }
-          AL[q] = s_;
-        }
-        for (int q = 0; q < ns; ++q) {
-          double s_ = 0;
-          for (int m = 0; m < 7; ++m) {
-            s_ += FP(m, 5 + q) * gp[m] + FM(m + 1, 5 + q) * gm[m];
-            atomicAdd(AFP(m, 5 + q), cs * al[q] * gp[m]);
-            atomicAdd(AFM(m + 1, 5 + q), cs * al[q] * gm[m]);
-          }
-          a_al[q] += cs * s_;
-        }
-        fvs_lrow_bwd(l, AL, alpha, Ukb, cm, c2i, gm1, um, vm, wm, kx, ky, kz, r);
-      } else {
-        double s_ = 0;
-        for (int m = 0; m < 7; ++m) {
-          s_ += FP(m, 0) * gp[m] + FM(m + 1, 0) * gm[m];
-          atomicAdd(AFP(m, 0), -svm[l - 5] * gp[m]);
-          atomicAdd(AFM(m + 1, 0), -svm[l - 5] * gm[m]);
-          atomicAdd(AFP(m, l), gp[m]);
-          atomicAdd(AFM(m + 1, l), gm[m]);
-        }
-        a_svm[l - 5] -= s_;
+    double a_hm = 0, a_cg = 0, ca = 0;
+    // reverse of fc = R fch (WENO.cu:1069-1117): the adjoint of the flow field l and, once its face value f is
+    // known, the adjoints of R
+    const double f4 = act ? afc(4) : 0.0;
+    double aca = 0;
+    if (act) {
+      aca = afc(0);
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) aca += roe(5 + l) * afc(5 + l);
+    }
+    auto flow_bar = [&](int l) -> double {
+      const double hc = hm - cg;
+      if (l == 0 || l == 4) {
+        const double c = l == 0 ? -cm : cm;
+        return aca + afc(1) * (um + kx * c) + afc(2) * (vm + ky * c) + afc(3) * (wm + kz * c) + f4 * (hm + Ukb * c);
       }
-    }
-    // Roe symbols -> Roe averages
-    r.gm1 += r.alpha * ekm;
-    r.um += r.alpha * gm1 * um + r.Ukb * kx;
-    r.vm += r.alpha * gm1 * vm + r.Ukb * ky;
-    r.wm += r.alpha * gm1 * wm + r.Ukb * kz;
-    double a_gamma = 0, a_tm = 0, a_mwinv = 0;
-    double a_al_sum = 0;
-    for (int l = 0; l < ns; ++l) {
-      a_gamma += a_al[l] * kRuD / c_mix.mw[l] * tm * c2i;
-      r.gm1 -= a_al[l] * hi[l] * c2i;
-      a_tm += a_al[l] * gamma * kRuD / c_mix.mw[l] * c2i;
-      a_al_sum += a_al[l] * al[l];
-    }
-    r.c2i += a_al_sum / c2i;
-    r.cm -= 2.0 * r.c2i * c2i / cm;
-    a_gamma += r.gm1;
-    a_gamma += r.cm * cm / (2 * gamma);
-    a_mwinv += r.cm * cm / (2 * mw_inv);
-    a_tm += r.cm * cm / (2 * tm);
-    const double a_cp = a_gamma / cvt, a_cvt = -a_gamma * gamma / cvt;
-    double dcp[Spec<NS>::A];
-    mix_dcp_dt<NS>(tm, dcp);
-    for (int l = 0; l < ns; ++l) {
-      a_svm[l] += a_cp * cpi[l] + a_cvt * (cpi[l] - c_mix.ru_mw[l]);
-      const double a_cpi = (a_cp + a_cvt) * svm[l];
-      const double a_hi = -a_al[l] * gm1 * c2i;
-      a_tm += a_hi * cpi[l] + a_cpi * dcp[l];
-    }
-    const double a_prm = a_tm / (kRuD * mw_inv);
-    a_mwinv -= a_tm * tm / mw_inv;
-    for (int l = 0; l < ns; ++l) a_svm[l] += a_mwinv / c_mix.mw[l];
-    // averages X = rlc X_l + rrc X_r of u, v, w, H, Y, p/rho; per side X = num / rho
-    double a_rlc = 0, a_rrc = 0;
-    double gl[Spec<NS>::A + 6], gr[Spec<NS>::A + 6];  // adjoints of cv[0..nv-1] and p, per side
-    for (int l = 0; l <= nv; ++l) gl[l] = gr[l] = 0.0;
-    auto avg = [&](double aX, double Xl, double Xr, int numl) {
-      // numl: index of the numerator in cv (or nv for p); X = num / rho
-      a_rlc += aX * Xl;
-      a_rrc += aX * Xr;
-      gl[numl] += aX * rlc * rli;
-      gr[numl] += aX * rrc * rri;
-      gl[0] -= aX * rlc * Xl * rli;
-      gr[0] -= aX * rrc * Xr * rri;
+      if (l == 1)
+        return aca * kx + afc(1) * kx * um + afc(2) * (kx * vm + kz * cm) + afc(3) * (kx * wm - ky * cm) +
+               f4 * (kx * hc + (kz * vm - ky * wm) * cm);
+      if (l == 2)
+        return aca * ky + afc(1) * (ky * um - kz * cm) + afc(2) * ky * vm + afc(3) * (ky * wm + kx * cm) +
+               f4 * (ky * hc + (kx * wm - kz * um) * cm);
+      return aca * kz + afc(1) * (kz * um + ky * cm) + afc(2) * (kz * vm - kx * cm) + afc(3) * kz * wm +
+             f4 * (kz * hc + (ky * um - kx * vm) * cm);
     };
-    avg(r.um, cvl[1] * rli, cvr[1] * rri, 1);
-    avg(r.vm, cvl[2] * rli, cvr[2] * rri, 2);
-    avg(r.wm, cvl[3] * rli, cvr[3] * rri, 3);
-    avg(a_hm, (cvl[4] + p_l) * rli, (cvr[4] + p_r) * rri, 4);
-    gl[nv] += a_hm * rlc * rli;  // H = (rho E + p) / rho
-    gr[nv] += a_hm * rrc * rri;
-    for (int l = 0; l < ns; ++l) avg(a_svm[l], cvl[5 + l] * rli, cvr[5 + l] * rri, 5 + l);
-    avg(a_prm, p_l * rli, p_r * rri, nv);
-    const double a_sl = (a_rlc - a_rrc) * sr / (den * den), a_sr = (a_rrc - a_rlc) * sl / (den * den);
-    gl[0] += a_sl / (2 * sl);
-    gr[0] += a_sr / (2 * sr);
-    double *rl = aR + ((long long)(t + 3) * TXL + lane) * (nv + 1);
-    double *rr = aR + ((long long)(t + 4) * TXL + lane) * (nv + 1);
-    for (int l = 0; l <= nv; ++l) {
-      atomicAdd(rl + l, gl[l]);
-      atomicAdd(rr + l, gr[l]);
+    auto flow_face = [&](int l, double f) {
+      if (l == 0 || l == 4) {
+        const double sg = l == 0 ? -1.0 : 1.0;
+        ca += f;
+        r.um += afc(1) * f;
+        r.vm += afc(2) * f;
+        r.wm += afc(3) * f;
+        r.cm += sg * f * (afc(1) * kx + afc(2) * ky + afc(3) * kz + f4 * Ukb);
+        r.Ukb += sg * f * f4 * cm;
+        a_hm += f4 * f;
+      } else {
+        const double k = l == 1 ? kx : l == 2 ? ky : kz;
+        const double fk = k * f, c4 = f4 * cm * f;
+        ca += fk;
+        r.um += afc(1) * fk;
+        r.vm += afc(2) * fk;
+        r.wm += afc(3) * fk;
+        if (l == 1) {
+          r.vm += kz * c4;
+          r.wm -= ky * c4;
+          r.cm += f * (afc(2) * kz - afc(3) * ky + f4 * (kz * vm - ky * wm));
+        } else if (l == 2) {
+          r.um -= kz * c4;
+          r.wm += kx * c4;
+          r.cm += f * (afc(3) * kx - afc(1) * kz + f4 * (kx * wm - kz * um));
+        } else {
+          r.um += ky * c4;
+          r.vm -= kx * c4;
+          r.cm += f * (afc(1) * ky - afc(2) * kx + f4 * (ky * um - kx * vm));
+        }
+        a_hm += f4 * fk;
+        a_cg -= f4 * fk;
+      }
+    };
+#pragma unroll 1
+    for (int sd = 0; sd < 2; ++sd) {
+      double W[7];
+#pragma unroll
+      for (int m = 0; m < 7; ++m) W[m] = 0.0;
+#pragma unroll 1
+      for (int l = 0; l < 5; ++l) {
+        double L[5], cs, g[7];
+        if (act) {
+          double v[7], AL[5];
+          fvs_lrow(l, alpha, Ukb, cm, c2i, gm1, um, vm, wm, kx, ky, kz, L, cs);
+#pragma unroll
+          for (int m = 0; m < 7; ++m) v[m] = 0.0;
+#pragma unroll 1
+          for (int q = 0; q < ns; ++q) {
+            const double al = cs * AL_(q);
+#pragma unroll
+            for (int m = 0; m < 7; ++m) v[m] += al * F(sd, 5 + q, m);
+          }
+#pragma unroll
+          for (int m = 0; m < 7; ++m)
+#pragma unroll
+            for (int q = 0; q < 5; ++q) v[m] += L[q] * F(sd, q, m);
+          flow_face(l, weno7_side_bwd(v, eps, flow_bar(l), g));
+#pragma unroll
+          for (int q = 0; q < 5; ++q) AL[q] = 0.0;
+#pragma unroll
+          for (int m = 0; m < 7; ++m) {
+            W[m] += cs * g[m];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) AL[q] += F(sd, q, m) * g[m];
+          }
+          fvs_lrow_bwd(l, AL, alpha, Ukb, cm, c2i, gm1, um, vm, wm, kx, ky, kz, r);
+        }
+        scatter(sd, 0, Five(), L, g);
+      }
+      double Z[7];
+#pragma unroll
+      for (int m = 0; m < 7; ++m) Z[m] = 0.0;
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) {
+        double g[7];
+        if (act) {
+          const double sv = roe(5 + l), al = AL_(l), f5 = afc(5 + l);
+          double v[7], s0 = 0, s1 = 0;
+#pragma unroll
+          for (int m = 0; m < 7; ++m) v[m] = F(sd, 5 + l, m) - sv * F(sd, 0, m);
+          const double f = weno7_side_bwd(v, eps, f5 - f4 * al * cg, g);
+#pragma unroll
+          for (int m = 0; m < 7; ++m) {
+            s0 += F(sd, 0, m) * g[m];
+            s1 += F(sd, 5 + l, m) * W[m];
+            Z[m] -= sv * g[m];
+            g[m] += al * W[m];
+          }
+          A_SV(l) -= s0;
+          A_AL(l) += s1 - f4 * f * cg;
+          a_cg -= f4 * al * f;
+        }
+        scatter(sd, 5 + l, One(), one, g);
+      }
+      scatter(sd, 0, One(), one, Z);
+    }
+    if (act) {
+      r.cm += a_cg * 2 * cm / gm1;
+      r.gm1 -= a_cg * cg / gm1;
+      // Roe symbols -> Roe averages
+      r.gm1 += r.alpha * ekm;
+      r.um += r.alpha * gm1 * um + r.Ukb * kx;
+      r.vm += r.alpha * gm1 * vm + r.Ukb * ky;
+      r.wm += r.alpha * gm1 * wm + r.Ukb * kz;
+      double a_gamma = 0, a_tm = 0, a_mwinv = 0, a_al_sum = 0;
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) {
+        double h, c;
+        mix_h_cp_one<double>(l, tm, h, c);
+        const double a = A_AL(l);
+        a_gamma += a * c_mix.ru_mw[l] * tm * c2i;
+        r.gm1 -= a * h * c2i;
+        a_tm += a * gamma * c_mix.ru_mw[l] * c2i;
+        a_al_sum += a * AL_(l);
+      }
+      r.c2i += a_al_sum / c2i;
+      r.cm -= 2.0 * r.c2i * c2i / cm;
+      a_gamma += r.gm1 + r.cm * cm / (2 * gamma);
+      a_mwinv += r.cm * cm / (2 * mw_inv);
+      a_tm += r.cm * cm / (2 * tm);
+      // cvt = sum Y (cp - Ru / W) of the Roe average: cp - cvt = Ru mw_inv and gamma = cp / cvt
+      const double cvt = kRuD * mw_inv / gm1;
+      const double a_cp = a_gamma / cvt, a_cvt = -a_gamma * gamma / cvt;
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l) {
+        double h, c;
+        mix_h_cp_one<double>(l, tm, h, c);
+        const double sv = roe(5 + l);
+        A_SV(l) += ca * afc(5 + l) + a_cp * c + a_cvt * (c - c_mix.ru_mw[l]);
+        a_tm += -A_AL(l) * gm1 * c2i * c + (a_cp + a_cvt) * sv * mix_dcp_dt_one(l, tm);
+      }
+      const double a_prm = a_tm / (kRuD * mw_inv);
+      a_mwinv -= a_tm * tm / mw_inv;
+      // averages X = rlc X_l + rrc X_r of u, v, w, H, Y, p/rho; per side X = num / rho
+      double a_rlc = 0, a_rrc = 0, g0l = 0, g0r = 0;
+      auto avg = [&](double aX, double nl, double nr, double *plane) {
+        // nl, nr: the numerators; their adjoints go to `plane` (of cv, or p)
+        const double Xl = nl * rli, Xr = nr * rri, gl = aX * wl, gr = aX * wr;
+        a_rlc += aX * Xl;
+        a_rrc += aX * Xr;
+        g0l -= gl * Xl;
+        g0r -= gr * Xr;
+        atomicAdd(plane + pl, gl);
+        atomicAdd(plane + pr, gr);
+      };
+      const double p_l = s.bv[4 * P + pl], p_r = s.bv[4 * P + pr];
+      avg(r.um, s.cv[P + pl], s.cv[P + pr], A.cv + P);
+      avg(r.vm, s.cv[2 * P + pl], s.cv[2 * P + pr], A.cv + 2 * P);
+      avg(r.wm, s.cv[3 * P + pl], s.cv[3 * P + pr], A.cv + 3 * P);
+      avg(a_hm, s.cv[4 * P + pl] + p_l, s.cv[4 * P + pr] + p_r, A.cv + 4 * P);  // H = (rho E + p) / rho
+      avg(a_prm, p_l, p_r, A.p);
+      atomicAdd(A.p + pl, a_hm * wl);
+      atomicAdd(A.p + pr, a_hm * wr);
+#pragma unroll 1
+      for (int l = 0; l < ns; ++l)
+        avg(A_SV(l) + a_mwinv * c_mix.imw[l], s.cv[(5 + l) * P + pl], s.cv[(5 + l) * P + pr], A.cv + (5 + l) * P);
+      const double den = sl + sr;
+      g0l += (a_rlc - a_rrc) * sr / (den * den) / (2 * sl);
+      g0r += (a_rrc - a_rlc) * sl / (den * den) / (2 * sr);
+      atomicAdd(A.cv + pl, g0l);
+      atomicAdd(A.cv + pr, g0r);
     }
   }
   __syncthreads();
-  // staged nodes: split-flux and Roe adjoints -> node planes
+  // staged nodes: split-flux adjoints -> node planes
   if (lane_ok) {
     for (int st = t; st < NST; st += TD) {
       const int nn = start - 4 + st;
       if (nn > nd + 3) continue;
       const long long p = pid(nn);
-      double Q[Spec<NS>::A + 5], aQ[Spec<NS>::A + 5];
-      const double *ra = aR + ((long long)st * TXL + lane) * (nv + 1);
-      for (int l = 0; l < nv; ++l) {
-        Q[l] = s.cv[l * P + p];
-        aQ[l] = ra[l];
-      }
-      double ap = ra[nv], ac = 0.0;
-      fvs_node_bwd(Q, s.bv[4 * P + p], s.acs[p], b.met[(DIR * 3 + 0) * P + p], b.met[(DIR * 3 + 1) * P + p],
-                   b.met[(DIR * 3 + 2) * P + p], b.jac[p], aFp + ((long long)st * TXL + lane) * nv,
-                   aFm + ((long long)st * TXL + lane) * nv, nv, aQ, ap, ac);
+      double Q[Spec<NS>::A + 5], aQ[Spec<NS>::A + 5], ap, ac;
+      for (int l = 0; l < nv; ++l) Q[l] = s.cv[l * P + p];
+      fvs_node_bwd<NS>(Q, s.bv[4 * P + p], s.acs[p], b.met[(DIR * 3 + 0) * P + p], b.met[(DIR * 3 + 1) * P + p],
+                       b.met[(DIR * 3 + 2) * P + p], b.jac[p], aFp + st * TXL + lane, aFm + st * TXL + lane, NN, aQ, ap, ac);
       for (int l = 0; l < nv; ++l)
         if (aQ[l] != 0.0) atomicAdd(A.cv + l * P + p, aQ[l]);
       if (ap != 0.0) atomicAdd(A.p + p, ap);
@@ -917,8 +951,12 @@ __global__ void __launch_bounds__(128, 4) k_adj_source(DevBlock b, DevState s, c
 // FieldOperation.cuh:107-134, compute_transport_property, Transport.cu:43-136) at every padded node:
 // adjoints of c, mu, lambda and rho*D_k -> adjoints of rho, p, T and Y.  Hand-written reverse of
 // mix_properties (one forward sweep keeping its intermediates, then the reverse sweep).
+// The powers, square roots and quotients are those of mix_properties (one log, one exp, one reciprocal
+// square root a species, the powers of the collision integrals' constants in the tables); with a pow per
+// species and pair and a square root per ratio it took 1.7 ms at 96 x 64 x 48, of a VJP of 11.6 then
+// and 5.0 now.
 template <int NS>
-__global__ void __launch_bounds__(128, 4) k_adj_props(DevBlock b, DevState s, DevAdj A) {
+__global__ void __launch_bounds__(128, 2) k_adj_props(DevBlock b, DevState s, DevAdj A) {
   const long long P = b.plane;
   const int ns = OSTC_NS;
   constexpr int SA = Spec<NS>::A;
@@ -928,148 +966,146 @@ __global__ void __launch_bounds__(128, 4) k_adj_props(DevBlock b, DevState s, De
     const double ac = A.c[p], amu = A.mu[p], alam = A.lam[p];
     double ard[SA];
     bool any = ac != 0.0 || amu != 0.0 || alam != 0.0;
+#pragma unroll
     for (int l = 0; l < ns; ++l) {
       ard[l] = A.rhod[(long long)l * P + p];
       any = any || ard[l] != 0.0;
     }
     if (!any) continue;
-    const double pr = s.bv[4 * P + p], t = s.bv[5 * P + p];
-    double y[SA], cp[SA], dcp[SA];
-    for (int l = 0; l < ns; ++l) y[l] = s.sv[l * P + p];
-    mix_h_cp<NS, double>(t, nullptr, cp);
-    mix_dcp_dt<NS>(t, dcp);
-    // ---- forward (as mix_properties)
+    const double pr = s.bv[4 * P + p], t = s.bv[5 * P + p], it = 1.0 / t;
+    const double st = sqrt(t), tp = exp(-0.145 * log(t)), dtp = -0.145 * tp * it;  // T^-0.145
     double smw = 0, cpt = 0, cvt = 0;
+#pragma unroll
     for (int l = 0; l < ns; ++l) {
-      smw += y[l] * c_mix.imw[l];
-      cpt += y[l] * cp[l];
-      cvt += y[l] * (cp[l] - c_mix.ru_mw[l]);
+      const double y = s.sv[l * P + p];
+      double h, cp;
+      mix_h_cp_one<double>(l, t, h, cp);
+      smw += y * c_mix.imw[l];
+      cpt += y * cp;
+      cvt += y * (cp - c_mix.ru_mw[l]);
     }
-    const double mw = 1 / smw;
-    const double gamma = cpt / cvt;
-    const double acoustic = sqrt(gamma * kRuD * t / mw);
-    double X[SA], vis[SA], dlvis[SA];  // dlvis = d ln(vis) / dT
-    const double st = sqrt(t);
+    const double mw = 1 / smw, gamma = cpt / cvt;
+    double X[SA], aX[SA];
+#pragma unroll
     for (int l = 0; l < ns; ++l) {
-      X[l] = y[l] * mw * c_mix.imw[l];
-      const double lj = c_mix.lj_potent_inv[l], tdl = t * lj;
-      const double a1 = pow(tdl, -0.145), a2 = pow(tdl + 0.5, -2.0);
-      const double ci = 1.147 * a1 + a2;
-      vis[l] = c_mix.vis_coeff[l] * st / ci;
-      const double dci = lj * (1.147 * -0.145 * a1 / tdl - 2.0 * a2 / (tdl + 0.5));
-      dlvis[l] = 0.5 / t - dci / ci;
+      X[l] = s.sv[l * P + p] * mw * c_mix.imw[l];
+      aX[l] = 0.0;
     }
-    double vt[SA], ct[SA];
-    for (int m = 0; m < ns; ++m) {
-      double v_ = 0;
-      for (int n = 0; n < ns; ++n) {
-        double pf = 1.0;
-        if (m != n) {
-          const double nm = 1 + sqrt(vis[m] / vis[n]) * c_mix.wj_div_wi_1_4[m][n];
-          pf = nm * nm * c_mix.sqrt_wiwj_8[m][n];
+    double arho = 0, aT = 0, ap = 0, amw = 0;
+    {
+      // rho D_l = rho t32p num_l / (den_l mw), den_l = sum (X_n + eps) w_ln, w = tp kbe_pow + q,
+      // q = 1 / (D (T* + 0.5)^2)
+      const double t32p = t * st / pr, eps = 1e-12;
+      double num[SA], den[SA];
+#pragma unroll
+      for (int l = 0; l < ns; ++l) num[l] = den[l] = 0;
+#pragma unroll
+      for (int l = 0; l < ns; ++l)
+#pragma unroll
+        for (int n = l + 1; n < ns; ++n) {
+          const double a = t * c_mix.kb_over_eps[l][n] + 0.5;
+          const double w = tp * c_mix.kbe_pow[l][n] + c_mix.inv_diff[l][n] / (a * a);
+          num[l] += (X[n] + eps) * c_mix.mw[n];
+          den[l] += (X[n] + eps) * w;
+          num[n] += (X[l] + eps) * c_mix.mw[l];
+          den[n] += (X[l] + eps) * w;
         }
-        v_ += pf * X[n];
+      double sum = 0, aden[SA], anum[SA];
+#pragma unroll
+      for (int l = 0; l < ns; ++l) {
+        const double id = 1.0 / den[l], f = ard[l] * (rho * smw * t32p) * id;  // ard rho D / num
+        sum += f * num[l];
+        anum[l] = f;
+        aden[l] = -f * num[l] * id;
       }
-      vt[m] = v_;
-      ct[m] = 1.065 * v_ - 0.065 * X[m];
-    }
-    const double t32p = t * st / pr;
-    const double eps = 1e-12;
-    double num[SA], den[SA];
-    for (int l = 0; l < ns; ++l) num[l] = den[l] = 0;
-    for (int l = 0; l < ns; ++l)
-      for (int n = l + 1; n < ns; ++n) {
-        const double tr = t * c_mix.kb_over_eps[l][n];
-        const double om = 1.0 / pow(tr, 0.145) + 1.0 / ((tr + 0.5) * (tr + 0.5));
-        const double dln = c_mix.binary_diff[l][n] * t32p / om;
-        num[l] += (X[n] + eps) * c_mix.mw[n];
-        den[l] += (X[n] + eps) / dln;
-        num[n] += (X[l] + eps) * c_mix.mw[l];
-        den[n] += (X[l] + eps) / dln;
-      }
-    // ---- reverse
-    double aX[SA], avis[SA], aY[SA], acp[SA], aden[SA], avt[SA];
-    for (int l = 0; l < ns; ++l) aX[l] = avis[l] = aY[l] = acp[l] = 0.0;
-    double arho = 0, aT = 0, ap = 0, amw = 0, at32p = 0;
-    // rho D_l = rho num_l / (den_l mw)
-    for (int l = 0; l < ns; ++l) {
-      const double rd = rho * num[l] / (den[l] * mw);
-      arho += ard[l] * rd / rho;
-      const double anum = ard[l] * rd / num[l];
-      aden[l] = -ard[l] * rd / den[l];
-      amw -= ard[l] * rd / mw;
-      for (int n = 0; n < ns; ++n)
-        if (n != l) aX[n] += anum * c_mix.mw[n];
-    }
-    for (int l = 0; l < ns; ++l)
-      for (int n = l + 1; n < ns; ++n) {
-        const double kbe = c_mix.kb_over_eps[l][n], tr = t * kbe;
-        const double a1 = pow(tr, 0.145), a2 = 1.0 / ((tr + 0.5) * (tr + 0.5));
-        const double om = 1.0 / a1 + a2;
-        const double bd = c_mix.binary_diff[l][n];
-        const double dln = bd * t32p / om;
-        const double idl = 1.0 / dln;
-        aX[n] += aden[l] * idl;
-        aX[l] += aden[n] * idl;
-        const double adln = -(aden[l] * (X[n] + eps) + aden[n] * (X[l] + eps)) * idl * idl;
-        at32p += adln * bd / om;
-        const double aom = -adln * dln / om;
-        // om = tr^-0.145 + (tr + 0.5)^-2
-        aT += aom * kbe * (-0.145 / (a1 * tr) - 2.0 * a2 / (tr + 0.5));
-      }
-    // t32p = T^1.5 / p
-    aT += at32p * 1.5 * t32p / t;
-    ap -= at32p * t32p / pr;
-    // lambda = sum lam_m X_m / ct_m, lam_m = vis_m (cp_m + 1.25 Ru / W_m); mu = sum vis_m X_m / vt_m
-    for (int m = 0; m < ns; ++m) {
-      const double lfac = cp[m] + 1.25 * c_mix.ru_mw[m];
-      const double lamm = vis[m] * lfac;
-      const double alm = alam * X[m] / ct[m];
-      aX[m] += alam * lamm / ct[m];
-      const double act = -alam * lamm * X[m] / (ct[m] * ct[m]);
-      avt[m] = 1.065 * act;
-      aX[m] -= 0.065 * act;
-      avis[m] += alm * lfac;
-      acp[m] += alm * vis[m];
-      avis[m] += amu * X[m] / vt[m];
-      aX[m] += amu * vis[m] / vt[m];
-      avt[m] -= amu * vis[m] * X[m] / (vt[m] * vt[m]);
-    }
-    // vt_m = sum_n pf_mn X_n, pf_mn = (1 + sqrt(vis_m / vis_n) w_mn)^2 s_mn
-    for (int m = 0; m < ns; ++m)
-      for (int n = 0; n < ns; ++n) {
-        if (m == n) {
-          aX[n] += avt[m];
-          continue;
+      arho += sum / rho;
+      amw -= sum * smw;
+      aT += 1.5 * sum * it;
+      ap -= sum / pr;
+#pragma unroll
+      for (int l = 0; l < ns; ++l)
+#pragma unroll
+        for (int n = l + 1; n < ns; ++n) {
+          const double kbe = c_mix.kb_over_eps[l][n], ia = 1.0 / (t * kbe + 0.5);
+          const double q = c_mix.inv_diff[l][n] * ia * ia, w = tp * c_mix.kbe_pow[l][n] + q;
+          aX[n] += aden[l] * w + anum[l] * c_mix.mw[n];
+          aX[l] += aden[n] * w + anum[n] * c_mix.mw[l];
+          aT += (aden[l] * (X[n] + eps) + aden[n] * (X[l] + eps)) * (c_mix.kbe_pow[l][n] * dtp - 2.0 * kbe * ia * q);
         }
-        const double r = sqrt(vis[m] / vis[n]), w = c_mix.wj_div_wi_1_4[m][n], sw = c_mix.sqrt_wiwj_8[m][n];
-        const double nm = 1 + r * w;
-        aX[n] += avt[m] * nm * nm * sw;
-        const double ar = avt[m] * X[n] * 2 * nm * sw * w;
-        avis[m] += ar * r / (2 * vis[m]);
-        avis[n] -= ar * r / (2 * vis[n]);
+    }
+    double aTv = 0, acp[SA];
+    {
+      double vis[SA], isv[SA], avis[SA], dlv[SA];  // dlv = d ln(vis) / dT
+#pragma unroll
+      for (int l = 0; l < ns; ++l) {
+        // vis = coeff sqrt(T) a^2 / d, d = lj_pow tp a^2 + 1
+        const double lj = c_mix.lj_potent_inv[l], a = t * lj + 0.5, a2 = a * a, e = c_mix.lj_pow[l] * tp * a2, d = e + 1.0;
+        const double q = 1.0 / (a * d);
+        vis[l] = c_mix.vis_coeff[l] * st * a2 * (a * q);
+        dlv[l] = 0.5 * it + (2.0 * lj + 0.145 * e * it * a) * q;
+        isv[l] = rsqrt(vis[l]);
+        avis[l] = 0.0;
       }
-    for (int l = 0; l < ns; ++l) aT += avis[l] * vis[l] * dlvis[l];
+      // lambda = sum lam_m X_m / ct_m, lam_m = vis_m (cp_m + 1.25 Ru / W_m); mu = sum vis_m X_m / vt_m;
+      // vt_m = sum_n pf_mn X_n, pf_mn = (1 + sqrt(vis_m / vis_n) w_mn)^2 s_mn
+#pragma unroll
+      for (int m = 0; m < ns; ++m) {
+        const double svm = vis[m] * isv[m];
+        double vt = X[m];
+#pragma unroll
+        for (int n = 0; n < ns; ++n) {
+          if (m == n) continue;
+          const double nm = 1 + svm * isv[n] * c_mix.wj_div_wi_1_4[m][n];
+          vt += nm * nm * c_mix.sqrt_wiwj_8[m][n] * X[n];
+        }
+        const double ct = 1.065 * vt - 0.065 * X[m];
+        const double q = 1.0 / (vt * ct), ivt = ct * q, ict = vt * q;
+        double h, cp;
+        mix_h_cp_one<double>(m, t, h, cp);
+        const double lfac = cp + 1.25 * c_mix.ru_mw[m];
+        const double al = alam * ict, au = amu * ivt;
+        const double act = -al * vis[m] * lfac * X[m] * ict;
+        const double avt = 1.065 * act - au * vis[m] * X[m] * ivt;
+        acp[m] = al * X[m] * vis[m];
+        aX[m] += al * vis[m] * lfac - 0.065 * act + au * vis[m] + avt;
+        double av = (al * lfac + au) * X[m];
+        const double ivm = isv[m] * isv[m];
+#pragma unroll
+        for (int n = 0; n < ns; ++n) {
+          if (m == n) continue;
+          const double w = c_mix.wj_div_wi_1_4[m][n], sw = c_mix.sqrt_wiwj_8[m][n];
+          const double r = svm * isv[n], nm = 1 + r * w;
+          aX[n] += avt * nm * nm * sw;
+          const double ar = avt * X[n] * nm * sw * w * r;  // half the adjoint of ln(vis_m / vis_n) times 2
+          av += ar * ivm;
+          avis[n] -= ar * (isv[n] * isv[n]);
+        }
+        avis[m] += av;
+      }
+#pragma unroll
+      for (int l = 0; l < ns; ++l) aTv += avis[l] * vis[l] * dlv[l];
+    }
+    aT += aTv;
     // c = sqrt(gamma Ru T / mw)
-    const double agamma = ac * acoustic / (2 * gamma);
-    aT += ac * acoustic / (2 * t);
-    amw -= ac * acoustic / (2 * mw);
-    // X_l = Y_l mw / W_l
-    for (int l = 0; l < ns; ++l) {
-      aY[l] += aX[l] * mw * c_mix.imw[l];
-      amw += aX[l] * y[l] * c_mix.imw[l];
-    }
-    // gamma = cpt / cvt; mw = 1 / sum Y / W; cp_l(T)
+    const double acoustic = sqrt(gamma * kRuD * t * smw), hc = 0.5 * ac * acoustic;
+    const double agamma = hc / gamma;
+    aT += hc * it;
+    amw -= hc * smw;
+    // X_l = Y_l mw / W_l; gamma = cpt / cvt; mw = 1 / sum Y / W; cp_l(T)
+#pragma unroll
+    for (int l = 0; l < ns; ++l) amw += aX[l] * s.sv[l * P + p] * c_mix.imw[l];
     const double acpt = agamma / cvt, acvt = -agamma * gamma / cvt;
+#pragma unroll
     for (int l = 0; l < ns; ++l) {
-      aY[l] += acpt * cp[l] + acvt * (cp[l] - c_mix.ru_mw[l]) - amw * mw * mw * c_mix.imw[l];
-      acp[l] += (acpt + acvt) * y[l];
-      aT += acp[l] * dcp[l];
+      double h, cp;
+      mix_h_cp_one<double>(l, t, h, cp);
+      A.Y[(long long)l * P + p] += aX[l] * mw * c_mix.imw[l] + acpt * cp + acvt * (cp - c_mix.ru_mw[l]) -
+                                   amw * mw * mw * c_mix.imw[l];
+      aT += (acp[l] + (acpt + acvt) * s.sv[l * P + p]) * mix_dcp_dt_one(l, t);
     }
     A.rho[p] += arho;
     A.p[p] += ap;
     A.T[p] += aT;
-    for (int l = 0; l < ns; ++l) A.Y[(long long)l * P + p] += aY[l];
   }
 }
 
