@@ -255,8 +255,13 @@ void launch_adjoint_t(ostc_ctx *ctx, BlockRes &B, DevState in, unsigned mask, co
       k_adj_visc<1, false, NS><<<g1, blk, 0, ctx->stream>>>(b, in, B.dqb, nv, A);
     }
   }
-  if ((mask & OSTC_TERM_SOURCE) && ctx->der.reaction == 1)
-    k_adj_source<NS><<<grid_for(ctx, b.n, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, A);
+  if ((mask & OSTC_TERM_SOURCE) && ctx->der.reaction == 1) {
+    if (ctx->mixtab.listed)
+      k_adj_source_listed<NS><<<grid_for(ctx, b.n, 128), 128, 5 * ctx->der.n_spec * 128 * sizeof(double), ctx->stream>>>(
+          b, in, B.dqb, A);
+    else
+      k_adj_source<NS><<<grid_for(ctx, b.n, 128), 128, 0, ctx->stream>>>(b, in, B.dqb, A);
+  }
   k_adj_props<NS><<<grid_for(ctx, b.plane, 128), 128, 0, ctx->stream>>>(b, in, A);
   k_adj_ghost_cv<NS><<<grid_for(ctx, b.plane, 128), 128, 0, ctx->stream>>>(b, in, A, nv);
 }
@@ -659,6 +664,8 @@ bool set_mix_attrs(int nv) {
     set((const void *)k_mix_source<kFixedNS, true>, src);
     set((const void *)k_mix_chem_epi<0, true>, epi);
     set((const void *)k_mix_chem_epi<kFixedNS, true>, epi);
+    set((const void *)k_adj_source_listed<0>, 5 * ns * 128 * sizeof(double));
+    set((const void *)k_adj_source_listed<kFixedNS>, 5 * ns * 128 * sizeof(double));
   }
   set((const void *)k_adj_fvs<0, 0>, adj_fvs_smem_bytes<0>(nv));
   set((const void *)k_adj_fvs<1, 0>, adj_fvs_smem_bytes<1>(nv));

@@ -947,6 +947,130 @@ __global__ void __launch_bounds__(128, 4) k_adj_source(DevBlock b, DevState s, c
   }
 }
 
+// The same over the reaction lists with the species arrays in shared memory (as mix_chemistry_listed):
+// d ln kf / dT = b / T + Ea / T^2 for the Arrhenius types, d g / dT = -h / (Ru T^2) for the equilibrium constant;
+// only fall-off reactions take Dual evaluations.  [96 x 64 x 48, 19 reactions:
+// dense 0.65 ms of the VJP, listed 0.4]
+template <int NS>
+__global__ void __launch_bounds__(128, 4) k_adj_source_listed(DevBlock b, DevState s, const double *__restrict__ dqb,
+                                                             DevAdj A) {
+  extern __shared__ double adj_src_smem[];
+  const long long P = b.plane;
+  const int ns = OSTC_NS, nr = c_mix.nr;
+  auto col = [&](int a) { return ChemColumn{adj_src_smem + a * ns * 128 + threadIdx.x, 128}; };
+  const ChemColumn c = col(0), ac = col(1), aw = col(2), g = col(3), dg = col(4);
+  for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < b.n; n += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(n % b.mx);
+    const long long r0 = n / b.mx;
+    const int j = (int)(r0 % b.my), k = (int)(r0 / b.my);
+    const long long p = b.id(i, j, k);
+    const double rho = s.bv[p], t = s.bv[5 * P + p], jac = b.jac[p];
+    bool any = false;
+    for (int l = 0; l < ns; ++l) {
+      const double a = jac * dqb[(5 + l) * b.n + n] * c_mix.mw[l] * 1e+3;
+      aw(l) = a;
+      any = any || a != 0.0;
+      c(l) = rho * s.sv[l * P + p] * c_mix.imw[l] * 1e-3;
+      ac(l) = 0.0;
+    }
+    if (!any) continue;
+    const double lt = log(t), ti = 1.0 / t;
+    if (c_mix.use_gibbs) {
+      double gr[Spec<NS>::A];
+      mix_gibbs_rt<NS, double>(t, gr);
+#pragma unroll
+      for (int l = 0; l < ns; ++l) {
+        double h, cp;
+        mix_h_cp_one<double>(l, t, h, cp);
+        g(l) = gr[l];
+        // below t_low the Gibbs energy is evaluated at t_low, a constant
+        dg(l) = t < c_mix.t_low[l] ? 0.0 : -h / c_mix.ru_mw[l] * (ti * ti);
+      }
+    }
+    double aT = 0;
+#pragma unroll 1
+    for (int r = 0; r < nr; ++r) {
+      const int ty = c_mix.label[r], nf = c_mix.n_f[r], nb = c_mix.n_b[r], nn = c_mix.n_net[r];
+      double aq = 0, sg = 0, sdg = 0;
+      for (int e = 0; e < nn; ++e) {
+        const int m = c_mix.net[r][e];
+        const double nu = c_mix.nu[r][e];
+        aq += nu * aw(m);
+        if (c_mix.use_gibbs) {
+          sg += nu * g(m);
+          sdg += nu * dg(m);
+        }
+      }
+      if (aq == 0.0) continue;
+      double cc = 0;
+      if (ty >= 4)
+        for (int l = 0; l < ns; ++l) cc += c(l) * c_mix.third_body[r][l];
+      // kf with its derivatives in T and the third-body sum
+      double kf, kf_t, kf_c = 0;
+      if (ty > 4) {
+        const Dual a = reaction_kf<Dual>(r, Dual(t, 1.0), Dual(lt, ti), Dual(ti, -ti * ti), Dual(cc));
+        const Dual d = reaction_kf<Dual>(r, Dual(t), Dual(lt), Dual(ti), Dual(cc, 1.0));
+        kf = a.v;
+        kf_t = a.d;
+        kf_c = d.d;
+      } else {
+        kf = arrhenius(lt, ti, c_mix.A[r], c_mix.b[r], c_mix.Ea[r]);
+        kf_t = kf * (c_mix.b[r] + c_mix.Ea[r] * ti) * ti;
+        if (ty == 3) {
+          const double k2 = arrhenius(lt, ti, c_mix.A2[r], c_mix.b2[r], c_mix.Ea2[r]);
+          kf += k2;
+          kf_t += k2 * (c_mix.b2[r] + c_mix.Ea2[r] * ti) * ti;
+        } else if (ty == 4) {
+          kf_c = kf;
+          kf *= cc;
+          kf_t *= cc;
+        }
+      }
+      // kb: kf over the equilibrium constant, whose ln changes with T by -sdg - order / T; else REV coefficients
+      double kb = reaction_kb<double>(r, lt, ti, cc, kf, sg), kb_t = 0, kb_c = 0;
+      if (ty != 0 && ty != 2 && c_mix.use_gibbs) {
+        const double ratio = reaction_kb<double>(r, lt, ti, cc, 1.0, sg);
+        kb_t = ratio * kf_t + kb * (sdg + c_mix.order[r] * ti);
+        kb_c = ratio * kf_c;
+      } else if (kb != 0.0) {
+        kb_t = kb * (c_mix.b2[r] + c_mix.Ea2[r] * ti) * ti;
+        if (ty == 4) kb_c = kb / cc;
+      }
+      double p1 = 1.0, p2 = 1.0;
+      for (int e = 0; e < nf; ++e) {
+        double d = 1.0;  // product of the other molecules: d p1 / d c of this one
+        for (int q = 0; q < nf; ++q)
+          if (q != e) d *= c(c_mix.mol_f[r][q]);
+        ac(c_mix.mol_f[r][e]) += aq * kf * d;
+        p1 *= c(c_mix.mol_f[r][e]);
+      }
+      if (ty != 0) {
+        for (int e = 0; e < nb; ++e) {
+          double d = 1.0;
+          for (int q = 0; q < nb; ++q)
+            if (q != e) d *= c(c_mix.mol_b[r][q]);
+          ac(c_mix.mol_b[r][e]) -= aq * kb * d;
+          p2 *= c(c_mix.mol_b[r][e]);
+        }
+      }
+      const double akf = aq * p1, akb = ty != 0 ? -aq * p2 : 0.0;
+      aT += akf * kf_t + akb * kb_t;
+      if (ty >= 4) {
+        const double acc = akf * kf_c + akb * kb_c;
+        for (int l = 0; l < ns; ++l) ac(l) += acc * c_mix.third_body[r][l];
+      }
+    }
+    double arho = 0;
+    for (int l = 0; l < ns; ++l) {
+      const double a = ac(l) * c_mix.imw[l] * 1e-3;
+      arho += a * s.sv[l * P + p];
+      A.Y[(long long)l * P + p] += a * rho;
+    }
+    A.rho[p] += arho;
+    A.T[p] += aT;
+  }
+}
+
 // Reverse of the transport and acoustic properties (update_physical_properties<mixture>,
 // FieldOperation.cuh:107-134, compute_transport_property, Transport.cu:43-136) at every padded node:
 // adjoints of c, mu, lambda and rho*D_k -> adjoints of rho, p, T and Y.  Hand-written reverse of
