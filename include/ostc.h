@@ -213,7 +213,7 @@ int ostc_profile_steps(ostc_ctx *ctx, int n_steps, int max, const char **names, 
 
 /* Pin the kernel shape of one inviscid sweep (AWENO path) instead of the autotuner's choice:
  * precision 0 = FP64, 1 = mixed; dir 0/1/2 = x/y/z; variant 0.. (x: 0 only, one thread per face;
- * y/z: 0 column march, 1-3 shared-memory tiles of three shapes), or
+ * y/z: 0-3 shared-memory tiles of four shapes), or
  * -1 to return the direction to the autotuner (forgetting its cached result for these block shapes).
  * Every variant computes the same face fluxes with the same expressions; the choice changes speed,
  * not results.  Takes effect at the next step.  No reference counterpart (its sweep kernels have one

@@ -5,8 +5,7 @@
 //   k_cfl_dt           [local_time_step + min_of_arr x2 + D2H + update_dt_global] first stage only:
 //                      spectral radius, warp-shuffle min, one 64-bit atomicMin into a device scalar
 //   k_flux_x           [compute_convective_term_aweno_1D + CDSPart1D, x]: staged row tile, one face per thread
-//   k_flux_march<1|2>  [same, y and z]: each thread marches one column, coalesced across i, with a
-//                      per-thread ring of 2*ngg+1 nodes in shared memory (no halo re-reads)
+//   k_flux_tile<1|2>   [same, y and z]: a tile of i lanes x nodes along the sweep, one or more faces a thread
 //   k_visc_update      [viscous_flux_fv/gv/hv + update_cv_and_bv_rk + update_physical_properties]
 //                      3-D tile, face fluxes staged in shared memory, RK combine and EOS fused
 //   k_bc_group, k_bc_face  [apply_* of the boundary faces, in the reference priority order]
@@ -140,184 +139,16 @@ __global__ void __launch_bounds__(128, FluxXOcc<T>::blocks) k_flux_x(DevBlock b,
   }
 }
 
-// Asynchronous global -> shared copies (cp.async, Ampere and later, plain non-bulk form).
-__device__ __forceinline__ void cp_async8(void *smem_dst, const void *gsrc) {
-  const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// Resident 64-thread blocks per SM the march kernel is compiled for.
-template <typename T> struct MarchOcc { static constexpr int blocks = 4; };
-template <> struct MarchOcc<float> { static constexpr int blocks = 6; };
-
-// y (DIR = 1) or z (DIR = 2) sweep.  Thread (i, o) marches nodes c = s0..s1-1 of its column (o is
-// k for y, j for z); warps are contiguous in i, so every load of a new node is coalesced.  A
-// per-thread ring in shared memory keeps the last 2*NG+1 nodes' cv(5), p and node flux(5); the
-// metric row and Jacobian of the face's two nodes travel in registers.
-// FP32 instantiation: the raw FP64 data of the next node (cv 5, rho/u/v/w/p 5, metric row 3,
-// Jacobian 1) and the metric row + Jacobian of the face's right node are prefetched with cp.async
-// one iteration ahead (double-buffered) so their latency hides behind the face computation
-// (measured 1.18x).  FP64 instantiation: plain loads - the prefetch buffers would cut it from 4 to 3
-// resident blocks, which costs more than the latency it hides (measured 0.79x).  Segments of `seg`
-// nodes split long columns across blocks.
-template <int DIR, int NG, int RS, typename T>
-__global__ void __launch_bounds__(64, MarchOcc<T>::blocks) k_flux_march(DevBlock b, DevState s,
-                                                                         double *__restrict__ dq, int seg) {
-  constexpr int W = 2 * NG + 1;
-  constexpr int NV = 11;
-  constexpr int NRAW = 14;
-  constexpr bool PIPE = std::is_same_v<T, float>;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int nthr = blockDim.x * blockDim.y;
-  T *ring = reinterpret_cast<T *>(smraw);
-  // prefetch buffers (FP32 only): raw [2][NRAW][nthr], metric [2][4][nthr], 16-byte aligned
-  double *raw = reinterpret_cast<double *>(
-      (reinterpret_cast<size_t>(smraw) + (size_t)W * NV * nthr * sizeof(T) + 15) & ~(size_t)15);
-  double *mraw = raw + 2 * NRAW * nthr;
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int o = blockIdx.y * blockDim.y + threadIdx.y;
-  const int n_dir = DIR == 1 ? b.my : b.mz;
-  const int n_o = DIR == 1 ? b.mz : b.my;
-  if (i >= b.mx || o >= n_o) return;
-  const int s0 = blockIdx.z * seg;
-  if (s0 >= n_dir) return;
-  const int s1 = min(s0 + seg, n_dir);
-  const long long P = b.plane;
-  const long long stride = DIR == 1 ? (long long)b.pitch : (long long)b.pitch * b.sy;
-  const long long base = DIR == 1 ? b.id(i, 0, o) : b.id(i, o, 0);
-  const double *__restrict__ mrow = b.met + (long long)DIR * 3 * P;
-  auto R = [&](int slot, int v) -> T & { return ring[(slot * NV + v) * nthr + tid]; };
-  auto Raw = [&](int sl, int v) -> double & { return raw[(sl * NRAW + v) * nthr + tid]; };
-  auto Mraw = [&](int sl, int v) -> double & { return mraw[(sl * 4 + v) * nthr + tid]; };
-  auto prefetch_node = [&](int n, int sl) {
-    const long long p = b.chk(base + (long long)n * stride);
-#pragma unroll
-    for (int l = 0; l < 5; ++l) cp_async8(&Raw(sl, l), s.cv + l * P + p);
-#pragma unroll
-    for (int l = 0; l < 5; ++l) cp_async8(&Raw(sl, 5 + l), s.bv + l * P + p);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) cp_async8(&Raw(sl, 10 + c), mrow + c * P + p);
-    cp_async8(&Raw(sl, 13), b.jac + p);
-  };
-  auto prefetch_metric = [&](int n, int sl) {
-    const long long p = b.chk(base + (long long)n * stride);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) cp_async8(&Mraw(sl, c), mrow + c * P + p);
-    cp_async8(&Mraw(sl, 3), b.jac + p);
-  };
-  // node n from its raw FP64 values into the ring
-  auto commit_node = [&](int n, const double *cv, const double *bv, const double *km, double jac) {
-    const int slot = (n + NG) % W;
-    T bb[5], kk[3];
-#pragma unroll
-    for (int l = 0; l < 5; ++l) {
-      R(slot, l) = (T)cv[l];
-      bb[l] = (T)bv[l];
-    }
-    R(slot, 5) = bb[4];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) kk[c] = (T)km[c];
-    T f[5];
-    node_flux<T>(bb, (T)cv[4], kk, (T)jac, f);
-#pragma unroll
-    for (int l = 0; l < 5; ++l) R(slot, 6 + l) = f[l];
-  };
-  auto load_direct = [&](int n) {
-    const long long p = b.chk(base + (long long)n * stride);
-    double cv[5], bv[5], km[3];
-#pragma unroll
-    for (int l = 0; l < 5; ++l) {
-      cv[l] = s.cv[l * P + p];
-      bv[l] = s.bv[l * P + p];
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) km[c] = mrow[c * P + p];
-    commit_node(n, cv, bv, km, b.jac[p]);
-  };
-  for (int n = s0 - NG; n <= s0 + NG - 2; ++n) load_direct(n);
-  if constexpr (PIPE) {
-    // first stage: node s0-1+NG and the right-node metric of face s0-1/2 (node s0)
-    prefetch_node(s0 - 1 + NG, 0);
-    prefetch_metric(s0, 0);
-    cp_async_commit();
-  }
-  T fprev[5] = {T(0), T(0), T(0), T(0), T(0)};
-  long long pc = b.chk(base + (long long)(s0 - 1) * stride);
-  T mt0[3] = {(T)mrow[pc], (T)mrow[P + pc], (T)mrow[2 * P + pc]};
-  T j0 = (T)b.jac[pc];
-  for (int c = s0 - 1; c < s1; ++c) {
-    T mt1[3], j1;
-    if constexpr (PIPE) {
-      cp_async_wait_all();
-      // both prefetch buffers alternate slots, so a copy never targets the slot just read
-      const int ms = (c - s0 + 1) & 1;
-      double cv[5], bv[5], km[3];
-#pragma unroll
-      for (int l = 0; l < 5; ++l) {
-        cv[l] = Raw(ms, l);
-        bv[l] = Raw(ms, 5 + l);
-      }
-#pragma unroll
-      for (int q3 = 0; q3 < 3; ++q3) km[q3] = Raw(ms, 10 + q3);
-      commit_node(c + NG, cv, bv, km, Raw(ms, 13));
-#pragma unroll
-      for (int q3 = 0; q3 < 3; ++q3) mt1[q3] = (T)Mraw(ms, q3);
-      j1 = (T)Mraw(ms, 3);
-      if (c + 1 < s1) {
-        prefetch_node(c + 1 + NG, ms ^ 1);
-        prefetch_metric(c + 2, ms ^ 1);
-        cp_async_commit();
-      }
-    } else {
-      load_direct(c + NG);
-      const long long pn = b.chk(pc + stride);
-#pragma unroll
-      for (int q3 = 0; q3 < 3; ++q3) mt1[q3] = (T)mrow[q3 * P + pn];
-      j1 = (T)b.jac[pn];
-      pc = pn;
-    }
-    const int b0 = (c + 1) % W;
-    auto q = [&](int st, int v) -> T {
-      int sl = b0 + st;
-      sl = sl >= W ? sl - W : sl;
-      return R(sl, v);
-    };
-    T fc[5];
-    aweno_face_flux<NG, RS, T>(q, mt0, mt1, j0, j1, fc);
-    if (c >= s0) {
-      const long long qi = DIR == 1 ? b.iq(i, c, o) : b.iq(i, o, c);
-      const bool cds = c < n_dir - 2 * NG;
-      const int bc = c % W;  // slot of node c - NG
-      auto f = [&](int m, int l) -> T {
-        int sl = bc + NG + m;
-        sl = sl >= W ? sl - W : sl;
-        return R(sl, 6 + l);
-      };
-#pragma unroll
-      for (int l = 0; l < 5; ++l) {
-        double d = dq[l * b.n + qi];
-        d -= (double)(fc[l] - fprev[l]);
-        if (cds) d += (double)cds_correction<NG, T>(f, l);
-        dq[l * b.n + qi] = d;
-      }
-    }
-#pragma unroll
-    for (int l = 0; l < 5; ++l) fprev[l] = fc[l];
-#pragma unroll
-    for (int q3 = 0; q3 < 3; ++q3) mt0[q3] = mt1[q3];
-    j0 = j1;
-  }
-  if constexpr (PIPE) cp_async_wait_all();
-}
-
 // y / z sweep as a tile: a block of TXL consecutive i (coalesced rows) x TD threads along the sweep
 // direction stages TF - 1 + 2*NG nodes per lane in shared memory (cv, p, node flux, metric row,
 // Jacobian), computes FPT faces per thread and finalises TF - 1 nodes per lane, as the x sweep does
-// for rows.  Against the column march it trades (TF - 1 + 2 NG) / (TF - 1) node loads per node for
-// independent faces with no serial dependence along the column; the autotuner picks between them.
+// for rows.  Bound by FP64 (FP32) arithmetic, ~50 % of the pipe, and the latency of the staging loads.  The
+// node's sum goes to dq by an atomicAdd whose result nobody reads, a reduction at L2: a load and a store made
+// the block hold its shared memory and registers until the load came back.  One thread adds to an entry in a
+// launch, so the sum is the plain one.  With it 512 x 256 x 128 WENO7 + HLLC, FP64: 3.13 -> 2.51 ms a sweep,
+// 385 x 257 x 129, FP32: 1.33 -> 1.19 (16 x 8 x 2 and 32 x 8 x 2 tiles).  A longer tile of half the lanes
+// re-reads fewer halo nodes (1.26 loads a node, 1.53 at TF = 16, NG = 4): 2.48 and 1.13 ms.  One thread marching
+// a column with a ring of nodes in shared memory, each node loaded once, took 3.84 and 2.17.
 // TF = TD * FPT faces per tile along the sweep (TF - 1 nodes finalised), FPT faces per thread.
 template <int NG, int TXL, int TF, typename T>
 constexpr size_t tile_smem_bytes() {
@@ -330,7 +161,7 @@ constexpr size_t tile_smem_bytes() {
 // blocks; the FP64 32-lane variant is shared-memory limited to two blocks anyway.
 template <typename T, int TXL, int NT>
 __host__ __device__ constexpr int tile_min_blocks() {
-  return sizeof(T) == 4 ? (NT == 256 ? 3 : 65536 / (NT * 128)) : (TXL == 16 ? (NT == 128 ? 3 : 2) : 2);
+  return sizeof(T) == 4 ? (NT == 256 ? 3 : 65536 / (NT * 128)) : (TXL <= 16 ? (NT == 128 ? 3 : 2) : 2);
 }
 
 template <int DIR, int NG, int RS, typename T, int TXL, int TD, int FPT>
@@ -405,20 +236,12 @@ __global__ void __launch_bounds__(TXL * TD, tile_min_blocks<T, TXL, TXL * TD>())
       const bool cds = d < nd - 2 * NG;
 #pragma unroll
       for (int l = 0; l < 5; ++l) {
-        double v = dq[l * b.n + qi];
-        v -= (double)(sfc[(l * TF + t) * TXL + lane] - sfc[(l * TF + t - 1) * TXL + lane]);
+        double v = (double)(sfc[(l * TF + t - 1) * TXL + lane] - sfc[(l * TF + t) * TXL + lane]);
         if (cds) v += (double)cds_correction<NG, T>(f, l);
-        dq[l * b.n + qi] = v;
+        atomicAdd(dq + l * b.n + qi, v);
       }
     }
   }
-}
-
-// Dynamic shared memory of one 64-thread march block: the ring, plus the prefetch buffers in FP32.
-template <typename T>
-constexpr size_t march_smem_bytes(int ng) {
-  return (size_t)(2 * ng + 1) * 11 * 64 * sizeof(T) +
-         (std::is_same_v<T, float> ? 16 + (2 * 14 + 8) * 64 * sizeof(double) : 0);
 }
 
 // ------------------------------------------------------- primitive reconstruction + Riemann

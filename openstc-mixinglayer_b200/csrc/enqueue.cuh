@@ -266,15 +266,16 @@ void launch_adjoint_t(ostc_ctx *ctx, BlockRes &B, DevState in, unsigned mask, co
   k_adj_ghost_cv<NS><<<grid_for(ctx, b.plane, 128), 128, 0, ctx->stream>>>(b, in, A, nv);
 }
 
-// y / z sweep variants: 0 = column march, 1..3 = tiles of the shapes below (per precision: rows
-// of 128 bytes, and a block small enough for the register budget of the FP64 face arithmetic).
+// y / z sweep variants: tiles of the shapes below, {lanes, threads along the sweep, faces per thread}.  Rows of
+// 64 bytes and 32 faces (variant 0) re-read the fewest halo nodes: 512 x 256 x 128, FP64, 2.48 ms against 2.51
+// of the next, 385 x 257 x 129, FP32, 1.13 against 1.19, 257 x 129, FP64, 11.1 us against 12.6; the others (rows
+// of 128 bytes) fit other extents with less of a tile left empty: 193 x 101 x 75, FP64, 178 us against 177.
 template <typename T> struct YzShapes;
-// {lanes, threads along the sweep, faces per thread} of tile variants 1..3
 template <> struct YzShapes<float> {
-  static constexpr int X1 = 32, D1 = 16, F1 = 1, X2 = 32, D2 = 8, F2 = 2, X3 = 32, D3 = 4, F3 = 4;
+  static constexpr int X0 = 16, D0 = 16, F0 = 2, X1 = 32, D1 = 16, F1 = 1, X2 = 32, D2 = 8, F2 = 2, X3 = 32, D3 = 4, F3 = 4;
 };
 template <> struct YzShapes<double> {
-  static constexpr int X1 = 16, D1 = 16, F1 = 1, X2 = 16, D2 = 8, F2 = 2, X3 = 32, D3 = 4, F3 = 4;
+  static constexpr int X0 = 8, D0 = 16, F0 = 2, X1 = 16, D1 = 16, F1 = 1, X2 = 16, D2 = 8, F2 = 2, X3 = 32, D3 = 4, F3 = 4;
 };
 constexpr int kYzVariants = 4;
 
@@ -282,28 +283,19 @@ template <typename T, int D, int N, int R>
 void launch_yz_v(ostc_ctx *ctx, BlockRes &B, DevState in, int variant) {
   const DevBlock &b = B.db;
   const int n_dir = D == 1 ? b.my : b.mz, n_o = D == 1 ? b.mz : b.my;
-  if (variant >= 1 && variant <= 3) {
-    using S = YzShapes<T>;
+  using S = YzShapes<T>;
 #define OSTC_TILE(X, DD, F)                                                                             \
   {                                                                                                   \
     constexpr int TF = DD * F;                                                                        \
     dim3 grid((b.mx + X - 1) / X, (n_dir + TF - 2) / (TF - 1), n_o);                                   \
-    k_flux_tile<D, N, R, T, X, DD, F><<<grid, dim3(X, DD), tile_smem_bytes<N, X, TF, T>(), ctx->stream>>>( \
-        b, in, B.dq);                                                                                 \
+    k_flux_tile<D, N, R, T, X, DD, F>                                                                 \
+        <<<grid, dim3(X, DD), tile_smem_bytes<N, X, TF, T>(), ctx->stream>>>(b, in, B.dq);             \
   }
-    if (variant == 1) OSTC_TILE(S::X1, S::D1, S::F1)
-    else if (variant == 2) OSTC_TILE(S::X2, S::D2, S::F2)
-    else OSTC_TILE(S::X3, S::D3, S::F3)
+  if (variant == 1) OSTC_TILE(S::X1, S::D1, S::F1)
+  else if (variant == 2) OSTC_TILE(S::X2, S::D2, S::F2)
+  else if (variant == 3) OSTC_TILE(S::X3, S::D3, S::F3)
+  else OSTC_TILE(S::X0, S::D0, S::F0)
 #undef OSTC_TILE
-    return;
-  }
-  // split columns into segments so that the grid fills the GPU at least ~4 waves deep
-  const long long cols = (long long)((b.mx + 31) / 32) * ((n_o + 1) / 2);
-  int nseg = (int)std::max<long long>(1, (ctx->sm_count * 12 + cols - 1) / cols);
-  int seg = std::max(2 * N, (n_dir + nseg - 1) / nseg);
-  nseg = (n_dir + seg - 1) / seg;
-  dim3 grid((b.mx + 31) / 32, (n_o + 1) / 2, nseg);
-  k_flux_march<D, N, R, T><<<grid, dim3(32, 2, 1), march_smem_bytes<T>(N), ctx->stream>>>(b, in, B.dq, seg);
 }
 
 // x sweep variants: 0 = one thread per face (k_flux_x) is the only shape; splitting each face over
@@ -437,7 +429,7 @@ int launch_flux(ostc_ctx *ctx, BlockRes &B, DevState in) {
     launch_x<T>(ctx, B, in, v < 0 ? 0 : v);
     end_t(ctx, tok);
   }
-  // y and z: the variant the autotuner chose for this block and precision (column march by default)
+  // y and z: the variant the autotuner chose for this block and precision (0 until it ran)
   for (int dir = 1; dir <= (is3d ? 2 : 1); ++dir) {
     const int v = B.yz_var[ctx->precision == OSTC_PREC_MIXED][dir - 1];
     long tok = begin_t(ctx, dir == 1 ? "flux_y" : "flux_z");
@@ -602,32 +594,17 @@ DevState state_of(BlockRes &B, int s) {
   return d;
 }
 
-// The march kernels stage 2*ngg+1 nodes x 11 values x 64 threads (plus the FP32 prefetch buffers)
-// in dynamic shared memory (up to 51 KB); raise the per-kernel limit once, outside any stream capture.
+// The sweep tiles stage their nodes in dynamic shared memory; raise the per-kernel limits once, outside any
+// stream capture.
 template <typename T>
-bool set_march_attrs() {
+bool set_sweep_attrs() {
   bool ok = true;
-  auto set = [&](const void *fn, int ng) {
-    const int bytes = (int)march_smem_bytes<T>(ng);
-    ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
-  };
-  set((const void *)k_flux_march<1, 3, 1, T>, 3);
-  set((const void *)k_flux_march<1, 3, 3, T>, 3);
-  set((const void *)k_flux_march<1, 3, 4, T>, 3);
-  set((const void *)k_flux_march<1, 4, 1, T>, 4);
-  set((const void *)k_flux_march<1, 4, 3, T>, 4);
-  set((const void *)k_flux_march<1, 4, 4, T>, 4);
-  set((const void *)k_flux_march<2, 3, 1, T>, 3);
-  set((const void *)k_flux_march<2, 3, 3, T>, 3);
-  set((const void *)k_flux_march<2, 3, 4, T>, 3);
-  set((const void *)k_flux_march<2, 4, 1, T>, 4);
-  set((const void *)k_flux_march<2, 4, 3, T>, 4);
-  set((const void *)k_flux_march<2, 4, 4, T>, 4);
   auto tset = [&](const void *fn, size_t bytes) {
     ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
   };
   using S = YzShapes<T>;
 #define OSTC_TSET(D, N, R)                                                                                      \
+  tset((const void *)k_flux_tile<D, N, R, T, S::X0, S::D0, S::F0>, tile_smem_bytes<N, S::X0, S::D0 * S::F0, T>()); \
   tset((const void *)k_flux_tile<D, N, R, T, S::X1, S::D1, S::F1>, tile_smem_bytes<N, S::X1, S::D1 * S::F1, T>()); \
   tset((const void *)k_flux_tile<D, N, R, T, S::X2, S::D2, S::F2>, tile_smem_bytes<N, S::X2, S::D2 * S::F2, T>()); \
   tset((const void *)k_flux_tile<D, N, R, T, S::X3, S::D3, S::F3>, tile_smem_bytes<N, S::X3, S::D3 * S::F3, T>());
