@@ -74,22 +74,29 @@ template <> struct FluxXOcc<float> { static constexpr int blocks = 5; };
 // x sweep.  A block of 128 threads stages 127 + 2*NG nodes of one (j,k) row in shared memory
 // (coalesced along i), computes the 128 faces i0-1/2 .. i0+126+1/2 (one per thread) and finalises
 // the 127 nodes between them: dq = -(fc(i+1/2) - fc(i-1/2)) + central correction.
-template <int NG, int RS, typename T>
-__global__ void __launch_bounds__(128, FluxXOcc<T>::blocks) k_flux_x(DevBlock b, DevState s, double *__restrict__ dq) {
+// RECT (rectilinear block): only the metric row's own component is staged, and the face flux runs on an
+// axis-aligned normal (air_math.cuh); the y / z tiles likewise.  FP64 arithmetic bounds the sweep, so a block that
+// can leave part of it out does: 512 x 256 x 128, WENO7 + HLLC, FP64, 2.74 -> 2.07 ms (four blocks an SM,
+// three: 2.14), y and z tiles 2.50 -> 1.85 (3: 1.97); 385 x 257 x 129, FP32, 1.07 -> 0.93, 1.13 -> 0.89 ms.
+template <int NG, int RS, typename T, bool RECT>
+__global__ void __launch_bounds__(128, RECT && sizeof(T) == 8 ? 4 : FluxXOcc<T>::blocks) k_flux_x(DevBlock b, DevState s, double *__restrict__ dq) {
   constexpr int L = 127;
   constexpr int NP = L + 2 * NG;
+  constexpr int AX = RECT ? 0 : -1, NM = RECT ? 1 : 3;  // metric components staged, then the Jacobian
   __shared__ T sq[6][NP];
   __shared__ T sf[5][NP];
-  __shared__ T sm[4][NP];
+  __shared__ T sm[NM + 1][NP];
   __shared__ T sfc[5][128];
   const int t = threadIdx.x;
   const int i0 = blockIdx.x * L;
   const int j = blockIdx.y, k = blockIdx.z;
   const long long P = b.plane;
   const long long base = b.id(0, j, k);
-  for (int n = t; n < NP; n += 128) {
-    const int i = i0 - NG + n;
-    if (i < b.mx + NG) {
+  // two rounds, unrolled: the second (7 threads) would otherwise wait for its loads after the first
+#pragma unroll
+  for (int rd = 0; rd < (NP + 127) / 128; ++rd) {
+    const int n = t + rd * 128, i = i0 - NG + n;
+    if (n < NP && i < b.mx + NG) {
       const long long p = base + i;
       T bb[5], kk[3];
 #pragma unroll
@@ -99,14 +106,14 @@ __global__ void __launch_bounds__(128, FluxXOcc<T>::blocks) k_flux_x(DevBlock b,
       }
       sq[5][n] = bb[4];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
+      for (int c = 0; c < NM; ++c) {
         kk[c] = (T)b.met[c * P + p];
         sm[c][n] = kk[c];
       }
       const T jj = (T)b.jac[p];
-      sm[3][n] = jj;
+      sm[NM][n] = jj;
       T f[5];
-      node_flux<T>(bb, (T)s.cv[4 * P + p], kk, jj, f);
+      node_flux<T, AX>(bb, (T)s.cv[4 * P + p], kk, jj, f);
 #pragma unroll
       for (int l = 0; l < 5; ++l) sf[l][n] = f[l];
     }
@@ -115,10 +122,14 @@ __global__ void __launch_bounds__(128, FluxXOcc<T>::blocks) k_flux_x(DevBlock b,
   const int face = i0 - 1 + t;
   if (face < b.mx) {
     auto q = [&](int st, int v) -> T { return sq[v][t + st]; };
-    const T mt0[3] = {sm[0][t + NG - 1], sm[1][t + NG - 1], sm[2][t + NG - 1]};
-    const T mt1[3] = {sm[0][t + NG], sm[1][t + NG], sm[2][t + NG]};
+    T mt0[3], mt1[3];
+#pragma unroll
+    for (int c = 0; c < NM; ++c) {
+      mt0[c] = sm[c][t + NG - 1];
+      mt1[c] = sm[c][t + NG];
+    }
     T fc[5];
-    aweno_face_flux<NG, RS, T>(q, mt0, mt1, sm[3][t + NG - 1], sm[3][t + NG], fc);
+    aweno_face_flux<NG, RS, T, AX>(q, mt0, mt1, sm[NM][t + NG - 1], sm[NM][t + NG], fc);
 #pragma unroll
     for (int l = 0; l < 5; ++l) sfc[l][t] = fc[l];
   }
@@ -150,22 +161,23 @@ __global__ void __launch_bounds__(128, FluxXOcc<T>::blocks) k_flux_x(DevBlock b,
 // re-reads fewer halo nodes (1.26 loads a node, 1.53 at TF = 16, NG = 4): 2.48 and 1.13 ms.  One thread marching
 // a column with a ring of nodes in shared memory, each node loaded once, took 3.84 and 2.17.
 // TF = TD * FPT faces per tile along the sweep (TF - 1 nodes finalised), FPT faces per thread.
-template <int NG, int TXL, int TF, typename T>
+template <int NG, int TXL, int TF, typename T, bool RECT>
 constexpr size_t tile_smem_bytes() {
-  return (size_t)(15 * (TF - 1 + 2 * NG) + 5 * TF) * TXL * sizeof(T);
+  return (size_t)((RECT ? 13 : 15) * (TF - 1 + 2 * NG) + 5 * TF) * TXL * sizeof(T);
 }
 
 // Resident blocks per SM a tile variant is compiled for: FP32 variants at 128 registers per thread,
 // but three 256-thread blocks (80 registers, measured faster despite small spills); FP64 16-lane
 // variants (half the shared memory of the 32-lane ones) at three 128-thread or two 256-thread
-// blocks; the FP64 32-lane variant is shared-memory limited to two blocks anyway.
+// blocks (128 threads on a rectilinear block: four); the FP64 32-lane variant is shared-memory limited to two
+// blocks anyway.
 template <typename T, int TXL, int NT>
 __host__ __device__ constexpr int tile_min_blocks() {
   return sizeof(T) == 4 ? (NT == 256 ? 3 : 65536 / (NT * 128)) : (TXL <= 16 ? (NT == 128 ? 3 : 2) : 2);
 }
 
-template <int DIR, int NG, int RS, typename T, int TXL, int TD, int FPT>
-__global__ void __launch_bounds__(TXL * TD, tile_min_blocks<T, TXL, TXL * TD>())
+template <int DIR, int NG, int RS, typename T, int TXL, int TD, int FPT, bool RECT>
+__global__ void __launch_bounds__(TXL * TD, RECT && sizeof(T) == 8 && TXL * TD == 128 && TXL <= 16 ? 4 : tile_min_blocks<T, TXL, TXL * TD>())
     k_flux_tile(DevBlock b, DevState s, double *__restrict__ dq) {
   constexpr int TF = TD * FPT;
   constexpr int L = TF - 1;
@@ -173,8 +185,9 @@ __global__ void __launch_bounds__(TXL * TD, tile_min_blocks<T, TXL, TXL * TD>())
   extern __shared__ __align__(16) unsigned char smraw[];
   T *sq = reinterpret_cast<T *>(smraw);  // [6][NP][TXL]  cv 0..4, p
   T *sf = sq + 6 * NP * TXL;             // [5][NP][TXL]  node flux
-  T *smt = sf + 5 * NP * TXL;            // [4][NP][TXL]  metric row, Jacobian
-  T *sfc = smt + 4 * NP * TXL;           // [5][TF][TXL]  face flux
+  constexpr int AX = RECT ? DIR : -1, NM = RECT ? 1 : 3, C0 = RECT ? DIR : 0;  // metric components C0 .. C0 + NM - 1
+  T *smt = sf + 5 * NP * TXL;            // [NM + 1][NP][TXL]  metric row, Jacobian
+  T *sfc = smt + (NM + 1) * NP * TXL;    // [5][TF][TXL]  face flux
   const int lane = threadIdx.x;
   const int i = blockIdx.x * TXL + lane;
   const int d0 = blockIdx.y * L;
@@ -187,9 +200,10 @@ __global__ void __launch_bounds__(TXL * TD, tile_min_blocks<T, TXL, TXL * TD>())
   const double *__restrict__ mrow = b.met + (long long)DIR * 3 * P;
   auto at = [&](T *a, int v, int n) -> T & { return a[(v * NP + n) * TXL + lane]; };
   if (lane_ok) {
-    for (int n = threadIdx.y; n < NP; n += TD) {
-      const int d = d0 - NG + n;
-      if (d >= nd + NG) continue;
+#pragma unroll
+    for (int rd = 0; rd < (NP + TD - 1) / TD; ++rd) {
+      const int n = threadIdx.y + rd * TD, d = d0 - NG + n;
+      if (n >= NP || d >= nd + NG) continue;
       const long long p = b.chk(base + (long long)d * stride);
       T bb[5], kk[3];
 #pragma unroll
@@ -199,14 +213,14 @@ __global__ void __launch_bounds__(TXL * TD, tile_min_blocks<T, TXL, TXL * TD>())
       }
       at(sq, 5, n) = bb[4];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        kk[c] = (T)mrow[c * P + p];
-        at(smt, c, n) = kk[c];
+      for (int c = 0; c < NM; ++c) {
+        kk[C0 + c] = (T)mrow[(C0 + c) * P + p];
+        at(smt, c, n) = kk[C0 + c];
       }
       const T jj = (T)b.jac[p];
-      at(smt, 3, n) = jj;
+      at(smt, NM, n) = jj;
       T f[5];
-      node_flux<T>(bb, (T)s.cv[4 * P + p], kk, jj, f);
+      node_flux<T, AX>(bb, (T)s.cv[4 * P + p], kk, jj, f);
 #pragma unroll
       for (int l = 0; l < 5; ++l) at(sf, l, n) = f[l];
     }
@@ -217,10 +231,14 @@ __global__ void __launch_bounds__(TXL * TD, tile_min_blocks<T, TXL, TXL * TD>())
     const int face = d0 - 1 + t;  // left node of this face
     if (lane_ok && face < nd) {
       auto q = [&](int st, int v) -> T { return at(sq, v, t + st); };
-      const T mt0[3] = {at(smt, 0, t + NG - 1), at(smt, 1, t + NG - 1), at(smt, 2, t + NG - 1)};
-      const T mt1[3] = {at(smt, 0, t + NG), at(smt, 1, t + NG), at(smt, 2, t + NG)};
+      T mt0[3], mt1[3];
+#pragma unroll
+      for (int c = 0; c < NM; ++c) {
+        mt0[C0 + c] = at(smt, c, t + NG - 1);
+        mt1[C0 + c] = at(smt, c, t + NG);
+      }
       T fc[5];
-      aweno_face_flux<NG, RS, T>(q, mt0, mt1, at(smt, 3, t + NG - 1), at(smt, 3, t + NG), fc);
+      aweno_face_flux<NG, RS, T, AX>(q, mt0, mt1, at(smt, NM, t + NG - 1), at(smt, NM, t + NG), fc);
 #pragma unroll
       for (int l = 0; l < 5; ++l) sfc[(l * TF + t) * TXL + lane] = fc[l];
     }
@@ -443,6 +461,36 @@ __device__ __forceinline__ void viscous_face(int d, const VA &V, const MA &Mt, T
   fv[3] = um * fv[0] + vm * fv[1] + wm * fv[2] + cond * (nx * gx[3] + ny * gy[3] + nz * gz[3]);
 }
 
+// The same on a rectilinear block, where only the diagonal metric entries are non-zero: Mt(c, s) is entry
+// (c, c) for c = 0..2 and the Jacobian for c = 3.  Each velocity derivative is one difference, the stress
+// components of the face normal need four cross differences instead of eight, and T only its normal one.
+template <typename T, bool DIM3, class VA, class MA>
+__device__ __forceinline__ void viscous_face_rect(int d, const VA &V, const MA &Mt, T iprandtl, const T *vref, T *fv) {
+  const int e[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
+  T m[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) m[c] = T(0.5) * (Mt(c, 0) + Mt(c, 1));
+  auto grad = [&](int q, int c) -> T {
+    if (c == d) return (V(q, e[d][0], e[d][1], e[d][2]) - V(q, 0, 0, 0)) * m[c];
+    if (c == 2 && !DIM3) return T(0);
+    const int a0 = e[c][0], a1 = e[c][1], a2 = e[c][2];
+    return T(0.25) * (V(q, a0, a1, a2) - V(q, -a0, -a1, -a2) + V(q, e[d][0] + a0, e[d][1] + a1, e[d][2] + a2) -
+                      V(q, e[d][0] - a0, e[d][1] - a1, e[d][2] - a2)) * m[c];
+  };
+  const int t1 = (d + 1) % 3, t2 = (d + 2) % 3;
+  const T mul = T(0.5) * (V(4, 0, 0, 0) + V(4, e[d][0], e[d][1], e[d][2]));
+  const T n = T(0.5) * (Mt(d, 0) * Mt(3, 0) + Mt(d, 1) * Mt(3, 1));
+  const T nm = n * mul;
+  fv[d] = nm * (T(4) * grad(d, d) - T(2) * grad(t1, t1) - T(2) * grad(t2, t2)) * T(1.0 / 3.0);
+  fv[t1] = nm * (grad(d, t1) + grad(t1, d));
+  fv[t2] = nm * (grad(d, t2) + grad(t2, d));
+  const T cp = T(kGamma * kRuD / kMwD / (kGamma - 1));
+  T work = mul * iprandtl * cp * (n * grad(3, d));
+#pragma unroll
+  for (int q = 0; q < 3; ++q) work += (vref[q] + T(0.5) * (V(q, 0, 0, 0) + V(q, e[d][0], e[d][1], e[d][2]))) * fv[q];
+  fv[3] = work;
+}
+
 struct StageArgs {
   DevState in, qn, out;
   double a, bcoef, c;
@@ -460,23 +508,28 @@ struct StageArgs {
 // Jacobian (no face of plane k reads the metric of plane k-1), each with a one-node halo in i and j,
 // loaded once (coalesced along i).  Every face flux is computed once: x and y faces of plane k into
 // shared memory, the z face k+1/2 in registers (carried to the next plane as k-1/2).
-template <typename T, bool DIM3, int TX, int TY>
+// RECT (rectilinear block): three metric planes and the Jacobian are staged instead of ten planes, and half the
+// cross differences are formed: 512 x 256 x 128, FP64, 2.21 -> 1.45 ms, 385 x 257 x 129, FP32, 1.14 -> 0.88.
+template <typename T, bool DIM3, int TX, int TY, bool RECT>
 constexpr size_t visc_smem_bytes() {
-  return sizeof(T) * ((DIM3 ? 3 * 5 + 2 * 10 : 15) * (TY + 2) * (TX + 2) + TY * (TX + 1) * 4 + (TY + 1) * TX * 4);
+  return sizeof(T) * (((DIM3 ? 3 : 1) * 5 + (DIM3 ? 2 : 1) * (RECT ? 4 : 10)) * (TY + 2) * (TX + 2) + TY * (TX + 1) * 4 +
+                      (TY + 1) * TX * 4);
 }
 
-template <typename T, bool DIM3, int TX, int TY>
+template <typename T, bool DIM3, int TX, int TY, bool RECT>
 // FP64: two blocks per SM at up to 255 registers; three fit in shared memory, but their 168-register
-// cap measured 5 % slower (40.1 against 38.05 ms per AWENO7 + HLLC step at 512 x 256 x 128)
-__global__ void __launch_bounds__(TX *TY, sizeof(T) == 8 ? 2 : 4) k_visc_update(DevBlock b, StageArgs a, double *__restrict__ dq,
+// cap measured 5 % slower (40.1 against 38.05 ms per AWENO7 + HLLC step at 512 x 256 x 128).  RECT needs less of
+// both: FP64 four blocks (1.44 ms; three 1.52, five 1.87), FP32 six (0.88 ms; eight 1.01)
+__global__ void __launch_bounds__(TX *TY, sizeof(T) == 8 ? (RECT ? 4 : 2) : (RECT ? 6 : 4)) k_visc_update(DevBlock b, StageArgs a, double *__restrict__ dq,
                                                                       int kseg) {
   constexpr int NP = DIM3 ? 3 : 1;  // planes in the u, v, w, T, mu ring
   constexpr int NM = DIM3 ? 2 : 1;  // planes in the metric ring
+  constexpr int NV = RECT ? 4 : 10;  // metric entries and Jacobian
   constexpr int SX = TX + 2, SY = TY + 2;
-  constexpr int NS = (NP * 5 + NM * 10) * SY * SX;  // staged values
+  constexpr int NS = (NP * 5 + NM * NV) * SY * SX;  // staged values
   extern __shared__ __align__(16) unsigned char vsm_raw[];
   auto sv = reinterpret_cast<T(*)[5][SY][SX]>(vsm_raw);
-  auto sm = reinterpret_cast<T(*)[10][SY][SX]>(vsm_raw + sizeof(T) * NP * 5 * SY * SX);
+  auto sm = reinterpret_cast<T(*)[NV][SY][SX]>(vsm_raw + sizeof(T) * NP * 5 * SY * SX);
   auto fxs = reinterpret_cast<T(*)[TX + 1][4]>(vsm_raw + sizeof(T) * NS);
   auto fys = reinterpret_cast<T(*)[TX][4]>(vsm_raw + sizeof(T) * (NS + TY * (TX + 1) * 4));
   auto mslot = [](int kk) { return DIM3 ? (kk & 1) : 0; };  // kk >= -1
@@ -513,13 +566,14 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 8 ? 2 : 4) k_visc_update(
       sv[slot][2][y][x] = (T)(a.in.bv[3 * P + p] - ref[2]);
       sv[slot][3][y][x] = (T)(a.in.bv[5 * P + p] - ref[3]);
       sv[slot][4][y][x] = (T)a.in.mul[p];
+      // metric entry r of the staged ones: all, or the diagonal
       if constexpr (std::is_same_v<T, float>) {
 #pragma unroll
-        for (int r = 0; r < 10; ++r) sm[ms][r][y][x] = b.met32[r * P + p];
+        for (int r = 0; r < NV; ++r) sm[ms][r][y][x] = b.met32[(r == NV - 1 ? 9 : RECT ? 4 * r : r) * P + p];
       } else {
 #pragma unroll
-        for (int r = 0; r < 9; ++r) sm[ms][r][y][x] = (T)b.met[r * P + p];
-        sm[ms][9][y][x] = (T)b.jac[p];
+        for (int r = 0; r < NV - 1; ++r) sm[ms][r][y][x] = (T)b.met[(RECT ? 4 * r : r) * P + p];
+        sm[ms][NV - 1][y][x] = (T)b.jac[p];
       }
     }
   };
@@ -536,7 +590,8 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 8 ? 2 : 4) k_visc_update(
       if (d == 1) return sm[m0][r][y + 1][x];
       return sm[mslot(kk + 1)][r][y][x];
     };
-    viscous_face<T, DIM3>(d, V, Mt, ipr, tref, fv);
+    if constexpr (RECT) viscous_face_rect<T, DIM3>(d, V, Mt, ipr, tref, fv);
+    else viscous_face<T, DIM3>(d, V, Mt, ipr, tref, fv);
   };
   T fz_prev[4] = {T(0), T(0), T(0), T(0)};
   if (a.viscous) {

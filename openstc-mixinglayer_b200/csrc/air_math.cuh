@@ -37,6 +37,23 @@ __device__ __forceinline__ double sutherland(double t) {
   return 1.7894e-5 * pow(t / 288.16, 1.5) * (288.16 + 110) / (t + 110);
 }
 
+// ------------------------------------------------------------------ axis-aligned metrics
+//
+// AX: the component of the metric row k that a sweep of a rectilinear block carries (DevBlock::rect: the
+// off-diagonal metric entries are zero); -1: all three.  The other two terms of every product with k are
+// zeros then and are left out.
+template <int AX, typename T>
+__device__ __forceinline__ T kdot(const T *k, const T *v) {
+  if constexpr (AX < 0) return k[0] * v[0] + k[1] * v[1] + k[2] * v[2];
+  else return k[AX] * v[AX];
+}
+// a + b k[q]
+template <int AX, typename T>
+__device__ __forceinline__ T kadd(T a, T b, const T *k, int q) {
+  if constexpr (AX < 0) return a + b * k[q];
+  else return q == AX ? a + b * k[AX] : a;
+}
+
 // ------------------------------------------------------------------ characteristic WENO-Z
 
 // Convex WENO-Z combination sum_k a_k q_k / sum_k a_k with a_k = d_k (1 + tau / D_k) and
@@ -102,23 +119,14 @@ template <> struct WenoComb<float> {
   }
 };
 
-// Characteristic WENO5-Z interpolation of one field at i+1/2 from the 6 points i-2..i+3
-// (AWENO.cu:156-210).  Lr: the field's row of the left eigenvector matrix; q(s, v) returns
-// conservative variable v of stencil point s.  Smoothness indicators and candidate interpolants are the
+// Characteristic WENO5-Z interpolation of one field, v its values at the 6 points i-2..i+3, at i+1/2
+// (AWENO.cu:156-210).  Smoothness indicators and candidate interpolants are the
 // reference's, written with the differences of consecutive points (which the stencils and the two sides
 // share) and, the candidates, as distances from point i: fewer operations, and none of the digits of the
 // field's level is lost.  (AWENO7 + HLLC at 512 x 256 x 128, three sweeps a stage: FP64 10.1 -> 8.9 ms, FP32 at
 // 385 x 257 x 129 4.3 -> 3.7 ms.)
-template <typename T, class Q>
-__device__ __forceinline__ void weno5_char(const T *Lr, const Q &q, T &vminus, T &vplus) {
-  T v[6];
-#pragma unroll
-  for (int s = 0; s < 6; ++s) {
-    T acc = T(0);
-#pragma unroll
-    for (int j = 0; j < 5; ++j) acc += Lr[j] * q(s, j);
-    v[s] = acc;
-  }
+template <typename T>
+__device__ __forceinline__ void weno5(const T *v, T &vminus, T &vplus) {
   const T d0 = v[1] - v[0], d1 = v[2] - v[1], d2 = v[3] - v[2], d3 = v[4] - v[3], d4 = v[5] - v[4];
   const T eps = T(1e-6), o8 = T(0.125);
   // 13/12 of the squared second differences
@@ -172,18 +180,12 @@ __device__ __forceinline__ void weno7_betas(const T *d, T v2, T v3, T &b0, T &b1
 }
 
 // Characteristic WENO7-Z interpolation from the 8 points i-3..i+4 (AWENO.cu:212-280), in differences as
-// weno5_char; the candidates are distances from point i.
-template <typename T, class Q>
-__device__ __forceinline__ void weno7_char(const T *Lr, const Q &q, T &vminus, T &vplus) {
-  T v[8], d[7];
+// weno5; the candidates are distances from point i.
+template <typename T>
+__device__ __forceinline__ void weno7(const T *v, T &vminus, T &vplus) {
+  T d[7];
 #pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    T acc = T(0);
-#pragma unroll
-    for (int j = 0; j < 5; ++j) acc += Lr[j] * q(s, j);
-    v[s] = acc;
-    if (s > 0) d[s - 1] = v[s] - v[s - 1];
-  }
+  for (int s = 0; s < 7; ++s) d[s] = v[s + 1] - v[s];
   const T eps = T(1e-6), o16 = T(0.0625);
   const T qb = o16 * (T(5) * d[3] + T(4) * d[2] - d[1]), qc = o16 * (d[2] + T(8) * d[3] - d[4]),
           qd = o16 * (T(11) * d[3] - T(4) * d[4] + d[5]);
@@ -211,6 +213,27 @@ __device__ __forceinline__ void weno7_char(const T *Lr, const Q &q, T &vminus, T
   vplus += v[3];
 }
 
+template <int NG, typename T>
+__device__ __forceinline__ void weno(const T *v, T &vminus, T &vplus) {
+  if constexpr (NG == 3) weno5<T>(v, vminus, vplus);
+  else weno7<T>(v, vminus, vplus);
+}
+
+// One characteristic field: the products of the row Lr of the left eigenvector matrix with the stencil's
+// conservative variables q(s, v), interpolated.
+template <int NG, typename T, class Q>
+__device__ __forceinline__ void weno_char(const T *Lr, const Q &q, T &vminus, T &vplus) {
+  T v[2 * NG];
+#pragma unroll
+  for (int s = 0; s < 2 * NG; ++s) {
+    T acc = T(0);
+#pragma unroll
+    for (int j = 0; j < 5; ++j) acc += Lr[j] * q(s, j);
+    v[s] = acc;
+  }
+  weno<NG, T>(v, vminus, vplus);
+}
+
 // AWENO_interpolation<Air> (AWENO.cu:15-154).  NG = 3 (WENO5) or 4 (WENO7); q(s, v) for
 // s in [0, 2*NG) is point i-NG+1+s, v = 0..4 conservative variables, v = 5 pressure.
 // mt0/mt1: metric row of the sweep direction at i and i+1.  pl/pr: rho,u,v,w,p,rhoE.
@@ -218,7 +241,11 @@ __device__ __forceinline__ void weno7_char(const T *Lr, const Q &q, T &vminus, T
 // by column, so only one row/column is live at a time; the reference's divisions by cm2, cm,
 // gradK and rho are replaced by multiplications with their reciprocals.  The back projection
 // accumulates field by field in the reference's summation order.
-template <int NG, typename T, class Q>
+// AX >= 0 (axis-aligned normal k = +-e_AX): the two acoustic fields and the entropy field share one
+// product X = alpha rho - (gamma - 1)(u . m - rhoE) per point (A = X / (2 c^2), B = (u rho - m)_n / (2 c):
+// A + B, A - B and rho - 2 A), and each shear field is (m_t - u_t rho) / c: 15 operations a point instead
+// of 25 (the signs k of the shear and entropy fields cancel between their rows and columns).
+template <int NG, typename T, int AX, class Q>
 __device__ __forceinline__ void aweno_interp(const Q &q, const T *mt0, const T *mt1, T *pl, T *pr) {
   constexpr int cl = NG - 1, cr = NG;
   const T gm1 = T(kGamma - 1), igm1 = T(1.0 / (kGamma - 1));
@@ -238,6 +265,66 @@ __device__ __forceinline__ void aweno_interp(const Q &q, const T *mt0, const T *
   const T cm2 = gm1 * (hm - ekm);
   const T icm = trsqrt(cm2);
   const T cm = cm2 * icm, icm2 = icm * icm;
+  const T alpha = gm1 * ekm;
+  const T h2 = T(0.5) * icm2;
+  T ql[5] = {T(0), T(0), T(0), T(0), T(0)}, qr[5] = {T(0), T(0), T(0), T(0), T(0)};
+  if constexpr (AX >= 0) {
+    constexpr int n = 1 + AX, t1 = 1 + (AX + 1) % 3, t2 = 1 + (AX + 2) % 3;
+    const T vel[4] = {T(0), um, vm, wm};
+    const T k = mt0[AX] + mt1[AX] < T(0) ? T(-1) : T(1), kc = k * cm;
+    T a[2 * NG], bq[2 * NG], v[2 * NG];
+#pragma unroll
+    for (int s = 0; s < 2 * NG; ++s) {
+      const T r = q(s, 0), m = q(s, n);
+      T X = alpha * r + gm1 * q(s, 4);
+      X -= gm1 * (vel[n] * m + vel[t1] * q(s, t1) + vel[t2] * q(s, t2));
+      a[s] = h2 * X;
+      bq[s] = (h2 * kc) * (vel[n] * r - m);
+    }
+    T vmi, vpl;
+#pragma unroll
+    for (int l = 0; l < 5; ++l) {
+      if (l == 0 || l == 4) {
+        const T sg = l == 0 ? T(-1) : T(1);
+#pragma unroll
+        for (int s = 0; s < 2 * NG; ++s) v[s] = l == 0 ? a[s] + bq[s] : a[s] - bq[s];
+        weno<NG, T>(v, vmi, vpl);
+        const T rn = vel[n] + sg * kc, re = hm + sg * kc * vel[n];
+        ql[0] += vmi;
+        qr[0] += vpl;
+        ql[n] += rn * vmi;
+        qr[n] += rn * vpl;
+        ql[t1] += vel[t1] * vmi;
+        qr[t1] += vel[t1] * vpl;
+        ql[t2] += vel[t2] * vmi;
+        qr[t2] += vel[t2] * vpl;
+        ql[4] += re * vmi;
+        qr[4] += re * vpl;
+      } else if (l == n) {
+#pragma unroll
+        for (int s = 0; s < 2 * NG; ++s) v[s] = q(s, 0) - T(2) * a[s];
+        weno<NG, T>(v, vmi, vpl);
+        ql[0] += vmi;
+        qr[0] += vpl;
+#pragma unroll
+        for (int m = 1; m < 4; ++m) {
+          ql[m] += vel[m] * vmi;
+          qr[m] += vel[m] * vpl;
+        }
+        ql[4] += ekm * vmi;
+        qr[4] += ekm * vpl;
+      } else {
+#pragma unroll
+        for (int s = 0; s < 2 * NG; ++s) v[s] = icm * (q(s, l) - vel[l] * q(s, 0));
+        weno<NG, T>(v, vmi, vpl);
+        ql[l] += cm * vmi;
+        qr[l] += cm * vpl;
+        const T re = vel[l] * cm;
+        ql[4] += re * vmi;
+        qr[4] += re * vpl;
+      }
+    }
+  } else {
   T kx = T(0.5) * (mt0[0] + mt1[0]);
   T ky = T(0.5) * (mt0[1] + mt1[1]);
   T kz = T(0.5) * (mt0[2] + mt1[2]);
@@ -246,9 +333,6 @@ __device__ __forceinline__ void aweno_interp(const Q &q, const T *mt0, const T *
   ky *= igk;
   kz *= igk;
   const T Uk = kx * um + ky * vm + kz * wm;
-  const T alpha = gm1 * ekm;
-  const T h2 = T(0.5) * icm2;
-  T ql[5] = {T(0), T(0), T(0), T(0), T(0)}, qr[5] = {T(0), T(0), T(0), T(0), T(0)};
 #pragma unroll
   for (int l = 0; l < 5; ++l) {
     T Lr[5], Rc[5];
@@ -292,16 +376,13 @@ __device__ __forceinline__ void aweno_interp(const Q &q, const T *mt0, const T *
       Rc[0] = T(1); Rc[1] = um + kx * cm; Rc[2] = vm + ky * cm; Rc[3] = wm + kz * cm; Rc[4] = hm + Uk * cm;
     }
     T vmi, vpl;
-    if constexpr (NG == 3) {
-      weno5_char<T>(Lr, q, vmi, vpl);
-    } else {
-      weno7_char<T>(Lr, q, vmi, vpl);
-    }
+    weno_char<NG, T>(Lr, q, vmi, vpl);
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
       ql[m] += Rc[m] * vmi;
       qr[m] += Rc[m] * vpl;
     }
+  }
   }
   const T iqq = T(1) / (ql[0] * qr[0]);
   const T iql = qr[0] * iqq, iqr = ql[0] * iqq;
@@ -323,16 +404,17 @@ __device__ __forceinline__ void aweno_interp(const Q &q, const T *mt0, const T *
 
 // riemannSolver_ausmPlus<Air> (RiemannSolver.cuh:9-96); divisions by the face-normal magnitude,
 // sound speed and densities go through reciprocals.
-template <typename T>
+template <typename T, int AX = -1>
 __device__ __forceinline__ void ausm_plus(const T *pl, const T *pr, const T *mt0, const T *mt1, T j0, T j1, T *fc) {
-  const T k1 = T(0.5) * (j0 * mt0[0] + j1 * mt1[0]);
-  const T k2 = T(0.5) * (j0 * mt0[1] + j1 * mt1[1]);
-  const T k3 = T(0.5) * (j0 * mt0[2] + j1 * mt1[2]);
-  const T k2s = k1 * k1 + k2 * k2 + k3 * k3;
+  T k[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    if (AX < 0 || q == AX) k[q] = T(0.5) * (j0 * mt0[q] + j1 * mt1[q]);
+  const T k2s = kdot<AX>(k, k);
   const T igkj = trsqrt(k2s);
   const T gkj = k2s * igkj;
-  const T ul = (k1 * pl[1] + k2 * pl[2] + k3 * pl[3]) * igkj;
-  const T ur = (k1 * pr[1] + k2 * pr[2] + k3 * pr[3]) * igkj;
+  const T ul = kdot<AX>(k, pl + 1) * igkj;
+  const T ur = kdot<AX>(k, pr + 1) * igkj;
   const T p_l = pl[4], p_r = pr[4], rho_l = pl[0], rho_r = pr[0];
   const T gam = T(kGamma);
   const T irl = T(1) / rho_l, irr = T(1) / rho_r;
@@ -368,14 +450,13 @@ __device__ __forceinline__ void ausm_plus(const T *pl, const T *pr, const T *mt0
   const bool left = mass_flux >= T(0);
   const T *s = left ? pl : pr;
   fc[0] = coeff;
-  fc[1] = coeff * s[1] + p_coeff * k1;
-  fc[2] = coeff * s[2] + p_coeff * k2;
-  fc[3] = coeff * s[3] + p_coeff * k3;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) fc[1 + q] = kadd<AX>(coeff * s[1 + q], p_coeff, k, q);
   fc[4] = coeff * (s[5] + s[4]) * (left ? irl : irr);
 }
 
 // riemannSolver_hllc<Air> (RiemannSolver.cuh:98-230), with shared reciprocals.
-template <typename T>
+template <typename T, int AX = -1>
 __device__ __forceinline__ void hllc(const T *pl, const T *pr, const T *mt0, const T *mt1, T j0, T j1, T *fc) {
   const T gam = T(kGamma);
   const T rsl = trsqrt(pl[0]), rsr = trsqrt(pr[0]);
@@ -392,25 +473,26 @@ __device__ __forceinline__ void hllc(const T *pl, const T *pr, const T *mt0, con
   const T ht = hl * rl_c + hr * rr_c;
   const T ekt = T(0.5) * (ut * ut + vt * vt + wt * wt);
   const T ct = tsqrt((gam - T(1)) * (ht - ekt));
-  const T kx = T(0.5) * (mt0[0] + mt1[0]);
-  const T ky = T(0.5) * (mt0[1] + mt1[1]);
-  const T kz = T(0.5) * (mt0[2] + mt1[2]);
-  const T k2s = kx * kx + ky * ky + kz * kz;
+  T k[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    if (AX < 0 || q == AX) k[q] = T(0.5) * (mt0[q] + mt1[q]);
+  const T k2s = kdot<AX>(k, k);
   const T igk = trsqrt(k2s);
   const T gradK = k2s * igk;
-  const T Ubar = (kx * ut + ky * vt + kz * wt) * igk;
+  const T vt3[3] = {ut, vt, wt};
+  const T Ubar = kdot<AX>(k, vt3) * igk;
   const T jac = T(0.5) * (j0 + j1);
-  const T Ul = kx * pl[1] + ky * pl[2] + kz * pl[3];
-  const T Ur = kx * pr[1] + ky * pr[2] + kz * pr[3];
+  const T Ul = kdot<AX>(k, pl + 1);
+  const T Ur = kdot<AX>(k, pr + 1);
   const T unl = Ul * igk, unr = Ur * igk;
   const T cl = tsqrt(gam * pl[4] * irl);
   const T sl = tmin(unl - cl, Ubar - ct);
   if (sl >= T(0)) {
     const T rU = pl[0] * Ul;
     fc[0] = jac * rU;
-    fc[1] = jac * (rU * pl[1] + pl[4] * kx);
-    fc[2] = jac * (rU * pl[2] + pl[4] * ky);
-    fc[3] = jac * (rU * pl[3] + pl[4] * kz);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) fc[1 + q] = jac * kadd<AX>(rU * pl[1 + q], pl[4], k, q);
     fc[4] = jac * ((pl[5] + pl[4]) * Ul);
     return;
   }
@@ -419,9 +501,8 @@ __device__ __forceinline__ void hllc(const T *pl, const T *pr, const T *mt0, con
   if (sr < T(0)) {
     const T rU = pr[0] * Ur;
     fc[0] = jac * rU;
-    fc[1] = jac * (rU * pr[1] + pr[4] * kx);
-    fc[2] = jac * (rU * pr[2] + pr[4] * ky);
-    fc[3] = jac * (rU * pr[3] + pr[4] * kz);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) fc[1 + q] = jac * kadd<AX>(rU * pr[1 + q], pr[4], k, q);
     fc[4] = jac * ((pr[5] + pr[4]) * Ur);
     return;
   }
@@ -435,32 +516,33 @@ __device__ __forceinline__ void hllc(const T *pl, const T *pr, const T *mt0, con
   const T Q = jac * pc * sm * (sk * gradK - Uk) * q[0];
   fc[0] = Q;
   const T dP = (sk * pm - sm * q[4]) * pc * jac;
-  fc[1] = Q * q[1] + dP * kx;
-  fc[2] = Q * q[2] + dP * ky;
-  fc[3] = Q * q[3] + dP * kz;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) fc[1 + c] = kadd<AX>(Q * q[1 + c], dP, k, c);
   fc[4] = Q * q[5] * irk + pc * jac * (sk * pm * sm * gradK - sm * q[4] * Uk);
 }
 
 // riemannSolver_laxFriedrich<Air> (RiemannSolver.cuh:420-460): face-averaged metric, the larger
 // spectral radius of the two sides.
-template <typename T>
+template <typename T, int AX = -1>
 __device__ __forceinline__ void lax_friedrichs(const T *pl, const T *pr, const T *mt0, const T *mt1, T j0, T j1,
                                                T *fc) {
-  const T kx = T(0.5) * (mt0[0] + mt1[0]);
-  const T ky = T(0.5) * (mt0[1] + mt1[1]);
-  const T kz = T(0.5) * (mt0[2] + mt1[2]);
-  const T gradK = tsqrt(kx * kx + ky * ky + kz * kz);
-  const T Ukl = pl[1] * kx + pl[2] * ky + pl[3] * kz;
-  const T Ukr = pr[1] * kx + pr[2] * ky + pr[3] * kz;
+  T k[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    if (AX < 0 || q == AX) k[q] = T(0.5) * (mt0[q] + mt1[q]);
+  const T gradK = tsqrt(kdot<AX>(k, k));
+  const T Ukl = kdot<AX>(k, pl + 1);
+  const T Ukr = kdot<AX>(k, pr + 1);
   const T cl = tsqrt(T(kGamma) * pl[4] / pl[0]);
   const T cr = tsqrt(T(kGamma) * pr[4] / pr[0]);
   const T sr = tmax(tabs(Ukl) + cl * gradK, tabs(Ukr) + cr * gradK);
   const T hj = T(0.25) * (j0 + j1);
   const T rUl = pl[0] * Ukl, rUr = pr[0] * Ukr;
   fc[0] = (rUl + rUr - sr * (pr[0] - pl[0])) * hj;
-  fc[1] = (rUl * pl[1] + rUr * pr[1] + kx * (pl[4] + pr[4]) - sr * (pr[1] * pr[0] - pl[1] * pl[0])) * hj;
-  fc[2] = (rUl * pl[2] + rUr * pr[2] + ky * (pl[4] + pr[4]) - sr * (pr[2] * pr[0] - pl[2] * pl[0])) * hj;
-  fc[3] = (rUl * pl[3] + rUr * pr[3] + kz * (pl[4] + pr[4]) - sr * (pr[3] * pr[0] - pl[3] * pl[0])) * hj;
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    fc[1 + q] = (kadd<AX>(rUl * pl[1 + q] + rUr * pr[1 + q], pl[4] + pr[4], k, q) -
+                 sr * (pr[1 + q] * pr[0] - pl[1 + q] * pl[0])) * hj;
   fc[4] = ((pl[5] + pl[4]) * Ukl + (pr[5] + pr[4]) * Ukr - sr * (pr[5] - pl[5])) * hj;
 }
 
@@ -599,29 +681,28 @@ __device__ __forceinline__ void pv_reconstruct(const V &v, int recon, T *pl, T *
 }
 
 // Whole AWENO face flux: interpolation then the selected Riemann solver (InviscidScheme.cu:333-345).
-template <int NG, int RS, typename T, class Q>
+template <int NG, int RS, typename T, int AX = -1, class Q>
 __device__ __forceinline__ void aweno_face_flux(const Q &q, const T *mt0, const T *mt1, T j0, T j1, T *fc) {
   T pl[6], pr[6];
-  aweno_interp<NG, T>(q, mt0, mt1, pl, pr);
+  aweno_interp<NG, T, AX>(q, mt0, mt1, pl, pr);
   if constexpr (RS == 4) {
-    hllc<T>(pl, pr, mt0, mt1, j0, j1, fc);
+    hllc<T, AX>(pl, pr, mt0, mt1, j0, j1, fc);
   } else if constexpr (RS == 1) {
-    lax_friedrichs<T>(pl, pr, mt0, mt1, j0, j1, fc);
+    lax_friedrichs<T, AX>(pl, pr, mt0, mt1, j0, j1, fc);
   } else {
-    ausm_plus<T>(pl, pr, mt0, mt1, j0, j1, fc);
+    ausm_plus<T, AX>(pl, pr, mt0, mt1, j0, j1, fc);
   }
 }
 
 // Physical flux of one node for the central-difference correction (AWENO.cu:307-321).
 // b: rho,u,v,w,p (bv 0..4); e: rho*E (cv 4); k: metric row of the sweep direction.
-template <typename T>
+template <typename T, int AX = -1>
 __device__ __forceinline__ void node_flux(const T *b, T e, const T *k, T jac, T *f) {
-  const T Uk = k[0] * b[1] + k[1] * b[2] + k[2] * b[3];
+  const T Uk = kdot<AX>(k, b + 1);
   const T rhoUk = b[0] * Uk;
   f[0] = rhoUk * jac;
-  f[1] = jac * (rhoUk * b[1] + k[0] * b[4]);
-  f[2] = jac * (rhoUk * b[2] + k[1] * b[4]);
-  f[3] = jac * (rhoUk * b[3] + k[2] * b[4]);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) f[1 + q] = jac * kadd<AX>(rhoUk * b[1 + q], b[4], k, q);
   f[4] = jac * Uk * (e + b[4]);
 }
 

@@ -108,7 +108,7 @@ int ostc_set_sweep_variant(ostc_ctx *ctx, int precision, int dir, int variant) {
     std::lock_guard<std::mutex> lk(g_tune_mutex);
     for (auto &B : ctx->blk) {
       const TuneKey key{ctx->device, B.db.mx, B.db.my, B.db.mz, B.db.g, ctx->der.riemann, ctx->der.inviscid_type,
-                        precision, dir};
+                        B.db.rect, precision, dir};
       g_tune_cache.erase(key);
     }
   }

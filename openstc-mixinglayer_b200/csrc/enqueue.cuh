@@ -267,9 +267,9 @@ void launch_adjoint_t(ostc_ctx *ctx, BlockRes &B, DevState in, unsigned mask, co
 }
 
 // y / z sweep variants: tiles of the shapes below, {lanes, threads along the sweep, faces per thread}.  Rows of
-// 64 bytes and 32 faces (variant 0) re-read the fewest halo nodes: 512 x 256 x 128, FP64, 2.48 ms against 2.51
-// of the next, 385 x 257 x 129, FP32, 1.13 against 1.19, 257 x 129, FP64, 11.1 us against 12.6; the others (rows
-// of 128 bytes) fit other extents with less of a tile left empty: 193 x 101 x 75, FP64, 178 us against 177.
+// 64 bytes and 32 faces (variant 0) re-read the fewest halo nodes and lead on large blocks; rows of 128 bytes
+// and 16 faces waste less on columns shorter than a long tile: 257 x 129, FP64, 11.1 / 13.3 us (0 / 1) in the
+// general kernels, 10.6 / 9.2 in the rectilinear ones; 193 x 101 x 75, FP64, 178 / 177 us (0 / 2).
 template <typename T> struct YzShapes;
 template <> struct YzShapes<float> {
   static constexpr int X0 = 16, D0 = 16, F0 = 2, X1 = 32, D1 = 16, F1 = 1, X2 = 32, D2 = 8, F2 = 2, X3 = 32, D3 = 4, F3 = 4;
@@ -288,8 +288,12 @@ void launch_yz_v(ostc_ctx *ctx, BlockRes &B, DevState in, int variant) {
   {                                                                                                   \
     constexpr int TF = DD * F;                                                                        \
     dim3 grid((b.mx + X - 1) / X, (n_dir + TF - 2) / (TF - 1), n_o);                                   \
-    k_flux_tile<D, N, R, T, X, DD, F>                                                                 \
-        <<<grid, dim3(X, DD), tile_smem_bytes<N, X, TF, T>(), ctx->stream>>>(b, in, B.dq);             \
+    if (b.rect)                                                                                       \
+      k_flux_tile<D, N, R, T, X, DD, F, true>                                                         \
+          <<<grid, dim3(X, DD), tile_smem_bytes<N, X, TF, T, true>(), ctx->stream>>>(b, in, B.dq);     \
+    else                                                                                              \
+      k_flux_tile<D, N, R, T, X, DD, F, false>                                                        \
+          <<<grid, dim3(X, DD), tile_smem_bytes<N, X, TF, T, false>(), ctx->stream>>>(b, in, B.dq);    \
   }
   if (variant == 1) OSTC_TILE(S::X1, S::D1, S::F1)
   else if (variant == 2) OSTC_TILE(S::X2, S::D2, S::F2)
@@ -307,7 +311,9 @@ template <typename T, int N, int R>
 void launch_x_v(ostc_ctx *ctx, BlockRes &B, DevState in, int variant) {
   (void)variant;
   const DevBlock &b = B.db;
-  k_flux_x<N, R, T><<<dim3((b.mx + 126) / 127, b.my, b.mz), 128, 0, ctx->stream>>>(b, in, B.dq);
+  const dim3 grid((b.mx + 126) / 127, b.my, b.mz);
+  if (b.rect) k_flux_x<N, R, T, true><<<grid, 128, 0, ctx->stream>>>(b, in, B.dq);
+  else k_flux_x<N, R, T, false><<<grid, 128, 0, ctx->stream>>>(b, in, B.dq);
 }
 
 template <typename T>
@@ -344,7 +350,7 @@ void launch_yz(ostc_ctx *ctx, BlockRes &B, DevState in, int variant) {
 // outside any stream capture, before the step graph is built.  Results are cached in the process by
 // (device, block extents, ngg, scheme, precision, direction), so further contexts of the same shape
 // (other blocks of the same extents, a second solver on the same case) reuse them.
-using TuneKey = std::tuple<int, int, int, int, int, int, int, int, int>;
+using TuneKey = std::tuple<int, int, int, int, int, int, int, int, int, int>;
 std::map<TuneKey, int> g_tune_cache;
 std::mutex g_tune_mutex;
 
@@ -357,7 +363,8 @@ int autotune_yz(ostc_ctx *ctx) {
   for (auto &B : ctx->blk) {
     const DevState in = state_of(B, 0);
     for (int dir = 0; dir <= (B.db.mz > 1 ? 2 : 1); ++dir) {
-      const TuneKey key{ctx->device, B.db.mx, B.db.my, B.db.mz, B.db.g, ctx->der.riemann, ctx->der.inviscid_type, pi, dir};
+      const TuneKey key{ctx->device, B.db.mx, B.db.my, B.db.mz, B.db.g, ctx->der.riemann, ctx->der.inviscid_type,
+                        B.db.rect, pi, dir};
       int &slot = dir == 0 ? B.x_var[pi] : B.yz_var[pi][dir - 1];
       if (ctx->forced[pi][dir] >= 0) {
         slot = ctx->forced[pi][dir];
@@ -440,25 +447,29 @@ int launch_flux(ostc_ctx *ctx, BlockRes &B, DevState in) {
   return OSTC_OK;
 }
 
-template <typename T>
-void launch_visc(ostc_ctx *ctx, BlockRes &B, const StageArgs &a) {
+template <typename T, bool RECT>
+void launch_visc_t(ostc_ctx *ctx, BlockRes &B, const StageArgs &a) {
   const DevBlock &b = B.db;
-  long tok = begin_t(ctx, "visc_update");
+  constexpr int TX = 32, TY = 4;
   if (b.mz > 1) {
-    constexpr int TX = 32, TY = 4;
     const long long cols = (long long)((b.mx + TX - 1) / TX) * ((b.my + TY - 1) / TY);
     int nseg = (int)std::max<long long>(1, (ctx->sm_count * 8 + cols - 1) / cols);
     int kseg = std::max(4, (b.mz + nseg - 1) / nseg);
     nseg = (b.mz + kseg - 1) / kseg;
     dim3 grid((b.mx + TX - 1) / TX, (b.my + TY - 1) / TY, nseg);
-    k_visc_update<T, true, TX, TY>
-        <<<grid, dim3(TX, TY, 1), visc_smem_bytes<T, true, TX, TY>(), ctx->stream>>>(b, a, B.dq, kseg);
+    k_visc_update<T, true, TX, TY, RECT>
+        <<<grid, dim3(TX, TY, 1), visc_smem_bytes<T, true, TX, TY, RECT>(), ctx->stream>>>(b, a, B.dq, kseg);
   } else {
-    constexpr int TX = 32, TY = 4;
     dim3 grid((b.mx + TX - 1) / TX, (b.my + TY - 1) / TY, 1);
-    k_visc_update<T, false, TX, TY>
-        <<<grid, dim3(TX, TY, 1), visc_smem_bytes<T, false, TX, TY>(), ctx->stream>>>(b, a, B.dq, 1);
+    k_visc_update<T, false, TX, TY, RECT>
+        <<<grid, dim3(TX, TY, 1), visc_smem_bytes<T, false, TX, TY, RECT>(), ctx->stream>>>(b, a, B.dq, 1);
   }
+}
+template <typename T>
+void launch_visc(ostc_ctx *ctx, BlockRes &B, const StageArgs &a) {
+  long tok = begin_t(ctx, "visc_update");
+  if (B.db.rect) launch_visc_t<T, true>(ctx, B, a);
+  else launch_visc_t<T, false>(ctx, B, a);
   end_t(ctx, tok);
 }
 
@@ -603,18 +614,25 @@ bool set_sweep_attrs() {
     ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
   };
   using S = YzShapes<T>;
-#define OSTC_TSET(D, N, R)                                                                                      \
-  tset((const void *)k_flux_tile<D, N, R, T, S::X0, S::D0, S::F0>, tile_smem_bytes<N, S::X0, S::D0 * S::F0, T>()); \
-  tset((const void *)k_flux_tile<D, N, R, T, S::X1, S::D1, S::F1>, tile_smem_bytes<N, S::X1, S::D1 * S::F1, T>()); \
-  tset((const void *)k_flux_tile<D, N, R, T, S::X2, S::D2, S::F2>, tile_smem_bytes<N, S::X2, S::D2 * S::F2, T>()); \
-  tset((const void *)k_flux_tile<D, N, R, T, S::X3, S::D3, S::F3>, tile_smem_bytes<N, S::X3, S::D3 * S::F3, T>());
+#define OSTC_TSET1(D, N, R, X, DD, F, RECT) \
+  tset((const void *)k_flux_tile<D, N, R, T, X, DD, F, RECT>, tile_smem_bytes<N, X, DD * F, T, RECT>());
+#define OSTC_TSET(D, N, R)                         \
+  OSTC_TSET1(D, N, R, S::X0, S::D0, S::F0, false)  \
+  OSTC_TSET1(D, N, R, S::X0, S::D0, S::F0, true)   \
+  OSTC_TSET1(D, N, R, S::X1, S::D1, S::F1, false)  \
+  OSTC_TSET1(D, N, R, S::X2, S::D2, S::F2, false)  \
+  OSTC_TSET1(D, N, R, S::X3, S::D3, S::F3, false)  \
+  OSTC_TSET1(D, N, R, S::X1, S::D1, S::F1, true)   \
+  OSTC_TSET1(D, N, R, S::X2, S::D2, S::F2, true)   \
+  OSTC_TSET1(D, N, R, S::X3, S::D3, S::F3, true)
   OSTC_TSET(1, 3, 1) OSTC_TSET(1, 3, 3) OSTC_TSET(1, 3, 4) OSTC_TSET(1, 4, 1) OSTC_TSET(1, 4, 3) OSTC_TSET(1, 4, 4)
   OSTC_TSET(2, 3, 1) OSTC_TSET(2, 3, 3) OSTC_TSET(2, 3, 4) OSTC_TSET(2, 4, 1) OSTC_TSET(2, 4, 3) OSTC_TSET(2, 4, 4)
 #undef OSTC_TSET
-  ok = ok && cudaFuncSetAttribute((const void *)k_visc_update<T, true, 32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)visc_smem_bytes<T, true, 32, 4>()) == cudaSuccess;
-  ok = ok && cudaFuncSetAttribute((const void *)k_visc_update<T, false, 32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)visc_smem_bytes<T, false, 32, 4>()) == cudaSuccess;
+#undef OSTC_TSET1
+  tset((const void *)k_visc_update<T, true, 32, 4, false>, visc_smem_bytes<T, true, 32, 4, false>());
+  tset((const void *)k_visc_update<T, false, 32, 4, false>, visc_smem_bytes<T, false, 32, 4, false>());
+  tset((const void *)k_visc_update<T, true, 32, 4, true>, visc_smem_bytes<T, true, 32, 4, true>());
+  tset((const void *)k_visc_update<T, false, 32, 4, true>, visc_smem_bytes<T, false, 32, 4, true>());
   return ok;
 }
 

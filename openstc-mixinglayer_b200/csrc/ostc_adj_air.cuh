@@ -464,7 +464,7 @@ __device__ __forceinline__ void weno_char_bwd(const double *v, double fm, double
       d[i] = v[i + 1] - v[i];
       gd[i] = 0;
     }
-    // candidates as distances from v[3] (weno7_char)
+    // candidates as distances from v[3] (weno7)
     const double o16 = 0.0625;
     const double qa = o16 * (19 * d[2] - 16 * d[1] + 5 * d[0]), qb = o16 * (5 * d[3] + 4 * d[2] - d[1]);
     const double qc = o16 * (d[2] + 8 * d[3] - d[4]), qd = o16 * (11 * d[3] - 4 * d[4] + d[5]);
@@ -637,8 +637,7 @@ __global__ void __launch_bounds__(128, 2) k_adj_air_face(DevBlock b, DevState s,
       double L[5], R[5], vm, vp;
       air_eigen(f, l, L, R);
       auto qq = [&](int sn, int v) -> double { return q(sn, v); };
-      if constexpr (NG == 3) weno5_char<double>(L, qq, vm, vp);
-      else weno7_char<double>(L, qq, vm, vp);
+      weno_char<NG, double>(L, qq, vm, vp);
 #pragma unroll
       for (int m = 0; m < 5; ++m) {
         ql[m] += R[m] * vm;
