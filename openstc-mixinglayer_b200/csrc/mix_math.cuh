@@ -557,41 +557,31 @@ __device__ __forceinline__ T fvs_beta7(T s1, T s2, T s3) {
   return s1 * (s1 + T(1.0 / 12) * s3) + T(13.0 / 12.0) * s2 * s2 + T(1043.0 / 960) * s3 * s3;
 }
 
-// (eps + beta)^2 of the Z weights; in FP32 floored at 1e-30 so that a smooth stencil (beta = 0,
-// where the scaled eps underflows) gives the linear weights instead of 0/0
-template <typename T>
-__device__ __forceinline__ T fvs_den(T eps, T beta) {
-  const T d = (eps + beta) * (eps + beta);
-  if constexpr (sizeof(T) == 4) return fmaxf(d, 1e-30f);
-  return d;
-}
-
-// tau / D_k of the four Z weights, D_k = (eps + beta_k)^2.  FP64: one division where the product of the
-// four D_k is representable, else one per pair (D_k >= eps^2 keeps the pair products in range for any
-// practical eps), else four.  FP32 (its scaled D_k may be as small as 1e-30): four fast divisions.
-__device__ __forceinline__ void fvs_ratios(double tau, const double *d, double *r) {
-  const double p01 = d[0] * d[1], p23 = d[2] * d[3], p = p01 * p23;
-  double r01, r23;
-  if (p > 1e-290) {
-    const double q = 1.0 / p;
-    r01 = tau * (p23 * q);
-    r23 = tau * (p01 * q);
-  } else if (p01 > 0.0 && p23 > 0.0) {
-    r01 = tau / p01;
-    r23 = tau / p23;
+// tau / D_k of the four Z weights, D_k = (eps + beta_k)^2.  FP64: the four 1 / (eps + beta_k) from one
+// division where the product of the four stays in range (an eps above 1e-75), else each
+// takes its own.  FP32: four fast divisions, D_k floored at 1e-30 so that a smooth stencil (beta = 0, where
+// the scaled eps underflows) gives the linear weights instead of 0/0.
+__device__ __forceinline__ void fvs_ratios(double tau, double eps, const double *b, double *r) {
+  const double g0 = eps + b[0], g1 = eps + b[1], g2 = eps + b[2], g3 = eps + b[3];
+  const double p01 = g0 * g1, p23 = g2 * g3, p = p01 * p23;
+  if (p > 1e-300 && p < 1e300) {
+    const double q = 1.0 / p, q01 = p23 * q, q23 = p01 * q;
+    r[0] = g1 * q01;
+    r[1] = g0 * q01;
+    r[2] = g3 * q23;
+    r[3] = g2 * q23;
   } else {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) r[k] = tau / d[k];
-    return;
+    r[0] = 1.0 / g0;
+    r[1] = 1.0 / g1;
+    r[2] = 1.0 / g2;
+    r[3] = 1.0 / g3;
   }
-  r[0] = d[1] * r01;
-  r[1] = d[0] * r01;
-  r[2] = d[3] * r23;
-  r[3] = d[2] * r23;
-}
-__device__ __forceinline__ void fvs_ratios(float tau, const float *d, float *r) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) r[k] = __fdividef(tau, d[k]);
+  for (int k = 0; k < 4; ++k) r[k] = tau * (r[k] * r[k]);
+}
+__device__ __forceinline__ void fvs_ratios(float tau, float eps, const float *b, float *r) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) r[k] = __fdividef(tau, fmaxf((eps + b[k]) * (eps + b[k]), 1e-30f));
 }
 
 // One side of the flux-split WENO7-Z (WENO.cu:1619-1693), its points v0..v6 upwind first: the face value
@@ -612,13 +602,10 @@ __device__ __forceinline__ void fvs_side(T v0, T v1, T v2, T v3, T v4, T v5, T v
   const T s2[4] = {e1 + t0, e2, e2, e3 - t3};
   const T s3[4] = {t0, t1, t2, t3};
   const T c[4] = {T(1.0 / 35), T(12.0 / 35), T(18.0 / 35), T(4.0 / 35)};
-  T b[4], d[4], r[4];
+  T b[4], r[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    b[k] = fvs_beta7(s1[k], s2[k], s3[k]);
-    d[k] = fvs_den(eps, b[k]);
-  }
-  fvs_ratios((b[0] - b[3]) * (b[0] - b[3]), d, r);
+  for (int k = 0; k < 4; ++k) b[k] = fvs_beta7(s1[k], s2[k], s3[k]);
+  fvs_ratios((b[0] - b[3]) * (b[0] - b[3]), eps, b, r);
   num = T(0);
   den = T(0);
 #pragma unroll

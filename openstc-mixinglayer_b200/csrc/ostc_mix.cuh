@@ -34,10 +34,10 @@ __device__ __forceinline__ void mix_cv_from_bv_node(const DevBlock &b, const Dev
 
 // update_physical_properties<mixture> over every padded node (FieldOperation.cuh:107-134), with the
 // node's state read in FP64 and the properties evaluated in T (FP32 in the mixed precision mode).
-// FP32 at four resident blocks (128 registers) measured 1.4 ms per step faster than uncapped; FP64
-// is fastest uncapped.
+// Bound by latency: FP64 uncapped took 255 registers, two blocks an SM; five (spilling) 0.19 ms against 0.31 at
+// 192 x 96 x 48 (four 0.19, three 0.25), 60 against 97 us at 97 x 65 x 33.  FP32 four blocks.
 template <int NS, typename T>
-__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 1 : 4) k_mix_props(DevBlock b, DevState s) {
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 5 : 4) k_mix_props(DevBlock b, DevState s) {
   const long long P = b.plane;
   const int ns = OSTC_NS;
   for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
@@ -151,10 +151,12 @@ template <int DIR> struct FvsTile {
   static constexpr int NST = TD + 7;  // staged nodes: stencils of 8 nodes around TD faces
 };
 
-// split fluxes of the staged nodes [2][nv][NST][TXL], then the face fluxes [nv][TD][TXL]
+// split fluxes of the staged nodes [2][nv][NST][TXL], then per thread the species' slots [ns][TD][TXL] and
+// the mass fractions', later the flow fluxes [max(ns, 5)][TD][TXL]
+__host__ __device__ constexpr int fvs_slots(int ns) { return ns + (ns > 5 ? ns : 5); }
 template <int DIR, typename T>
 __host__ __device__ constexpr size_t fvs_smem_bytes(int nv) {
-  return (size_t)(2 * FvsTile<DIR>::NST + FvsTile<DIR>::TD) * FvsTile<DIR>::TXL * nv * sizeof(T);
+  return (size_t)(2 * FvsTile<DIR>::NST * nv + FvsTile<DIR>::TD * fvs_slots(nv - 5)) * FvsTile<DIR>::TXL * sizeof(T);
 }
 
 // compute_convective_term_weno_x/_y/_z (WENO.cu:8-461) for inviscid_scheme 72 (characteristic,
@@ -166,12 +168,15 @@ __host__ __device__ constexpr size_t fvs_smem_bytes(int nv) {
 // Bound by FP64 arithmetic at the occupancy its shared memory and registers leave (40 % of the FP64 pipe;
 // DRAM 8 %).  The staged values are laid out variable by variable, so that a warp's threads read
 // consecutive words; with the variables of a node side by side (a stride of 14 doubles) every read was a
-// two-way bank conflict.  Species arrays live in the thread's face-flux slots and the staged values are read
+// two-way bank conflict.  Species arrays live in the thread's slots and the staged values are read
 // again per row: spills 2.8 KB -> 0.3 KB a thread.  192 x 96 x 48, FP64: 0.86 / 0.79 / 0.85 -> 0.60 / 0.58 /
 // 0.64 ms (x / y / z); 257 x 129 x 65, FP32: 1.32 / 1.19 / 1.27 -> 0.85 / 0.78 / 0.85 ms.  Resident blocks
 // per SM: FP64 4 (three sweeps 1.82 ms; 3: 1.92), FP32 6 (2.48 ms; 8: 2.54).  dq takes the differences by an
 // atomicAdd whose result nobody reads (a reduction at L2; one thread adds to an entry), so that the block ends
-// without waiting for a load of dq: 1.80 -> 1.62 ms (FP64), 2.50 -> 2.24 ms (FP32).
+// without waiting for a load of dq: 1.80 -> 1.62 ms (FP64), 2.50 -> 2.24 ms (FP32).  The averaged mass fractions
+// keep slots of their own, formed once, not once in each of two loops, and the four
+// weights take one division: 1.62 -> 1.43 ms (FP64), 2.24 -> 2.17 ms (FP32).  Tiles of 4 lanes and 32 faces
+// (8 and 16 here): 1.52 and 2.29 ms.
 template <int DIR, int NS, typename T>
 __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T) == 8 ? 4 : 6) k_fvs(DevBlock b, DevState s,
                                                                                double *__restrict__ dq, int nv,
@@ -233,7 +238,8 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
   const bool face_ok = lane_ok && n < nd;
   auto FP = [&](int m, int l) -> T { return Fp[(l * NST + t + m) * TXL + lane]; };
   auto FM = [&](int m, int l) -> T { return Fm[(l * NST + t + m + 1) * TXL + lane]; };  // node m of the - side
-  auto FC = [&](int tt, int l) -> T & { return fcs[(l * TD + tt) * TXL + lane]; };
+  auto SP = [&](int tt, int l) -> T & { return fcs[(l * TD + tt) * TXL + lane]; };         // species l
+  auto FL = [&](int tt, int l) -> T & { return fcs[((ns + l) * TD + tt) * TXL + lane]; };  // mass fractions, flow fluxes
   if (face_ok && scheme == 71) {
     const long long pl = pid(n), pr = pid(n + 1);
     const double j1 = b.jac[pl], j2 = b.jac[pr];
@@ -251,11 +257,11 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
         vp[m] = FP(m, l);
         vm[m] = FM(m, l);
       }
-      FC(t, l) = fvs_weno7(vp, vm, e);
+      (l < 5 ? FL(t, l) : SP(t, l - 5)) = fvs_weno7(vp, vm, e);
     }
   } else if (face_ok) {
-    // Roe-averaged mixture eigensystem at the face (WENO.cu:747-821).  The species' alpha_l of L wait in
-    // this thread's own face-flux slots until the species loop replaces them.
+    // Roe-averaged mixture eigensystem at the face (WENO.cu:747-821).  The averaged mass fractions and the
+    // species' alpha_l of L wait in this thread's own slots until the fluxes replace them.
     const long long pl = pid(n), pr = pid(n + 1);
     const T rl = (T)s.cv[pl], rr = (T)s.cv[pr];
     const T p_l = (T)s.bv[4 * P + pl], p_r = (T)s.bv[4 * P + pr];
@@ -275,7 +281,7 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
       for (int l = 0; l < ns; ++l) {
         const T sv = roe(5 + l);
         mw_inv += sv * (T)c_mix.imw[l];
-        FC(t, 5 + l) = sv;
+        FL(t, l) = sv;
       }
       const T tm = (wl * p_l + wr * p_r) / (T(kRuD) * mw_inv);
       T cp = 0, cvt = 0;
@@ -283,10 +289,10 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
       for (int l = 0; l < ns; ++l) {
         T h, c;
         mix_h_cp_one<T>(l, tm, h, c);
-        const T sv = FC(t, 5 + l);
+        const T sv = FL(t, l);
         cp += sv * c;
         cvt += sv * (c - (T)c_mix.ru_mw[l]);
-        FC(t, 5 + l) = h;
+        SP(t, l) = h;
       }
       const T gamma = cp / cvt;
       const T c2 = gamma * T(kRuD) * mw_inv * tm;
@@ -299,8 +305,8 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
       for (int m = 0; m < 7; ++m) sp[m] = sm[m] = T(0);
 #pragma unroll 1
       for (int l = 0; l < ns; ++l) {
-        const T al = (gamma * (T)c_mix.ru_mw[l] * tm - gm1 * FC(t, 5 + l)) * c2i;
-        FC(t, 5 + l) = al;
+        const T al = (gamma * (T)c_mix.ru_mw[l] * tm - gm1 * SP(t, l)) * c2i;
+        SP(t, l) = al;
 #pragma unroll
         for (int m = 0; m < 7; ++m) {
           sp[m] += al * FP(m, 5 + l);
@@ -397,7 +403,7 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
     T add = 0;
 #pragma unroll 1
     for (int l = 0; l < ns; ++l) {
-      const T sv = roe(5 + l);
+      const T sv = FL(t, l);
       T vp[7], vmn[7];
 #pragma unroll
       for (int m = 0; m < 7; ++m) {
@@ -405,18 +411,19 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
         vmn[m] = FM(m, 5 + l) - sv * m0[m];
       }
       const T fch = fvs_weno7(vp, vmn, eps);
-      add += FC(t, 5 + l) * fch;
-      FC(t, 5 + l) = sv * fc[0] + fch;
+      add += SP(t, l) * fch;
+      SP(t, l) = sv * fc[0] + fch;
     }
     fc[4] -= add * cm * cm / gm1;
 #pragma unroll
-    for (int l = 0; l < 5; ++l) FC(t, l) = fc[l];
+    for (int l = 0; l < 5; ++l) FL(t, l) = fc[l];
   }
   __syncthreads();
   if (face_ok && t >= 1) {
     const long long q = DIR == 0 ? b.iq(n, j0, k0) : DIR == 1 ? b.iq(i0, n, k0) : b.iq(i0, j0, n);
 #pragma unroll
-    for (int l = 0; l < nv; ++l) atomicAdd(dq + l * b.n + q, (double)(FC(t - 1, l) - FC(t, l)));
+    for (int l = 0; l < nv; ++l)
+      atomicAdd(dq + l * b.n + q, (double)(l < 5 ? FL(t - 1, l) - FL(t, l) : SP(t - 1, l - 5) - SP(t, l - 5)));
   }
 }
 
@@ -468,8 +475,8 @@ __device__ __forceinline__ void mix_visc_face(const DevBlock &b, const DevState 
   T wn[3];
   for (int c = 0; c < 3; ++c) wn[c] = nx * m[c * 3] + ny * m[c * 3 + 1] + nz * m[c * 3 + 2];
   const bool cross = wn[(d + 1) % 3] != T(0) || wn[(d + 2) % 3] != T(0);
-  auto normal = [&](const double *B) -> T {
-    if (!cross) return wn[d] * (T)(B[p1] - B[p0]);
+  auto along = [&](const double *B) -> T { return wn[d] * (T)(B[p1] - B[p0]); };
+  auto mixed = [&](const double *B) -> T {
     T g[3];
     diff(B, g);
     return wn[0] * g[0] + wn[1] * g[1] + wn[2] * g[2];
@@ -494,21 +501,27 @@ __device__ __forceinline__ void mix_visc_face(const DevBlock &b, const DevState 
   const T vm = (T)(0.5 * (s.bv[2 * P + p0] + s.bv[2 * P + p1]));
   const T wm = (T)(0.5 * (s.bv[3 * P + p0] + s.bv[3 * P + p1]));
   const T cond = (T)(0.5 * (s.cond[p0] + s.cond[p1]));
-  fv[4] = um * fv[1] + vm * fv[2] + wm * fv[3] + cond * normal(s.bv + 5 * P);
+  fv[4] = um * fv[1] + vm * fv[2] + wm * fv[3] + cond * (cross ? mixed(s.bv + 5 * P) : along(s.bv + 5 * P));
   const int ns = OSTC_NS;
   T dif[Spec<NS>::A], yk[Spec<NS>::A], ddf[Spec<NS>::A];
   T sgw = 0, srdy = 0, corr = 0, mwt = 0;
-  for (int l = 0; l < ns; ++l) {
-    const double *Y = s.sv + (long long)l * P;
-    yk[l] = (T)(0.5 * (Y[p0] + Y[p1]));
-    dif[l] = (T)(0.5 * (s.rhod[l * P + p0] + s.rhod[l * P + p1]));
-    const T gdy = normal(Y);
-    ddf[l] = gdy;
-    corr += dif[l] * gdy;
-    sgw += gdy * (T)c_mix.imw[l];
-    mwt += yk[l] * (T)c_mix.imw[l];
-    srdy += dif[l] * yk[l];
-  }
+  // one branch around the whole loop, so that the loads of all species can be in flight together
+  auto species = [&](auto normal) {
+#pragma unroll
+    for (int l = 0; l < ns; ++l) {
+      const double *Y = s.sv + (long long)l * P;
+      yk[l] = (T)(0.5 * (Y[p0] + Y[p1]));
+      dif[l] = (T)(0.5 * (s.rhod[l * P + p0] + s.rhod[l * P + p1]));
+      const T gdy = normal(Y);
+      ddf[l] = gdy;
+      corr += dif[l] * gdy;
+      sgw += gdy * (T)c_mix.imw[l];
+      mwt += yk[l] * (T)c_mix.imw[l];
+      srdy += dif[l] * yk[l];
+    }
+  };
+  if (cross) species(mixed);
+  else species(along);
   mwt = T(1) / mwt;
   corr -= mwt * srdy * sgw;
   T h[Spec<NS>::A];
@@ -524,8 +537,8 @@ __device__ __forceinline__ void mix_visc_face(const DevBlock &b, const DevState 
 // then dq += fv(i+1/2) - fv(i-1/2) through shared memory; tiles as the flux-split sweeps.
 // Bound by the latency of its loads at the registers' occupancy.  dq takes the difference by an atomicAdd whose
 // result nobody reads (a reduction at L2; one thread an entry), with no load of dq to wait for, and the faces
-// are laid out variable by variable, free of bank conflicts: three sweeps of 192 x 96 x 48, FP64, 0.69 -> 0.40 ms, of
-// 257 x 129 x 65, FP32, 1.63 -> 1.03 ms.
+// are laid out variable by variable, free of bank conflicts; the species' loads go out together (mix_visc_face): three sweeps of 192 x 96 x 48, FP64, 0.69 -> 0.33 ms, of
+// 257 x 129 x 65, FP32, 1.63 -> 0.79 ms.
 template <int DIR, bool DIM3, int NS, typename T>
 __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T) == 8 ? 4 : 5) k_mix_visc(DevBlock b, DevState s,
                                                                                     double *__restrict__ dq, int nv) {
