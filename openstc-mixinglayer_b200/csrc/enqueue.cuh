@@ -58,14 +58,16 @@ void launch_flux_pv_rs(ostc_ctx *ctx, BlockRes &B, DevState in) {
   }
   for (int dir = 1; dir <= (is3d ? 2 : 1); ++dir) {
     const int n_dir = dir == 1 ? b.my : b.mz, n_o = dir == 1 ? b.mz : b.my;
-    const long long cols = (long long)((b.mx + 127) / 128) * n_o;
-    int nseg = (int)std::max<long long>(1, (ctx->sm_count * 16 + cols - 1) / cols);
-    int seg = std::max(8, (n_dir + nseg - 1) / nseg);
-    nseg = (n_dir + seg - 1) / seg;
-    dim3 grid((b.mx + 127) / 128, n_o, nseg);
+    const dim3 grid((b.mx + 15) / 16, (n_dir + 14) / 15, n_o), blk(16, 16);
     long tok = begin_t(ctx, dir == 1 ? "flux_y" : "flux_z");
-    if (dir == 1) k_flux_pv_march<1, RS, T><<<grid, 128, 0, ctx->stream>>>(b, in, a, B.dq, seg);
-    else k_flux_pv_march<2, RS, T><<<grid, 128, 0, ctx->stream>>>(b, in, a, B.dq, seg);
+    // Roe's two physical fluxes and its entropy fix read the whole metric
+    if (RS != 2 && b.rect) {
+      if (dir == 1) k_flux_pv_tile<1, RS, T, RS != 2><<<grid, blk, 0, ctx->stream>>>(b, in, a, B.dq);
+      else k_flux_pv_tile<2, RS, T, RS != 2><<<grid, blk, 0, ctx->stream>>>(b, in, a, B.dq);
+    } else {
+      if (dir == 1) k_flux_pv_tile<1, RS, T, false><<<grid, blk, 0, ctx->stream>>>(b, in, a, B.dq);
+      else k_flux_pv_tile<2, RS, T, false><<<grid, blk, 0, ctx->stream>>>(b, in, a, B.dq);
+    }
     end_t(ctx, tok);
   }
 }
