@@ -18,13 +18,17 @@ namespace ostc {
 
 // ------------------------------------------------------------------------------ time step
 
-__global__ void k_dt_reset(unsigned long long *dtbits) { *dtbits = (unsigned long long)__double_as_longlong(1e6); }
-
 // local_time_step<Air, Laminar> (TimeAdvanceFunc.cuh:28-83) fused with the global minimum of
 // global_time_step (TimeAdvanceFunc.cu:39-64).  Positive doubles order like their bit patterns, so
-// the minimum is one 64-bit atomicMin per block after a warp-shuffle reduction.
+// the minimum is one 64-bit atomicMin per block after a warp-shuffle reduction.  The last of `total` blocks
+// (of every mesh block's launch) to arrive writes dt and leaves the minimum and the count ready for the next
+// step, which would otherwise take two more launches (257 x 129: 16 -> 11 us a step).
+struct DtScratch {
+  unsigned long long bits;
+  unsigned arrived;
+};
 __global__ void __launch_bounds__(256) k_cfl_dt(DevBlock b, DevState s, double cfl, double prandtl, int dim3,
-                                                unsigned long long *dtbits) {
+                                                DtScratch *w, unsigned total, double *dt) {
   double local = 1e6;
   const long long P = b.plane;
   for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < b.n; n += (long long)gridDim.x * blockDim.x) {
@@ -61,7 +65,13 @@ __global__ void __launch_bounds__(256) k_cfl_dt(DevBlock b, DevState s, double c
   if (threadIdx.x == 0) {
     double m = wmin[0];
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmin(m, wmin[w]);
-    atomicMin(dtbits, (unsigned long long)__double_as_longlong(m));
+    atomicMin(&w->bits, (unsigned long long)__double_as_longlong(m));
+    __threadfence();
+    if (atomicAdd(&w->arrived, 1u) == total - 1) {
+      __threadfence();
+      *dt = __longlong_as_double((long long)atomicExch(&w->bits, (unsigned long long)__double_as_longlong(1e6)));
+      w->arrived = 0;
+    }
   }
 }
 
@@ -1117,8 +1127,6 @@ __global__ void k_step_end(double *t, const double *dt, long long *step) {
   *t += *dt;
   *step += 1;
 }
-
-__global__ void k_dt_decode(const unsigned long long *bits, double *dt) { *dt = __longlong_as_double((long long)*bits); }
 
 // ------------------------------------------------------------------------------ digital-filter inflow
 

@@ -343,7 +343,7 @@ int ostc_create(const char *setup_txt, const char *input_dir, int device, ostc_c
     ctx->blk.push_back(R);
   }
   ctx->block_set.assign(ctx->blk.size(), 0);
-  bool ok = cudaMalloc(&ctx->d_dtbits, sizeof(unsigned long long)) == cudaSuccess &&
+  bool ok = cudaMalloc(&ctx->d_dtw, sizeof(DtScratch)) == cudaSuccess &&
             cudaMalloc(&ctx->d_dt, sizeof(double)) == cudaSuccess && cudaMalloc(&ctx->d_time, sizeof(double)) == cudaSuccess &&
             cudaMalloc(&ctx->d_sums, 4 * sizeof(double)) == cudaSuccess &&
             cudaMalloc(&ctx->d_step, sizeof(long long)) == cudaSuccess &&
@@ -504,6 +504,10 @@ int ostc_create(const char *setup_txt, const char *input_dir, int device, ostc_c
     }
   const double dt0 = ctx->der.fixed_time_step ? ctx->der.dt : 1e6;
   cudaMemcpy(ctx->d_dt, &dt0, sizeof(double), cudaMemcpyHostToDevice);
+  DtScratch dtw{};
+  const double dt_max = 1e6;
+  std::memcpy(&dtw.bits, &dt_max, sizeof(double));
+  cudaMemcpy(ctx->d_dtw, &dtw, sizeof(dtw), cudaMemcpyHostToDevice);
   cudaMemset(ctx->d_time, 0, sizeof(double));
   cudaMemset(ctx->d_step, 0, sizeof(long long));
   cudaMemset(ctx->d_flags, 0, sizeof(unsigned));
@@ -605,7 +609,7 @@ void ostc_destroy(ostc_ctx *ctx) {
                   (void *)ctx->df.vold, (void *)ctx->df.fluc, (void *)ctx->df.lund, (void *)ctx->df.by,
                   (void *)ctx->df.bz, (void *)ctx->df.yface, (void *)ctx->d_zero})
     cudaFree(p);
-  cudaFree(ctx->d_dtbits);
+  cudaFree(ctx->d_dtw);
   cudaFree(ctx->d_dt);
   cudaFree(ctx->d_time);
   cudaFree(ctx->d_sums);

@@ -79,7 +79,7 @@ struct ostc_ctx {
   int precision = OSTC_PREC_FP64;
   bool state_set = false, initialised = false;
   std::vector<char> block_set;
-  unsigned long long *d_dtbits = nullptr;
+  DtScratch *d_dtw = nullptr;
   double *d_dt = nullptr, *d_time = nullptr, *d_sums = nullptr, *d_staging = nullptr;
   long long *d_step = nullptr;
   unsigned *d_flags = nullptr;

@@ -721,11 +721,11 @@ void for_blocks(ostc_ctx *ctx, F f) {
 // CFL time step of the current state (slot 0) into d_dt (local_time_step + global_time_step)
 void enqueue_cfl_dt(ostc_ctx *ctx) {
   long tok = begin_t(ctx, "cfl_dt");
-  k_dt_reset<<<1, 1, 0, ctx->stream>>>(ctx->d_dtbits);
+  unsigned total = 0;
+  for (auto &B : ctx->blk) total += (unsigned)grid_for(ctx, B.db.n, 256);
   for (auto &B : ctx->blk)
-    k_cfl_dt<<<grid_for(ctx, B.db.n, 256), 256, 0, ctx->stream>>>(B.db, state_of(B, 0), ctx->der.cfl,
-                                                                 ctx->der.prandtl, B.db.mz > 1, ctx->d_dtbits);
-  k_dt_decode<<<1, 1, 0, ctx->stream>>>(ctx->d_dtbits, ctx->d_dt);
+    k_cfl_dt<<<grid_for(ctx, B.db.n, 256), 256, 0, ctx->stream>>>(B.db, state_of(B, 0), ctx->der.cfl, ctx->der.prandtl,
+                                                                 B.db.mz > 1, ctx->d_dtw, total, ctx->d_dt);
   end_t(ctx, tok);
 }
 
