@@ -61,24 +61,24 @@ METRIC = "cell-steps/s on 1 B200: mixed vs FP64 RHS at stated rel-L2 error; % of
 UNIT = "cell-steps/s"
 FALLBACK_HBM_GBS = 6650.0
 # Compulsory bytes per interior node of each kernel family (FP64 loads/stores the kernel must make):
-#   flux_x      cv(5) + rho,u,v,w,p(5) + metric row(3) + jac(1) read, dq(5) written          = 19 x 8
-#   flux_y/z    the same reads, dq(5) read-modify-written                                     = 24 x 8
-#   visc_update u,v,w,T(4) + mu + metric(9) + jac + dq(5) + cv_in(5) + q^n(5) read,
-#               cv(5) + bv(6) + mu written                                                    = 42 x 8
+# (of the rectilinear kernels, which the uniform grids here take):
+#   flux_x      cv(5) + rho,u,v,w,p(5) + metric(1) + jac(1) read, dq(5) written              = 17 x 8
+#   flux_y/z    the same reads, dq(5) read-modify-written                                     = 22 x 8
+#   visc_update u,v,w,T(4) + mu + metric(3) + jac + dq(5) + cv_in(5) + q^n(5) read,
+#               cv(5) + bv(6) + mu written                                                    = 36 x 8
 #   cfl_dt      metric(9) + rho,u,v,w,T(5) + mu read                                          = 15 x 8
-ALGO_BYTES_PER_NODE = {"flux_x": 152, "flux_y": 192, "flux_z": 192, "visc_update": 336, "cfl_dt": 120}
+ALGO_BYTES_PER_NODE = {"flux_x": 136, "flux_y": 176, "flux_z": 176, "visc_update": 288, "cfl_dt": 120}
 # DRAM bytes per node measured by one ncu capture of the kernel (dram__bytes_read.sum +
 # dram__bytes_write.sum over the nodes of the launch, 256x128x64 case of the same workload; traffic
 # grows with the node count, so a full-size launch moves this figure times its nodes).  The y/z
-# sweeps have several designs picked by the library's autotuner; at 512x256x128 it keeps 16-lane
-# tiles, and the capture is of the 16 x 16 x 1 tile (the column march moved 209.8, the 32x4x4 tile
-# 194-203 B per node).
-MEASURED_TRAFFIC_PER_NODE = {"flux_y": 214.5, "flux_z": 214.5}
+# sweeps have several tile shapes picked by the library's autotuner; the capture is of the
+# 8 x 16 x 2 tile on a rectilinear block.
+MEASURED_TRAFFIC_PER_NODE = {"flux_y": 175.1, "flux_z": 182.2}
 # FP64 operations per face of the y/z sweep (AWENO7 + HLLC, central correction), from the same
 # capture's instruction counters: 2 x DFMA + DMUL + DADD thread-instructions over the launch's faces.
 # Against the FP64 FMA peak of the part (64 DFMA per cycle per SM) this is the roof the sweeps run
 # into; the HBM fraction above stays far from 1 because the sweeps are arithmetic bound.
-FP64_FLOP_PER_FACE = 3275
+FP64_FLOP_PER_FACE = 2060
 FP64_DFMA_PER_CYCLE_PER_SM = 64
 # Whole fused stage (three state passes + metric): 8 (3 n_var + 10) bytes per cell-stage, n_var = 5
 STAGE_BYTES = 8 * (3 * 5 + 10)
