@@ -10,7 +10,6 @@ namespace ostc {
 
 constexpr int kMS = 16;  // species capacity of the device tables
 constexpr int kMR = 64;  // reaction capacity
-constexpr int kMV = 5 + kMS;
 constexpr int kMol = 4, kNet = 6;  // molecules a side and species of a reaction in the lists of MixTables
 constexpr double kPatmD = 101325.0;
 

@@ -560,8 +560,7 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
   }
   const int n = start - 1 + t;
   const bool face_ok = i0 < b.mx && n < nd;
-  T fv[Spec<NS>::A + 5];
-  for (int l = 0; l < kMV; ++l) fv[l] = T(0);
+  T fv[Spec<NS>::A + 5] = {};
   if (face_ok) {
     const long long p0 = DIR == 0 ? b.id(n, j0, k0) : DIR == 1 ? b.id(i0, n, k0) : b.id(i0, j0, n);
     mix_visc_face<DIM3, NS, T>(b, s, p0, DIR, nv, fv);
