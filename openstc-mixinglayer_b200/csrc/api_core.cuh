@@ -162,7 +162,7 @@ int ostc_create(const char *setup_txt, const char *input_dir, int device, ostc_c
     return OSTC_ECUDA;
   }
   cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device);
-  if (!set_sweep_attrs<double>() || !set_sweep_attrs<float>() || !set_mix_attrs(ctx->nv)) {
+  if (!set_sweep_attrs<double>() || !set_sweep_attrs<float>() || !set_mix_attrs()) {
     g_create_error = "cudaFuncSetAttribute (dynamic shared memory) failed";
     return OSTC_ECUDA;
   }

@@ -638,38 +638,33 @@ bool set_sweep_attrs() {
   return ok;
 }
 
-// dynamic shared memory of the flux-split and mixture viscous sweeps (up to ~45 KB at n_var 14)
-bool set_mix_attrs(int nv) {
+// Dynamic shared memory limits of the mixture kernels.  A limit belongs to the kernel, not to a context, and a
+// launch that asks for more fails; contexts of several species counts live side by side, so every kernel gets
+// the limit of the most species it can run: kFixedNS in the instantiation for that count, the tables' capacity
+// in the generic one.  (Setting it again for the next context changes nothing; the occupancy follows each
+// launch's own size.)  9 species: sweeps up to 60 KB, implicit chemistry 55 KB, reverse sweeps 110 KB; 16
+// species: 94, 156, 173 KB.
+bool set_mix_attrs() {
   bool ok = true;
   auto set = [&](const void *fn, size_t bytes) {
     ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
   };
-#define OSTC_FSET(T)                                                      \
-  set((const void *)k_fvs<0, 0, T>, fvs_smem_bytes<0, T>(nv));            \
-  set((const void *)k_fvs<1, 0, T>, fvs_smem_bytes<1, T>(nv));            \
-  set((const void *)k_fvs<2, 0, T>, fvs_smem_bytes<2, T>(nv));            \
-  set((const void *)k_fvs<0, kFixedNS, T>, fvs_smem_bytes<0, T>(nv));     \
-  set((const void *)k_fvs<1, kFixedNS, T>, fvs_smem_bytes<1, T>(nv));     \
-  set((const void *)k_fvs<2, kFixedNS, T>, fvs_smem_bytes<2, T>(nv));
-  OSTC_FSET(double)
-  OSTC_FSET(float)
-#undef OSTC_FSET
-  const int ns = nv - 5;
-  if (ns > 0) {
-    const size_t src = chem_columns(ns, false) * 128 * sizeof(double), epi = chem_columns(ns, true) * 64 * sizeof(double);
-    set((const void *)k_mix_source<0, true>, src);
-    set((const void *)k_mix_source<kFixedNS, true>, src);
-    set((const void *)k_mix_chem_epi<0, true>, epi);
-    set((const void *)k_mix_chem_epi<kFixedNS, true>, epi);
-    set((const void *)k_adj_source_listed<0>, 5 * ns * 128 * sizeof(double));
-    set((const void *)k_adj_source_listed<kFixedNS>, 5 * ns * 128 * sizeof(double));
-  }
-  set((const void *)k_adj_fvs<0, 0>, adj_fvs_smem_bytes<0>(nv));
-  set((const void *)k_adj_fvs<1, 0>, adj_fvs_smem_bytes<1>(nv));
-  set((const void *)k_adj_fvs<2, 0>, adj_fvs_smem_bytes<2>(nv));
-  set((const void *)k_adj_fvs<0, kFixedNS>, adj_fvs_smem_bytes<0>(nv));
-  set((const void *)k_adj_fvs<1, kFixedNS>, adj_fvs_smem_bytes<1>(nv));
-  set((const void *)k_adj_fvs<2, kFixedNS>, adj_fvs_smem_bytes<2>(nv));
+#define OSTC_MSET(NS, N)                                                                     \
+  set((const void *)k_fvs<0, NS, double>, fvs_smem_bytes<0, double>(5 + N));                 \
+  set((const void *)k_fvs<1, NS, double>, fvs_smem_bytes<1, double>(5 + N));                 \
+  set((const void *)k_fvs<2, NS, double>, fvs_smem_bytes<2, double>(5 + N));                 \
+  set((const void *)k_fvs<0, NS, float>, fvs_smem_bytes<0, float>(5 + N));                   \
+  set((const void *)k_fvs<1, NS, float>, fvs_smem_bytes<1, float>(5 + N));                   \
+  set((const void *)k_fvs<2, NS, float>, fvs_smem_bytes<2, float>(5 + N));                   \
+  set((const void *)k_mix_source<NS, true>, chem_columns(N, false) * 128 * sizeof(double));  \
+  set((const void *)k_mix_chem_epi<NS, true>, chem_columns(N, true) * 64 * sizeof(double));  \
+  set((const void *)k_adj_source_listed<NS>, 5 * N * 128 * sizeof(double));                  \
+  set((const void *)k_adj_fvs<0, NS>, adj_fvs_smem_bytes<0>(5 + N));                         \
+  set((const void *)k_adj_fvs<1, NS>, adj_fvs_smem_bytes<1>(5 + N));                         \
+  set((const void *)k_adj_fvs<2, NS>, adj_fvs_smem_bytes<2>(5 + N));
+  OSTC_MSET(0, kMS)
+  OSTC_MSET(kFixedNS, kFixedNS)
+#undef OSTC_MSET
   return ok;
 }
 
