@@ -1032,9 +1032,10 @@ __global__ void __launch_bounds__(128, 4) k_adj_source_listed(DevBlock b, DevSta
         const double ratio = reaction_kb<double>(r, lt, ti, cc, 1.0, sg);
         kb_t = ratio * kf_t + kb * (sdg + c_mix.order[r] * ti);
         kb_c = ratio * kf_c;
-      } else if (kb != 0.0) {
+      } else if (ty != 0 && c_mix.rev_type[r] == 1) {
         kb_t = kb * (c_mix.b2[r] + c_mix.Ea2[r] * ti) * ti;
-        if (ty == 4) kb_c = kb / cc;
+        // times the third-body sum, which is zero where no collider is present (its derivative is not)
+        if (ty == 4) kb_c = arrhenius(lt, ti, c_mix.A2[r], c_mix.b2[r], c_mix.Ea2[r]);
       }
       double p1 = 1.0, p2 = 1.0;
       for (int e = 0; e < nf; ++e) {
