@@ -231,9 +231,10 @@ int ostc_tune_report(ostc_ctx *ctx, int block, int precision, int dir, int *chos
 int ostc_total_nodes(const ostc_ctx *ctx, long long *n);
 
 /* Host-only parse of a case directory (no device is touched): runs the setup/grid/boundary readers
- * and writes out[0..13] = ngg, inviscid_type, n_var, n_scalar, n_block, dimension, mx, my, mz of
+ * and writes out[0..14] = ngg, inviscid_type, n_var, n_scalar, n_block, dimension, mx, my, mz of
  * block 0, number of boundary faces of block 0, reconstruction, inviscid_scheme, viscous_order,
- * number of boundary-face applications per stage.  On failure msg receives the reason
+ * number of boundary-face applications per stage, number of blocks whose grid lines are the coordinate
+ * axes (they take the kernels without the off-diagonal metric terms).  On failure msg receives the reason
  * (Parameter::deduce_known_info / Mesh::Mesh checks, Parameter.cpp:187-437, Mesh.cpp:592-641). */
 int ostc_probe_case(const char *setup_txt, const char *input_dir, int out[16], char *msg, int msg_len);
 

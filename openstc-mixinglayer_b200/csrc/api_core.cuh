@@ -236,17 +236,7 @@ int ostc_create(const char *setup_txt, const char *input_dir, int device, ostc_c
           hj[d] = HB.jac[h];
           for (int r = 0; r < 9; ++r) hm[r * b.plane + d] = HB.metric[r * HP + h];
         }
-    // rectilinear: every off-diagonal metric entry the kernels read (nodes with at most one index among
-    // the ghosts) is zero but for the rounding of the ghost grid's reflections
-    b.rect = 1;
-    for (int k = -b.gz; k < b.mz + b.gz && b.rect; ++k)
-      for (int j = -b.g; j < b.my + b.g && b.rect; ++j)
-        for (int i = -b.g; i < b.mx + b.g && b.rect; ++i) {
-          if ((i < 0 || i >= b.mx) + (j < 0 || j >= b.my) + (k < 0 || k >= b.mz) > 1) continue;
-          const long long q = b.id(i, j, k);
-          for (int r = 0; r < 9; ++r)
-            if (r % 4 != 0 && !(std::fabs(hm[r * b.plane + q]) <= 1e-12 * std::fabs(hm[r / 3 * 4 * b.plane + q]))) b.rect = 0;
-        }
+    b.rect = rectilinear(HB, ctx->mesh.dimension);
     cudaMemcpy(R.met, hm.data(), hm.size() * sizeof(double), cudaMemcpyHostToDevice);
     cudaMemcpy(R.jac, hj.data(), hj.size() * sizeof(double), cudaMemcpyHostToDevice);
     b.met = R.met;

@@ -75,10 +75,12 @@ int ostc_probe_case(const char *setup_txt, const char *input_dir, int out[16], c
   }
   const auto order = bc_order(setup, mesh);
   const HostBlock &B = mesh.blocks[0];
-  const int vals[14] = {der.ngg, der.inviscid_type, der.n_var, der.n_scalar, (int)mesh.blocks.size(), mesh.dimension,
+  int n_rect = 0;
+  for (const auto &Q : mesh.blocks) n_rect += rectilinear(Q, mesh.dimension);
+  const int vals[15] = {der.ngg, der.inviscid_type, der.n_var, der.n_scalar, (int)mesh.blocks.size(), mesh.dimension,
                         B.mx, B.my, B.mz, (int)B.faces.size(), der.reconstruction, der.inviscid_scheme,
-                        der.viscous_order, (int)order.size()};
-  for (int i = 0; i < 14; ++i) out[i] = vals[i];
+                        der.viscous_order, (int)order.size(), n_rect};
+  for (int i = 0; i < 15; ++i) out[i] = vals[i];
   return OSTC_OK;
 }
 

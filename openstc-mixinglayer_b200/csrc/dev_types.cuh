@@ -19,8 +19,8 @@ struct DevBlock {
   // air: FP32 copies of the 9 metric planes and the Jacobian (plane 9), read by the mixed-precision
   // viscous sweep (the values it would round from met / jac); null for mixtures
   const float *met32;
-  // rectilinear block: the off-diagonal metric entries are zero (to 1e-12 of their row's diagonal, the
-  // rounding of the ghost grid), and the kernels leave their terms out
+  // rectilinear block (rectilinear() in host.h): the off-diagonal metric entries are zero but for rounding, and
+  // the kernels leave their terms out
   int rect;
   __host__ __device__ __forceinline__ long long id(int i, int j, int k) const {
 #if defined(OSTC_BOUNDS_CHECK) && defined(__CUDA_ARCH__)

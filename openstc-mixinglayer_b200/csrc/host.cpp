@@ -627,6 +627,31 @@ void inner_ghost_grid(HostMesh &mesh) {
 }
 }  // namespace
 
+bool rectilinear(const HostBlock &B, int dimension) {
+  const int n[3] = {B.mx, B.my, B.mz};
+  // f(i, j, k) at the nodes with at most one index among `g` ghost layers (no z ghosts in 2-D)
+  auto every = [&](int g, auto f) {
+    const int gz = dimension == 3 ? g : 0;
+    for (int k = -gz; k < n[2] + gz; ++k)
+      for (int j = -g; j < n[1] + g; ++j)
+        for (int i = -g; i < n[0] + g; ++i)
+          if ((i < 0 || i >= n[0]) + (j < 0 || j >= n[1]) + (k < 0 || k >= n[2]) <= 1 && !f(i, j, k)) return false;
+    return true;
+  };
+  if (!every(B.ngg + 1, [&](int i, int j, int k) {
+        const long p = B.cidx(i, j, k);
+        return B.x[p] == B.x[B.cidx(i, 0, 0)] && B.y[p] == B.y[B.cidx(0, j, 0)] && B.z[p] == B.z[B.cidx(0, 0, k)];
+      }))
+    return false;
+  const long P = B.padded();
+  return every(B.ngg, [&](int i, int j, int k) {
+    const double *m = B.metric.data() + B.gidx(i, j, k);
+    for (int r = 0; r < 9; ++r)
+      if (r % 4 != 0 && !(std::fabs(m[r * P]) <= 1e-12 * std::fabs(m[r / 3 * 4 * P]))) return false;
+    return true;
+  });
+}
+
 bool read_mesh(const std::string &dir, const Derived &d, HostMesh &mesh, std::string &err) {
   const std::string gpath = dir + "/grid/grid   0.dat";
   FILE *fp = std::fopen(gpath.c_str(), "rb");

@@ -161,6 +161,13 @@ struct HostMesh {
   std::vector<HostBlock> blocks;
 };
 
+// Whether the block's grid lines are the coordinate axes: x a function of i alone, y of j, z of k, bit for bit,
+// at every node with at most one index among the ghosts.  The off-diagonal metric entries the kernels read are
+// then zero but for the rounding of the parallelogram rule that makes the ghost grid's edges, so leaving their
+// terms out leaves out rounding; a block where that rounding passes 1e-12 of an entry's diagonal (the bar of the
+// parity tests: coordinates above ~1e3 spacings from the origin) counts as general all the same.
+bool rectilinear(const HostBlock &B, int dimension);
+
 // Reads "<dir>/grid/grid   0.dat" (binary, Mesh.cpp:663-697), the boundary and inner-face files
 // (Mesh.cpp:790-844), scales, builds ghost grids and metrics.
 bool read_mesh(const std::string &input_dir, const Derived &d, HostMesh &mesh, std::string &err);

@@ -127,7 +127,7 @@ def probe_case(input_dir: str, setup: str | None = None) -> dict:
     if rc != 0:
         raise OstcError(rc, msg.value.decode())
     keys = ["ngg", "inviscid_type", "n_var", "n_scalar", "n_block", "dimension", "mx", "my", "mz",
-            "n_faces", "reconstruction", "inviscid_scheme", "viscous_order", "n_bc_launches"]
+            "n_faces", "reconstruction", "inviscid_scheme", "viscous_order", "n_bc_launches", "n_rectilinear"]
     return {k: out[i] for i, k in enumerate(keys)}
 
 
