@@ -318,13 +318,12 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
     const double kxJd = b.met[(DIR * 3 + 0) * P + pl] * jld + b.met[(DIR * 3 + 0) * P + pr] * jrd;
     const double kyJd = b.met[(DIR * 3 + 1) * P + pl] * jld + b.met[(DIR * 3 + 1) * P + pr] * jrd;
     const double kzJd = b.met[(DIR * 3 + 2) * P + pl] * jld + b.met[(DIR * 3 + 2) * P + pr] * jrd;
-    const double eps = 1e-40 * c_mix.weno_eps_scale * 0.25 * (kxJd * kxJd + kyJd * kyJd + kzJd * kzJd);
-    // the unit normal: the Jacobian-weighted mean metric, its length cancels
-    T kx = (T)kxJd, ky = (T)kyJd, kz = (T)kzJd;
-    const T igk = T(1) / tsqrt(kx * kx + ky * ky + kz * kz);
-    kx *= igk;
-    ky *= igk;
-    kz *= igk;
+    const double k2 = kxJd * kxJd + kyJd * kyJd + kzJd * kzJd;
+    const double eps = 1e-40 * c_mix.weno_eps_scale * 0.25 * k2;
+    // the unit normal: the Jacobian-weighted mean metric, its length cancels.  In FP64 for either T: the square
+    // of a face area leaves the FP32 range below 1e-19 (and above 1e19) square grid units
+    const double igk = 1.0 / sqrt(k2);
+    const T kx = (T)(kxJd * igk), ky = (T)(kyJd * igk), kz = (T)(kzJd * igk);
     const T Ukb = kx * um + ky * vm_ + kz * wm;
     const T alpha = gm1 * ekm, icm = cm * c2i, h2 = half * c2i;
     const T hc = hm - cm * cm / gm1;

@@ -1,0 +1,59 @@
+"""The flux-split sweeps far from the usual grid sizes.  Their weights do not change when the grid is scaled (the
+epsilon follows the split fluxes), so with a grid scaled by a power of two, which scales every metric entry without
+rounding, the inviscid right-hand side is that of the plain grid times the square of the factor.
+
+Tolerance: the operations are the same ones on scaled operands; what may differ is the rounding where a quotient
+takes another of its equivalent forms: a few rounding errors of the terms that sum to an entry, 1e-6 (FP32) of each
+variable's largest entry.
+"""
+import numpy as np
+import pytest
+
+import ostc_cases as oc
+
+pytestmark = pytest.mark.gpu
+
+
+def layer(scheme, power, zero_half=()):
+    """9 species on a grid scaled by 2^power; species of zero_half are absent from the half with low i."""
+    case = oc.reacting_mixing_layer_3d(18, 14, 10, inviscid_scheme=scheme, finite_rate=False)
+    case.grid_scale = case.grid_scale * 2.0 ** power
+    tb = case.mixture["tables"]
+    for n in zero_half:
+        l = tb.names.index(n)
+        case.sv[tb.names.index("N2"), ..., :9] += case.sv[l, ..., :9]
+        case.sv[l, ..., :9] = 0.0
+    mw = 1 / np.einsum("l...,l->...", case.sv, 1 / tb.mw)
+    case.bv[0] = case.bv[4] * mw / (oc.R_U * case.bv[5])
+    return case
+
+
+def relative(a, b):
+    """Largest difference of each variable over its largest entry (the three momentum components share one)."""
+    top = [np.max(np.abs(v)) for v in b]
+    top[1:4] = [max(top[1:4])] * 3
+    return max(np.max(np.abs(x - y)) / t for x, y, t in zip(a, b, top))
+
+
+def solver(case, path):
+    import ostc
+
+    s = ostc.Solver(str(oc.write_case(case, path)))
+    s.set_state(case.bv, sv=case.sv)
+    return s
+
+
+@pytest.mark.parametrize("scheme", [71, 72])
+@pytest.mark.parametrize("power", [-25, 25])
+def test_mixed_precision(built, tmp_path, scheme, power):
+    """2^-25: face areas of 1e-23, whose squares FP32 cannot hold."""
+    import ostc
+
+    out = []
+    for p in (0, power):
+        s = solver(layer(scheme, p), tmp_path / f"p{p}")
+        s.set_precision(ostc.PREC_MIXED)
+        out.append(s.rhs(1))
+        s.close()
+    assert np.all(np.isfinite(out[1]))
+    assert relative(out[1] * 2.0 ** (-2 * power), out[0]) <= 1e-6
