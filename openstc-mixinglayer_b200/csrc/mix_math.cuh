@@ -556,11 +556,9 @@ __device__ __forceinline__ T fvs_beta7(T s1, T s2, T s3) {
   return s1 * (s1 + T(1.0 / 12) * s3) + T(13.0 / 12.0) * s2 * s2 + T(1043.0 / 960) * s3 * s3;
 }
 
-// tau / D_k of the four Z weights, D_k = (eps + beta_k)^2.  FP64: the four 1 / (eps + beta_k) from one
-// division where the product of the four stays in range (an eps above 1e-75), else each
-// takes its own.  FP32: four fast divisions, D_k floored at 1e-30 so that a smooth stencil (beta = 0, where
-// the scaled eps underflows) gives the linear weights instead of 0/0.
-__device__ __forceinline__ void fvs_ratios(double tau, double eps, const double *b, double *r) {
+// 1 / (eps + beta_k) of the four Z weights: from one division where the product of the four stays in range (on
+// a smooth stencil, an eps above 1e-75), else each takes its own.
+__device__ __forceinline__ void fvs_inverses(double eps, const double *b, double *r) {
   const double g0 = eps + b[0], g1 = eps + b[1], g2 = eps + b[2], g3 = eps + b[3];
   const double p01 = g0 * g1, p23 = g2 * g3, p = p01 * p23;
   if (p > 1e-300 && p < 1e300) {
@@ -575,6 +573,12 @@ __device__ __forceinline__ void fvs_ratios(double tau, double eps, const double 
     r[2] = 1.0 / g2;
     r[3] = 1.0 / g3;
   }
+}
+
+// tau / D_k of the four Z weights, D_k = (eps + beta_k)^2.  FP32: four fast divisions, D_k floored at 1e-30 so that
+// a smooth stencil (beta = 0, where the scaled eps underflows) gives the linear weights instead of 0/0.
+__device__ __forceinline__ void fvs_ratios(double tau, double eps, const double *b, double *r) {
+  fvs_inverses(eps, b, r);
 #pragma unroll
   for (int k = 0; k < 4; ++k) r[k] = tau * (r[k] * r[k]);
 }

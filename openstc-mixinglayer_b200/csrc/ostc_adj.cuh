@@ -41,24 +41,7 @@ __device__ __forceinline__ double weno7_side_bwd(const double *v, double eps, do
   double b[4], id[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) b[k] = fvs_beta7(s1[k], s2[k], s3[k]);
-  {
-    // 1 / (eps + b_k) from one division; their product is at least eps^4, and where that leaves the range
-    // (an eps below 1e-75) each takes its own
-    const double g0 = eps + b[0], g1 = eps + b[1], g2 = eps + b[2], g3 = eps + b[3];
-    const double p01 = g0 * g1, p23 = g2 * g3, P = p01 * p23;
-    if (P > 1e-300) {
-      const double q = 1.0 / P, q01 = p23 * q, q23 = p01 * q;
-      id[0] = g1 * q01;
-      id[1] = g0 * q01;
-      id[2] = g3 * q23;
-      id[3] = g2 * q23;
-    } else {
-      id[0] = 1.0 / g0;
-      id[1] = 1.0 / g1;
-      id[2] = 1.0 / g2;
-      id[3] = 1.0 / g3;
-    }
-  }
+  fvs_inverses(eps, b, id);
   const double db = b[0] - b[3], tau = db * db;
   double a[4], q[4], S = 0, num = 0;
 #pragma unroll

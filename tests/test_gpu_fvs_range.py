@@ -3,8 +3,8 @@ epsilon follows the split fluxes), so with a grid scaled by a power of two, whic
 rounding, the inviscid right-hand side is that of the plain grid times the square of the factor.
 
 Tolerance: the operations are the same ones on scaled operands; what may differ is the rounding where a quotient
-takes another of its equivalent forms: a few rounding errors of the terms that sum to an entry, 1e-6 (FP32) of each
-variable's largest entry.
+takes another of its equivalent forms: a few rounding errors of the terms that sum to an entry, 1e-6 (FP32) and 1e-12
+(FP64, whose adjoint adds a node's ~200 terms in any order) of each variable's largest entry.
 """
 import numpy as np
 import pytest
@@ -57,3 +57,19 @@ def test_mixed_precision(built, tmp_path, scheme, power):
         s.close()
     assert np.all(np.isfinite(out[1]))
     assert relative(out[1] * 2.0 ** (-2 * power), out[0]) <= 1e-6
+
+
+@pytest.mark.parametrize("scheme", [71, 72])
+@pytest.mark.parametrize("power", [-25, 70, 75])
+def test_fp64_and_adjoint(built, tmp_path, scheme, power):
+    """Radicals absent from half of the block: eps alone in the weights' denominators there.  2^-25 takes the product
+    of four of them below the FP64 range; 2^70 and 2^75 take that of four indicators above it."""
+    rhs, vjp = [], []
+    for p in (0, power):
+        s = solver(layer(scheme, p, ("OH", "O", "H", "HO2", "H2O2")), tmp_path / f"p{p}")
+        rhs.append(s.rhs(1))
+        vjp.append(s.rhs_vjp(np.random.default_rng(3).standard_normal(rhs[0].shape), 1))
+        s.close()
+    for out in (rhs, vjp):
+        assert np.all(np.isfinite(out[1])) and np.any(out[0])
+        assert relative(out[1] * 2.0 ** (-2 * power), out[0]) <= 1e-12
