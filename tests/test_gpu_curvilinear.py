@@ -1,7 +1,7 @@
 """Wavy (non-orthogonal) grids and tile edges against the CPU oracle: the general metric branch of the
 mixture viscous faces (cross differences of T and the mass fractions, which a rectilinear grid skips),
 the flux-split and AWENO sweeps with all three metric components, extents at the edges of the sweeps'
-tiles, mass fractions far below rounding (the flux-split weights' divisions in pairs) and reactions with
+tiles, mass fractions far below rounding (the flux-split weights' epsilon) and reactions with
 more species than the reaction lists hold (the dense chemistry).
 
 Tolerances: 1e-12 relative per conserved variable over two RK3 steps as the other trajectory tests; the
@@ -70,8 +70,8 @@ def test_mixture_tile_edges(built, tmp_path, dims):
 
 @pytest.mark.parametrize("scale", [1e-12, 1e-60])
 def test_mixture_vanishing_species(built, tmp_path, scale):
-    """Radicals scaled towards zero: the products of the flux-split weights' denominators leave the FP64
-    range, and the quotients fall back to one division per pair and then per weight."""
+    """Radicals scaled towards zero: their indicators fall towards epsilon (1e-12) and far below it (1e-60).  The
+    four weights still share a division here; tests/test_gpu_fvs_range.py leaves that form at both ends."""
     case = oc.reacting_mixing_layer_3d(mx=20, my=18, mz=10, finite_rate=False)
     names = case.mixture["tables"].names
     for n in ("OH", "O", "H", "HO2", "H2O2"):

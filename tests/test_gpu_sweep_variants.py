@@ -1,5 +1,5 @@
 """Every kernel shape of the AWENO sweeps computes the same face fluxes: pinned through
-ostc_set_sweep_variant, each y / z variant (column march; three shared-memory tiles) advances the case
+ostc_set_sweep_variant, each y / z variant (shared-memory tiles of four shapes) advances the case
 to the same state as the default shapes - FP64 and mixed precision, WENO7-Z + HLLC and WENO5-Z + AUSM+,
 3-D - within 1e-13 relative (the expressions are the same; the compiler may fuse a multiply-add
 differently in another kernel body), and the FP64 one matches the oracle to 1e-12."""
