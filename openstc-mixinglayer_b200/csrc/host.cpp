@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <fstream>
+#include <limits>
 #include <sstream>
 
 namespace ostc {
@@ -638,9 +639,20 @@ bool rectilinear(const HostBlock &B, int dimension) {
           if ((i < 0 || i >= n[0]) + (j < 0 || j >= n[1]) + (k < 0 || k >= n[2]) <= 1 && !f(i, j, k)) return false;
     return true;
   };
+  double top[3] = {0, 0, 0};
+  for (size_t p = 0; p < B.x.size(); ++p) {
+    top[0] = std::max(top[0], std::fabs(B.x[p]));
+    top[1] = std::max(top[1], std::fabs(B.y[p]));
+    top[2] = std::max(top[2], std::fabs(B.z[p]));
+  }
+  const double eps = std::numeric_limits<double>::epsilon();
   if (!every(B.ngg + 1, [&](int i, int j, int k) {
+        const bool own = i >= 0 && i < n[0] && j >= 0 && j < n[1] && k >= 0 && k < n[2];
+        const double tol = own ? 0.0 : 4 * eps;
         const long p = B.cidx(i, j, k);
-        return B.x[p] == B.x[B.cidx(i, 0, 0)] && B.y[p] == B.y[B.cidx(0, j, 0)] && B.z[p] == B.z[B.cidx(0, 0, k)];
+        return std::fabs(B.x[p] - B.x[B.cidx(i, 0, 0)]) <= tol * top[0] &&
+               std::fabs(B.y[p] - B.y[B.cidx(0, j, 0)]) <= tol * top[1] &&
+               std::fabs(B.z[p] - B.z[B.cidx(0, 0, k)]) <= tol * top[2];
       }))
     return false;
   const long P = B.padded();

@@ -161,11 +161,14 @@ struct HostMesh {
   std::vector<HostBlock> blocks;
 };
 
-// Whether the block's grid lines are the coordinate axes: x a function of i alone, y of j, z of k, bit for bit,
-// at every node with at most one index among the ghosts.  The off-diagonal metric entries the kernels read are
-// then zero but for the rounding of the parallelogram rule that makes the ghost grid's edges, so leaving their
-// terms out leaves out rounding; a block where that rounding passes 1e-12 of an entry's diagonal (the bar of the
-// parity tests: coordinates above ~1e3 spacings from the origin) counts as general all the same.
+// Whether the block's grid lines are the coordinate axes: x a function of i alone, y of j, z of k, at every node
+// with at most one index among the ghosts - bit for bit at the block's own nodes, within 4 epsilon of the largest
+// coordinate in the ghost layers, where a neighbour's coordinates stand beside reflected ones (up to eight
+// roundings of half an epsilon: two of the mirror node, one of the node, the result and the neighbour's, and of
+// the generator's sums).  The off-diagonal metric entries the kernels read are then zero but for that rounding and
+// the ghost edges' (the parallelogram rule), so leaving their terms out leaves out rounding; a block where it passes
+// 1e-12 of an entry's diagonal (the bar of the parity tests: coordinates above ~1e3 spacings from the origin)
+// counts as general all the same.
 bool rectilinear(const HostBlock &B, int dimension);
 
 // Reads "<dir>/grid/grid   0.dat" (binary, Mesh.cpp:663-697), the boundary and inner-face files

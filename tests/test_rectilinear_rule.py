@@ -1,5 +1,6 @@
 """Which blocks run the kernels without the off-diagonal metric terms (host side, no GPU): those whose grid lines
-are the coordinate axes bit for bit.  A shear of any size, or one node off its line by one ulp, is not."""
+are the coordinate axes, bit for bit at their own nodes and to rounding in their ghost layers.  A shear of any size, or one node
+off its line by one ulp, is not."""
 import numpy as np
 import pytest
 
@@ -59,3 +60,10 @@ def test_chain(built, tmp_path):
     case.blocks[1].x = case.blocks[1].x + 1e-13 * case.blocks[1].y
     # the sheared block, and its neighbours, whose ghosts are its nodes
     assert _count(case, tmp_path) == 0
+
+
+def test_chain_of_uneven_blocks(built, tmp_path):
+    """Interfaces on parts of a side: the ghost layer holds the neighbour's coordinates beside reflected ones, which
+    differ by rounding."""
+    case = oc.multiblock_mixing_layer_3d(nb=6, lo=16, hi=40, seed=3, uneven_axes=True)
+    assert _count(case, tmp_path) == 6
