@@ -83,28 +83,35 @@ void launch_flux_pv(ostc_ctx *ctx, BlockRes &B, DevState in) {
 }
 
 // flux-split WENO7 sweeps (inviscid_type 3, schemes 71 / 72), accumulating into dq
-template <int NS, typename T>
-void launch_fvs_t(ostc_ctx *ctx, BlockRes &B, DevState in) {
+template <int NS, typename T, bool EPS0>
+void launch_fvs_e(ostc_ctx *ctx, BlockRes &B, DevState in) {
   const DevBlock &b = B.db;
   const int nv = ctx->nv, sch = ctx->der.inviscid_scheme;
   {
     long tok = begin_t(ctx, "flux_x");
     dim3 grid((b.mx + FvsTile<0>::TD - 2) / (FvsTile<0>::TD - 1), b.my, b.mz);
-    k_fvs<0, NS, T><<<grid, FvsTile<0>::TD, fvs_smem_bytes<0, T>(nv), ctx->stream>>>(b, in, B.dq, nv, sch);
+    k_fvs<0, NS, T, EPS0><<<grid, FvsTile<0>::TD, fvs_smem_bytes<0, T>(nv), ctx->stream>>>(b, in, B.dq, nv, sch);
     end_t(ctx, tok);
   }
   {
     long tok = begin_t(ctx, "flux_y");
     dim3 grid((b.mx + FvsTile<1>::TXL - 1) / FvsTile<1>::TXL, (b.my + FvsTile<1>::TD - 2) / (FvsTile<1>::TD - 1), b.mz);
-    k_fvs<1, NS, T><<<grid, dim3(FvsTile<1>::TXL, FvsTile<1>::TD), fvs_smem_bytes<1, T>(nv), ctx->stream>>>(b, in, B.dq, nv, sch);
+    k_fvs<1, NS, T, EPS0><<<grid, dim3(FvsTile<1>::TXL, FvsTile<1>::TD), fvs_smem_bytes<1, T>(nv), ctx->stream>>>(b, in, B.dq, nv, sch);
     end_t(ctx, tok);
   }
   if (b.mz > 1) {
     long tok = begin_t(ctx, "flux_z");
     dim3 grid((b.mx + FvsTile<2>::TXL - 1) / FvsTile<2>::TXL, (b.mz + FvsTile<2>::TD - 2) / (FvsTile<2>::TD - 1), b.my);
-    k_fvs<2, NS, T><<<grid, dim3(FvsTile<2>::TXL, FvsTile<2>::TD), fvs_smem_bytes<2, T>(nv), ctx->stream>>>(b, in, B.dq, nv, sch);
+    k_fvs<2, NS, T, EPS0><<<grid, dim3(FvsTile<2>::TXL, FvsTile<2>::TD), fvs_smem_bytes<2, T>(nv), ctx->stream>>>(b, in, B.dq, nv, sch);
     end_t(ctx, tok);
   }
+}
+
+// FP64 without a reference state: the weights' epsilon is 0 (FP32 divides each side's quotient in any case)
+template <int NS, typename T>
+void launch_fvs_t(ostc_ctx *ctx, BlockRes &B, DevState in) {
+  if (sizeof(T) == 8 && ctx->mixtab.weno_eps_scale == 0) launch_fvs_e<NS, T, sizeof(T) == 8>(ctx, B, in);
+  else launch_fvs_e<NS, T, false>(ctx, B, in);
 }
 
 // mixture viscous sweeps, accumulating into dq
@@ -653,6 +660,9 @@ bool set_mix_attrs() {
   set((const void *)k_fvs<0, NS, double>, fvs_smem_bytes<0, double>(5 + N));                 \
   set((const void *)k_fvs<1, NS, double>, fvs_smem_bytes<1, double>(5 + N));                 \
   set((const void *)k_fvs<2, NS, double>, fvs_smem_bytes<2, double>(5 + N));                 \
+  set((const void *)k_fvs<0, NS, double, true>, fvs_smem_bytes<0, double>(5 + N));           \
+  set((const void *)k_fvs<1, NS, double, true>, fvs_smem_bytes<1, double>(5 + N));           \
+  set((const void *)k_fvs<2, NS, double, true>, fvs_smem_bytes<2, double>(5 + N));           \
   set((const void *)k_fvs<0, NS, float>, fvs_smem_bytes<0, float>(5 + N));                   \
   set((const void *)k_fvs<1, NS, float>, fvs_smem_bytes<1, float>(5 + N));                   \
   set((const void *)k_fvs<2, NS, float>, fvs_smem_bytes<2, float>(5 + N));                   \

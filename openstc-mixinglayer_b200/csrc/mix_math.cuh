@@ -620,28 +620,28 @@ __device__ __forceinline__ void fvs_side(T v0, T v1, T v2, T v3, T v4, T v5, T v
 }
 
 // Both sides of the flux-split WENO7-Z: f+ + f-, the - side mirrored.  FP64 forms the two quotients with
-// one division where the product of the two weight sums stays in range: a sum is at most tau / eps^2, ~1e80 with the
-// epsilon of a reference state, but without one epsilon is 0 and a substencil of vanishing fluxes (a mass fraction of
-// 1e-40 beside one of 1e-3) has a weight of 1e150.
-template <typename T>
+// one division by the product of the two weight sums, which are at most tau / eps^2, ~1e80 with the epsilon of a
+// reference state.  EPS0: no reference state, epsilon 0; a substencil of vanishing fluxes (a mass fraction of 1e-50
+// beside one of 1e-3) then has a weight of 1e190 and each side takes its own division.
+template <typename T, bool EPS0 = false>
 __device__ __forceinline__ T fvs_weno7_core(const T *vp, const T *vm, T eps) {
   T np, dp, nm, dm;
   fvs_side(vp[0], vp[1], vp[2], vp[3], vp[4], vp[5], vp[6], eps, np, dp);
   fvs_side(vm[6], vm[5], vm[4], vm[3], vm[2], vm[1], vm[0], eps, nm, dm);
-  if constexpr (sizeof(T) == 8) {
-    const T dd = dp * dm;
-    return vp[3] + vm[3] + (dd < 1e250 ? (np * dm + nm * dp) / dd : np / dp + nm / dm);
-  } else return vp[3] + vm[3] + (__fdividef(np, dp) + __fdividef(nm, dm));
+  if constexpr (sizeof(T) == 8) return vp[3] + vm[3] + (EPS0 ? np / dp + nm / dm : (np * dm + nm * dp) / (dp * dm));
+  else return vp[3] + vm[3] + (__fdividef(np, dp) + __fdividef(nm, dm));
 }
 
+template <bool EPS0 = false>
 __device__ __forceinline__ double fvs_weno7(const double *vp, const double *vm, double eps) {
-  return fvs_weno7_core<double>(vp, vm, eps);
+  return fvs_weno7_core<double, EPS0>(vp, vm, eps);
 }
 
 // FP32 form.  beta ~ v^2 and tau ~ v^4, so the split fluxes of a minor species (|v| ~ 1e-11) or the
 // energy flux of a coarse grid (|v| ~ 1e10) leave the FP32 range although the weights themselves
 // (tau / (eps + beta)^2, scale-free as eps -> 0) are O(1).  The stencil is therefore scaled by the
 // power of two 2^-E below its largest magnitude (exact), eps by 2^-2E, and the face value scaled back.
+template <bool EPS0 = false>
 __device__ __forceinline__ float fvs_weno7(const float *vp, const float *vm, double eps) {
   float m = 0.f;
 #pragma unroll

@@ -177,7 +177,9 @@ __host__ __device__ constexpr size_t fvs_smem_bytes(int nv) {
 // keep slots of their own, formed once, not once in each of two loops, and the four
 // weights take one division: 1.62 -> 1.43 ms (FP64), 2.24 -> 2.17 ms (FP32).  Tiles of 4 lanes and 32 faces
 // (8 and 16 here): 1.52 and 2.29 ms.
-template <int DIR, int NS, typename T>
+// EPS0: the epsilon of the weights is 0 (no reference state; fvs_weno7_core).  A kernel of its own, since a test per
+// face value costs every case 1 % of the sweep.
+template <int DIR, int NS, typename T, bool EPS0 = false>
 __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T) == 8 ? 4 : 6) k_fvs(DevBlock b, DevState s,
                                                                                double *__restrict__ dq, int nv,
                                                                                int scheme) {
@@ -257,7 +259,7 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
         vp[m] = FP(m, l);
         vm[m] = FM(m, l);
       }
-      (l < 5 ? FL(t, l) : SP(t, l - 5)) = fvs_weno7(vp, vm, e);
+      (l < 5 ? FL(t, l) : SP(t, l - 5)) = fvs_weno7<EPS0>(vp, vm, e);
     }
   } else if (face_ok) {
     // Roe-averaged mixture eigensystem at the face (WENO.cu:747-821).  The averaged mass fractions and the
@@ -388,7 +390,7 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
           vmn[m] += L[q] * FM(m, q);
         }
       }
-      const T fch = fvs_weno7(vp, vmn, eps);
+      const T fch = fvs_weno7<EPS0>(vp, vmn, eps);
 #pragma unroll
       for (int q = 0; q < 5; ++q) fc[q] += R[q] * fch;
     }
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T
         vp[m] = FP(m, 5 + l) - sv * p0[m];
         vmn[m] = FM(m, 5 + l) - sv * m0[m];
       }
-      const T fch = fvs_weno7(vp, vmn, eps);
+      const T fch = fvs_weno7<EPS0>(vp, vmn, eps);
       add += SP(t, l) * fch;
       SP(t, l) = sv * fc[0] + fch;
     }
