@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) k_cfl_dt(DevBlock b, DevState s, double c
   __syncthreads();
   if (threadIdx.x == 0) {
     double m = wmin[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmin(m, wmin[w]);
+    for (int q = 1; q < (int)(blockDim.x >> 5); ++q) m = fmin(m, wmin[q]);
     atomicMin(&w->bits, (unsigned long long)__double_as_longlong(m));
     __threadfence();
     if (atomicAdd(&w->arrived, 1u) == total - 1) {
@@ -163,13 +163,13 @@ __global__ void __launch_bounds__(128, RECT && sizeof(T) == 8 ? 4 : FluxXOcc<T>:
 // y / z sweep as a tile: a block of TXL consecutive i (coalesced rows) x TD threads along the sweep
 // direction stages TF - 1 + 2*NG nodes per lane in shared memory (cv, p, node flux, metric row,
 // Jacobian), computes FPT faces per thread and finalises TF - 1 nodes per lane, as the x sweep does
-// for rows.  Bound by FP64 (FP32) arithmetic, ~50 % of the pipe, and the latency of the staging loads.  The
-// node's sum goes to dq by an atomicAdd whose result nobody reads, a reduction at L2: a load and a store made
-// the block hold its shared memory and registers until the load came back.  One thread adds to an entry in a
-// launch, so the sum is the plain one.  With it 512 x 256 x 128 WENO7 + HLLC, FP64: 3.13 -> 2.51 ms a sweep,
-// 385 x 257 x 129, FP32: 1.33 -> 1.19 (16 x 8 x 2 and 32 x 8 x 2 tiles).  A longer tile of half the lanes
-// re-reads fewer halo nodes (1.26 loads a node, 1.53 at TF = 16, NG = 4): 2.48 and 1.13 ms.  One thread marching
-// a column with a ring of nodes in shared memory, each node loaded once, took 3.84 and 2.17.
+// for rows.  Bound by FP64 (FP32) arithmetic and the latency of the staging loads.  The
+// node's sum goes to dq by an atomicAdd whose result nobody reads, a reduction at L2: a load and a store make
+// the block hold its shared memory and registers until the load comes back (20 % slower).  One thread adds to an
+// entry in a launch, so the sum is the plain one.  512 x 256 x 128, WENO7 + HLLC, FP64, a sweep: 1.85 ms on a rectilinear
+// block, 2.48 with the whole metric; 385 x 257 x 129, FP32: 0.89 and 1.13 (8 x 16 x 2 and 16 x 16 x 2 tiles).  A longer tile of
+// half the lanes re-reads fewer halo nodes (1.26 loads a node, 1.53 at TF = 16, NG = 4).  One thread marching
+// a column with a ring of nodes in shared memory, each node loaded once, took 3.84 and 2.17 ms.
 // TF = TD * FPT faces per tile along the sweep (TF - 1 nodes finalised), FPT faces per thread.
 template <int NG, int TXL, int TF, typename T, bool RECT>
 constexpr size_t tile_smem_bytes() {

@@ -1,7 +1,9 @@
 // air_math.cuh -- per-face / per-node arithmetic of the calorically-perfect-air RHS, written once and
-// instantiated for T = double (plain FP64 path) and T = float (mixed path).  The operation order of
-// every expression follows the reference source it cites, so the FP64 instantiation reproduces the
-// reference to rounding.
+// instantiated for T = double (plain FP64 path) and T = float (mixed path).  The expressions are
+// algebraically those of the reference source they cite, in forms of their own (differences of points, shared
+// quotients, products in place of divisions); parity with the reference, 1e-12, is what the tests check.  On a
+// rectilinear block (rectilinear() in host.h) the terms of the off-diagonal metric entries, rounding there, are
+// left out on purpose.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -5,13 +5,12 @@
 // the discrete adjoint of the forward kernels in ostc_mix.cuh, term by term:
 //   1. face sweeps (hand-written reverse): dq_bar -> adjoints of the node quantities they read
 //      (cv, p, acoustic speed; u, v, w, T, Y, mu, lambda, rho*D), accumulated per padded node;
-//   2. chemistry and transport properties (node-local, forward-mode Dual evaluations of the same
-//      templated device code, one seeded input per pass): -> adjoints of rho, p, T, Y;
+//   2. chemistry and transport properties (node-local, hand-written; Dual evaluations only of fall-off rates
+//      and, for mechanisms that do not fit the reaction lists, of every rate): -> adjoints of rho, p, T, Y;
 //   3. equation of state reverse (rho, u, v, w, p, T, Y as functions of cv, T through the
 //      implicit energy relation) -> cv adjoint per padded node;
 //   4. ghost fills in reverse order: a ghost's cv adjoint is added to the node it was copied from.
-// Accumulation into shared memory and into the node planes uses atomicAdd, so results are
-// reproducible to rounding, not bitwise.
+// Accumulation into the node planes uses atomicAdd, so results are reproducible to rounding, not bitwise.
 #pragma once
 
 #include "ostc_mix.cuh"
@@ -251,8 +250,7 @@ __host__ __device__ constexpr size_t adj_fvs_smem_bytes(int nv) {
 // steps.  The flow rows reach the species' split fluxes with one factor alpha_l times a sum W[m] over the
 // rows, and the species fields reach the density's with a sum Z[m], so those go out once per side.  One
 // pass over the fields: the WENO reverse returns the face value too, which the adjoints of R need.
-// [96 x 64 x 48, 9 species: 2.4-2.6 ms a direction with the atomics; without, and with the tables of
-// k_adj_props, the whole VJP went from 11.6 to 5.0 ms]
+// 96 x 64 x 48, 9 species: 0.95 / 0.89 / 0.94 ms (x / y / z); with FP64 shared-memory atomics 2.4-2.6 ms each.
 template <int DIR, int NS>
 __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, 2) k_adj_fvs(DevBlock b, DevState s,
                                                                                       const double *__restrict__ dqb,
@@ -932,8 +930,7 @@ __global__ void __launch_bounds__(128, 4) k_adj_source(DevBlock b, DevState s, c
 
 // The same over the reaction lists with the species arrays in shared memory (as mix_chemistry_listed):
 // d ln kf / dT = b / T + Ea / T^2 for the Arrhenius types, d g / dT = -h / (Ru T^2) for the equilibrium constant;
-// only fall-off reactions take Dual evaluations.  [96 x 64 x 48, 19 reactions:
-// dense 0.65 ms of the VJP, listed 0.4]
+// only fall-off reactions take Dual evaluations.  96 x 64 x 48, 19 reactions: 0.31 ms; dense 0.65.
 template <int NS>
 __global__ void __launch_bounds__(128, 4) k_adj_source_listed(DevBlock b, DevState s, const double *__restrict__ dqb,
                                                              DevAdj A) {
@@ -1060,9 +1057,8 @@ __global__ void __launch_bounds__(128, 4) k_adj_source_listed(DevBlock b, DevSta
 // adjoints of c, mu, lambda and rho*D_k -> adjoints of rho, p, T and Y.  Hand-written reverse of
 // mix_properties (one forward sweep keeping its intermediates, then the reverse sweep).
 // The powers, square roots and quotients are those of mix_properties (one log, one exp, one reciprocal
-// square root a species, the powers of the collision integrals' constants in the tables); with a pow per
-// species and pair and a square root per ratio it took 1.7 ms at 96 x 64 x 48, of a VJP of 11.6 then
-// and 5.0 now.
+// square root a species, the powers of the collision integrals' constants in the tables): 0.27 ms at 96 x 64 x 48;
+// with a pow per species and pair and a square root per ratio 1.7 ms.
 template <int NS>
 __global__ void __launch_bounds__(128, 2) k_adj_props(DevBlock b, DevState s, DevAdj A) {
   const long long P = b.plane;

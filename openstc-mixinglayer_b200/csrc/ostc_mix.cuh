@@ -167,16 +167,14 @@ __host__ __device__ constexpr size_t fvs_smem_bytes(int nv) {
 // type of the fluxes (FP32 in the mixed precision mode: state read in FP64, dq accumulated in FP64).
 // Bound by FP64 arithmetic at the occupancy its shared memory and registers leave (40 % of the FP64 pipe;
 // DRAM 8 %).  The staged values are laid out variable by variable, so that a warp's threads read
-// consecutive words; with the variables of a node side by side (a stride of 14 doubles) every read was a
-// two-way bank conflict.  Species arrays live in the thread's slots and the staged values are read
-// again per row: spills 2.8 KB -> 0.3 KB a thread.  192 x 96 x 48, FP64: 0.86 / 0.79 / 0.85 -> 0.60 / 0.58 /
-// 0.64 ms (x / y / z); 257 x 129 x 65, FP32: 1.32 / 1.19 / 1.27 -> 0.85 / 0.78 / 0.85 ms.  Resident blocks
-// per SM: FP64 4 (three sweeps 1.82 ms; 3: 1.92), FP32 6 (2.48 ms; 8: 2.54).  dq takes the differences by an
-// atomicAdd whose result nobody reads (a reduction at L2; one thread adds to an entry), so that the block ends
-// without waiting for a load of dq: 1.80 -> 1.62 ms (FP64), 2.50 -> 2.24 ms (FP32).  The averaged mass fractions
-// keep slots of their own, formed once, not once in each of two loops, and the four
-// weights take one division: 1.62 -> 1.43 ms (FP64), 2.24 -> 2.17 ms (FP32).  Tiles of 4 lanes and 32 faces
-// (8 and 16 here): 1.52 and 2.29 ms.
+// consecutive words; with the variables of a node side by side (a stride of 14 doubles) every read is a
+// two-way bank conflict.  Species arrays (the averaged mass fractions, then the fluxes) live in the thread's own
+// slots and the staged values are read again per row, or 2.8 KB a thread would spill (0.3 KB now).  dq takes the
+// differences by an atomicAdd whose result nobody reads (a reduction at L2; one thread adds to an entry), so that
+// the block ends without waiting for a load of dq (10 % of the sweep).  Three sweeps: 192 x 96 x 48, FP64, 1.43 ms (2.50
+// with node-wise staging, arrays in registers and a division per weight), 257 x 129 x 65, FP32, 2.17 ms (3.78).
+// Resident blocks per SM: FP64 4 (3: 5 % slower), FP32 6 (8: 2 % slower); tiles of 4 lanes and 32 faces instead of 8
+// and 16: 1.52 and 2.29 ms.
 // EPS0: the epsilon of the weights is 0 (no reference state; fvs_weno7_core).  A kernel of its own, since a test per
 // face value costs every case 1 % of the sweep.
 template <int DIR, int NS, typename T, bool EPS0 = false>
@@ -536,10 +534,11 @@ __device__ __forceinline__ void mix_visc_face(const DevBlock &b, const DevState 
 
 // viscous_flux_fv/gv/hv (SchemeSelector.cuh:69-154) for mixtures: one thread per face of the tile,
 // then dq += fv(i+1/2) - fv(i-1/2) through shared memory; tiles as the flux-split sweeps.
-// Bound by the latency of its loads at the registers' occupancy.  dq takes the difference by an atomicAdd whose
-// result nobody reads (a reduction at L2; one thread an entry), with no load of dq to wait for, and the faces
-// are laid out variable by variable, free of bank conflicts; the species' loads go out together (mix_visc_face): three sweeps of 192 x 96 x 48, FP64, 0.69 -> 0.33 ms, of
-// 257 x 129 x 65, FP32, 1.63 -> 0.79 ms.
+// Bound by the latency of its loads at the registers' occupancy, so the species' loads go out together
+// (mix_visc_face) and dq takes the difference by an atomicAdd whose result nobody reads (a reduction at L2; one
+// thread an entry), with no load of dq to wait for; the faces are laid out variable by variable, free of bank
+// conflicts.  Three sweeps: 192 x 96 x 48, FP64, 0.33 ms (0.69 with a branch per species and a load of dq), 257 x 129 x
+// 65, FP32, 0.79 ms (1.63).
 template <int DIR, bool DIM3, int NS, typename T>
 __global__ void __launch_bounds__(FvsTile<DIR>::TD * FvsTile<DIR>::TXL, sizeof(T) == 8 ? 4 : 5) k_mix_visc(DevBlock b, DevState s,
                                                                                     double *__restrict__ dq, int nv) {
