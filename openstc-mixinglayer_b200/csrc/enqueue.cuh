@@ -203,11 +203,16 @@ void launch_mix_source(ostc_ctx *ctx, BlockRes &B, DevState in, bool chem) {
   if (ctx->der.n_spec == kFixedNS) launch_mix_source_t<kFixedNS>(ctx, B, in, chem);
   else launch_mix_source_t<0>(ctx, B, in, chem);
 }
+// Over the lists, a cell's matrix in shared memory, while an SM holds two blocks (up to 13 species) or the block of
+// cells is one wave of one block an SM; else over every species with the matrices in local memory, whose 4 blocks of
+// 128 an SM then outrun the one of 64.  Three stages, listed / dense, ms: 9 species, 97 x 65 x 33, 1.11 / 1.62, 13
+// 3.79 / 4.62, 14 8.18 / 5.59, 16 9.40 / 6.92; 14 species, 21 x 21 x 21 (one wave) 0.39 / 0.68, 27 x 21 x 21 0.76 / 0.68.
 template <int NS>
 void launch_chem_epi_t(ostc_ctx *ctx, BlockRes &B, DevState in) {
-  if (ctx->mixtab.listed)
-    k_mix_chem_epi<NS, true><<<grid_for(ctx, B.db.n, 64), 64, chem_columns(ctx->der.n_spec, true) * 64 * sizeof(double),
-                               ctx->stream>>>(B.db, in, B.dq, ctx->d_dt);
+  const size_t smem = chem_columns(ctx->der.n_spec, true) * 64 * sizeof(double);
+  const bool fits = 2 * (smem + 1024) <= 228 * 1024 || B.db.n <= 64LL * ctx->sm_count;
+  if (ctx->mixtab.listed && fits)
+    k_mix_chem_epi<NS, true><<<grid_for(ctx, B.db.n, 64), 64, smem, ctx->stream>>>(B.db, in, B.dq, ctx->d_dt);
   else
     k_mix_chem_epi<NS, false><<<grid_for(ctx, B.db.n, 128), 128, 0, ctx->stream>>>(B.db, in, B.dq, ctx->d_dt);
 }
